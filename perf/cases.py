@@ -49,7 +49,7 @@ def listed():
              precision="mixed", fov="matched", batch=128),
         # a whole 512^3 scan in FP32
         dict(name="recon_512_fp32", kind="recon", nx=512, ny=512, nz=512, nu=512, nv=512, views=512,
-             precision="fp32", fov="matched", batch=512),
+             precision="fp32", fov="covered", batch=512),
         # a rank's slab pair of a 2048^3 volume: one batch of filtered views that another stage left on the device
         dict(name="bp_2048_mixed", kind="bp", nx=2048, ny=2048, nz=2048, slab=64, nu=2048, nv=2048, views=64,
              precision="mixed", fov="covered"),
