@@ -755,7 +755,7 @@ def run_ours(args, param, rank: int, world: int, local: int) -> None:
                            "peak_source": tc_src, "algorithmic_flops_per_step": flops, "launch_ms": flt_step_ms,
                            "hbm_view_gbs": flt_bytes / (flt_step_ms * 1e-3) / 1e9, "traffic": None}
         else:
-            filter_roof = {"kernel": "filter_mirror_kernel", "bound": "hbm",
+            filter_roof = {"kernel": "filter_kernel", "bound": "hbm",
                            "achieved": flt_bytes / (flt_step_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                            "frac": flt_bytes / (flt_step_ms * 1e-3) / 1e9 / hbm_peak,
                            "algorithmic_bytes_per_launch": flt_bytes, "launch_ms": flt_step_ms,

@@ -2,28 +2,25 @@
 // ramp/window filter by FFT, crop, and the store in the layout the backprojection reads.
 //
 // Reference semantics: FilterEngine::Filtering (Filterlib/FilterLib.h:167-196) and the cuFFT
-// plugin (FilterlibCufft/cudaFftFilter.cu:14-61, 283-392).  One CTA filters two detector rows
-// at once -- row r and its mirror row nv-1-r -- as the real and imaginary parts of one complex
-// FFT of length W: with a real, even response H the two filtered rows come back as the real
-// and imaginary parts of the inverse transform.  Pairing r with nv-1-r is what lets the same
-// CTA emit the backprojection's mirror-pair layout directly.
+// plugin (FilterlibCufft/cudaFftFilter.cu:14-61, 283-392).  Two detector rows -- row r and its
+// mirror row nv-1-r -- are the real and imaginary parts of one complex FFT of length W: with a
+// real, even response H the two filtered rows come back as the real and imaginary parts of the
+// inverse transform.  Pairing r with nv-1-r is what lets one CTA emit the backprojection's
+// mirror-pair layout directly.
 //
-// FFT: radix-2 decimation in frequency (natural -> bit-reversed order), pointwise multiply by
-// H[bitrev(p)]/W, radix-2 decimation in time (bit-reversed -> natural), in shared memory.
-// Three consecutive radix-2 stages run per pass in registers: the stages of a pass touch three
-// adjacent index bits, so the 8 elements that differ only in those bits form a closed group.
-// Every butterfly is the plain radix-2 one, so the arithmetic is that of the stage-by-stage
-// transform, with a third of the shared-memory round trips and barriers.  Twiddles come from
-// an FP64-computed table, rearranged per pass so that a group reads its own with vector loads.
-//
-// The backprojection's MIRROR layout is written by filter_mirror_kernel: a CTA filters G row
-// pairs in turn, collects their outputs as an nu x G tile per side in shared memory, and writes
-// each detector column's G consecutive elements as one 16-byte store.
+// FFT: W / 16 threads hold the W points of a row pair in registers, 16 each, and run at most three
+// passes a direction (W = 16 x 16 x W/256; 4096 = 16^3), a radix-16 transform in registers each.
+// The samples go from global memory straight into the first pass's registers and from the last
+// pass's registers out again, the spectrum is multiplied by H between the forward and the inverse
+// half of the innermost pass, and so a row pair crosses shared memory four times in all.  Bound:
+// shared-memory wavefronts and FP32 issue about equally (per 512 points and warp some 460
+// wavefronts and 1100 FP32 instructions at W = 4096).
 #include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.h"
@@ -36,372 +33,382 @@ struct FilterArgs {
     void *dst;          // output, layout dependent
     const float *cos;   // nv x nu (pitch cos_pitch) or nullptr
     const float2 *tw;   // W/2 twiddles exp(-2 pi i k / W)
-    const float2 *twp;  // per pass and group, the group's twiddles (FilterTables::twp) or nullptr
-    const float *hb;    // W: H[bitrev(p)] / W
-    int nu, nv, W, log2W, off, pad_n;
+    const float2 *twp;  // the passes' twiddles (FilterTables::twp), or nullptr: gathered from tw
+    const float *hb;    // W: H / W in the order of the transform's registers (FilterTables)
+    int nu, nv, off, pad_n, n_pairs;
     int src_pitch, dst_pitch, cos_pitch;
     long long src_vstride, dst_vstride;
+    int layout, half;         // FDK_LAYOUT_*, FP16 output
+    int pair_stores;          // MIRROR: dst takes a pair as one store
     float out_scale;          // multiplies every output sample (FP16 range control)
     unsigned int *overflow;   // set to 1 when a scaled FP16 output exceeds the format (or NULL)
 };
 
-template <typename OUT>
-__device__ __forceinline__ OUT to_out(const FilterArgs &a, float y) {
-    if constexpr (sizeof(OUT) == 2) {
-        const float s = y * a.out_scale;
-        if (a.overflow && !(fabsf(s) <= 65504.f)) atomicOr(a.overflow, 1u);
-        return __float2half_rn(s);
-    } else {
-        return y * a.out_scale;
-    }
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// a * w, or a * conj(w)
+template <bool CONJ>
+__device__ __forceinline__ float2 cmul(float2 a, float2 w) {
+    if (CONJ) return make_float2(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
+    return make_float2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
 }
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
-    return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
-
-// Weighted sample of row r at column c of the current view.
-__device__ __forceinline__ float row_sample(const FilterArgs &a, const float *view, int r, int c) {
-    float x = __ldg(view + (long long)r * a.src_pitch + c);
-    if (a.cos) x *= __ldg(a.cos + (long long)r * a.cos_pitch + c);
-    return x;
+// A table load that stays where it is written.  The forward and the inverse half read the same
+// twiddles; as plain read-only loads the compiler merges the two and keeps 32 to 64 registers alive
+// from one half to the other, as spills to local memory (300 bytes a thread at W = 4096, which
+// missed L1 and made two thirds of the kernel's L2 traffic: 1469 against 1139 us for 32 views of
+// 2048^2 to MIRROR FP32, before the CTA size was chosen).
+__device__ __forceinline__ float4 load_here(const float4 *p) {
+    float4 f;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(p) : "memory");
+    return f;
 }
 
-// Shared-memory position of element i of an FFT: i ^ ((i >> 4) & 15), a permutation inside each
-// block of 16 float2.  Later DIF and early DIT passes read groups 8 or 64 elements apart, which
-// in the plain layout fall into the same banks (up to 16-way conflicts); the swizzle spreads
-// them, and contiguous runs stay contiguous within their block (about 2.5 wavefronts per warp
-// access against 6 for the plain layout, in a model of the passes at W = 512 .. 4096).
-__device__ __forceinline__ int fsw(int i) { return i ^ ((i >> 4) & 15); }
+// 4-point transform of v[b], v[b + s], v[b + 2s], v[b + 3s] in place, exp(-2 pi i / 4) or, INV, its conjugate
+template <bool INV, int N>
+__device__ __forceinline__ void dft4(float2 (&v)[N], int b, int s) {
+    const float2 t0 = cadd(v[b], v[b + 2 * s]), t1 = csub(v[b], v[b + 2 * s]);
+    const float2 t2 = cadd(v[b + s], v[b + 3 * s]), t3 = csub(v[b + s], v[b + 3 * s]);
+    const float2 r = INV ? make_float2(-t3.y, t3.x) : make_float2(t3.y, -t3.x);  // +-i t3
+    v[b] = cadd(t0, t2);
+    v[b + s] = cadd(t1, r);
+    v[b + 2 * s] = csub(t0, t2);
+    v[b + 3 * s] = csub(t1, r);
+}
 
-// Twiddles of a group.  A DIF pass starting at stage s0 needs, for stage t and butterfly j,
-// tw[(g_low + (j mod 2^(NS-1-t)) 2^low) << (s0 + t)], and a DIT pass starting at bit b0
-// tw[(g_low + (j mod 2^t) 2^b0) << (log2W - 1 - b0 - t)] (g_low: the group's index bits below
-// the pass): 2^NS - 1 distinct values, listed stage by stage and padded to 2^NS.  FilterTables
-// keeps every pass's lists as 2^(NS-1) planes of 16-byte pairs, plane k holding pair k of every
-// group in group order, so a warp's k-th load covers consecutive 16-byte words; without that
-// table (twp == nullptr) the list is gathered from tw.  (One scattered load per butterfly made
-// the kernel L1-bound.)
-
-// One pass of NS consecutive radix-2 DIF stages, the first being stage s0 (half = W >> (s0+1)).
-// Those stages touch index bits hbit .. hbit-NS+1; a group is the 2^NS elements that differ only
-// there.  Butterfly: (x, y) -> (x + y, (x - y) tw[(i & (half-1)) << stage]).  hb_tab (last pass
-// only) multiplies the bit-reversed result by H[bitrev(p)] / W.  twp: this pass's group lists.
-template <int NS>
-__device__ __forceinline__ void dif_pass(float2 *buf0, const float2 *__restrict__ tw, const float2 *__restrict__ twp,
-                                         const float *__restrict__ hb_tab, int W, int log2W, int s0, int count) {
-    constexpr int GS = 1 << NS;
-    const int hbit = log2W - 1 - s0;
-    const int low = hbit - NS + 1;
-    for (int gg = threadIdx.x; gg < (count << (log2W - NS)); gg += blockDim.x) {
-        float2 *buf = buf0 + ((gg >> (log2W - NS)) << log2W);  // FFT gg / (W >> NS) of count
-        const int g = gg & ((W >> NS) - 1);
-        const int g_low = g & ((1 << low) - 1);
-        const int base = ((g >> low) << (hbit + 1)) | g_low;
-        float2 v[GS];
+// R-point transform of v[b .. b + R-1], natural order in and out (the final reordering is a renaming
+// of registers).
+template <int R, bool INV, int N>
+__device__ __forceinline__ void dft(float2 (&v)[N], int b) {
+    constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508977f, h = 0.70710678118654752f;
+    if constexpr (R == 2) {
+        const float2 x = v[b], y = v[b + 1];
+        v[b] = cadd(x, y);
+        v[b + 1] = csub(x, y);
+    } else if constexpr (R == 4) {
+        dft4<INV>(v, b, 1);
+    } else if constexpr (R == 8) {  // 4 x 2
+        dft4<INV>(v, b, 2);
+        dft4<INV>(v, b + 1, 2);
+        v[b + 3] = cmul<INV>(v[b + 3], make_float2(h, -h));
+        v[b + 5] = INV ? make_float2(-v[b + 5].y, v[b + 5].x) : make_float2(v[b + 5].y, -v[b + 5].x);
+        v[b + 7] = cmul<INV>(v[b + 7], make_float2(-h, -h));
+        float2 o[8];
 #pragma unroll
-        for (int j = 0; j < GS; j++) v[j] = buf[fsw(base + (j << low))];
-        float2 tq[GS];  // stage t's list starts at GS - (GS >> t)
-        if (twp) {
-            const float4 *q = reinterpret_cast<const float4 *>(twp) + g_low;
-#pragma unroll
-            for (int k = 0; k < GS / 2; k++) {
-                const float4 f = __ldg(q + (k << low));  // plane k of 2^low groups
-                tq[2 * k] = make_float2(f.x, f.y);
-                tq[2 * k + 1] = make_float2(f.z, f.w);
-            }
-        } else {
-#pragma unroll
-            for (int t = 0; t < NS; t++)
-#pragma unroll
-                for (int jt = 0; jt < (GS >> (t + 1)); jt++)
-                    tq[GS - (GS >> t) + jt] = __ldg(tw + ((g_low + (jt << low)) << (s0 + t)));
+        for (int k = 0; k < 4; k++) {
+            o[k] = cadd(v[b + 2 * k], v[b + 2 * k + 1]);
+            o[k + 4] = csub(v[b + 2 * k], v[b + 2 * k + 1]);
         }
 #pragma unroll
-        for (int t = 0; t < NS; t++) {
-            const int hstep = GS >> (t + 1);
+        for (int k = 0; k < 8; k++) v[b + k] = o[k];
+    } else if constexpr (R == 16) {  // 4 x 4
 #pragma unroll
-            for (int j = 0; j < GS; j++) {
-                if (j & hstep) continue;
-                const float2 w = tq[GS - (GS >> t) + (j & ((1 << (NS - 1 - t)) - 1))];
-                const float2 x = v[j], y = v[j + hstep];
-                v[j] = make_float2(x.x + y.x, x.y + y.y);
-                v[j + hstep] = cmul(make_float2(x.x - y.x, x.y - y.y), w);
-            }
-        }
-        if (hb_tab) {
+        for (int q = 0; q < 4; q++) dft4<INV>(v, b + q, 4);
+        // v[b + q + 4 k] *= w16^(q k)
+        v[b + 5] = cmul<INV>(v[b + 5], make_float2(c1, -s1));
+        v[b + 6] = cmul<INV>(v[b + 6], make_float2(h, -h));
+        v[b + 7] = cmul<INV>(v[b + 7], make_float2(s1, -c1));
+        v[b + 9] = cmul<INV>(v[b + 9], make_float2(h, -h));
+        v[b + 10] = INV ? make_float2(-v[b + 10].y, v[b + 10].x) : make_float2(v[b + 10].y, -v[b + 10].x);
+        v[b + 11] = cmul<INV>(v[b + 11], make_float2(-h, -h));
+        v[b + 13] = cmul<INV>(v[b + 13], make_float2(s1, -c1));
+        v[b + 14] = cmul<INV>(v[b + 14], make_float2(-h, -h));
+        v[b + 15] = cmul<INV>(v[b + 15], make_float2(-c1, s1));
 #pragma unroll
-            for (int j = 0; j < GS; j++) {
-                const float h = __ldg(hb_tab + base + (j << low));
-                v[j] = make_float2(v[j].x * h, v[j].y * h);
-            }
-        }
+        for (int k = 0; k < 4; k++) dft4<INV>(v, b + 4 * k, 1);
+        float2 o[16];
 #pragma unroll
-        for (int j = 0; j < GS; j++) buf[fsw(base + (j << low))] = v[j];
-    }
-}
-template <int NS>
-__device__ __forceinline__ void dit_pass(float2 *buf0, const float2 *__restrict__ tw, const float2 *__restrict__ twp,
-                                         int W, int log2W, int b0, int count) {
-    constexpr int GS = 1 << NS;
-    for (int gg = threadIdx.x; gg < (count << (log2W - NS)); gg += blockDim.x) {
-        float2 *buf = buf0 + ((gg >> (log2W - NS)) << log2W);
-        const int g = gg & ((W >> NS) - 1);
-        const int g_low = g & ((1 << b0) - 1);
-        const int base = ((g >> b0) << (b0 + NS)) | g_low;
-        float2 v[GS];
+        for (int k = 0; k < 16; k++) o[k] = v[b + 4 * (k & 3) + (k >> 2)];
 #pragma unroll
-        for (int j = 0; j < GS; j++) v[j] = buf[fsw(base + (j << b0))];
-        float2 tq[GS];  // stage t's list starts at 2^t - 1
-        if (twp) {
-            const float4 *q = reinterpret_cast<const float4 *>(twp) + g_low;
-#pragma unroll
-            for (int k = 0; k < GS / 2; k++) {
-                const float4 f = __ldg(q + (k << b0));  // plane k of 2^b0 groups
-                tq[2 * k] = make_float2(f.x, f.y);
-                tq[2 * k + 1] = make_float2(f.z, f.w);
-            }
-        } else {
-#pragma unroll
-            for (int t = 0; t < NS; t++)
-#pragma unroll
-                for (int jt = 0; jt < (1 << t); jt++)
-                    tq[(1 << t) - 1 + jt] = __ldg(tw + ((g_low + (jt << b0)) << (log2W - 1 - b0 - t)));
-        }
-#pragma unroll
-        for (int t = 0; t < NS; t++) {
-            const int hstep = 1 << t;
-#pragma unroll
-            for (int j = 0; j < GS; j++) {
-                if (j & hstep) continue;
-                const float2 w = tq[(1 << t) - 1 + (j & ((1 << t) - 1))];
-                const float2 x = v[j];
-                const float2 u = cmulc(v[j + hstep], w);
-                v[j] = make_float2(x.x + u.x, x.y + u.y);
-                v[j + hstep] = make_float2(x.x - u.x, x.y - u.y);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < GS; j++) buf[fsw(base + (j << b0))] = v[j];
+        for (int k = 0; k < 16; k++) v[b + k] = o[k];
     }
 }
 
-// Forward transform, multiply by H, inverse transform of `count` W-point FFTs stored one after
-// the other in buf; ends after a barrier.
-__device__ __forceinline__ void filter_fft(float2 *buf, const FilterArgs &a, int count = 1) {
-    long long off = 0;  // this pass's group lists in a.twp: the DIF passes', then the DIT passes'
-    for (int s = 0; s < a.log2W; s += 3) {
-        const int ns = min(3, a.log2W - s);
-        const float *h = (s + ns == a.log2W) ? a.hb : nullptr;
-        const float2 *twp = a.twp ? a.twp + off : nullptr;
-        if (ns == 3) dif_pass<3>(buf, a.tw, twp, h, a.W, a.log2W, s, count);
-        else if (ns == 2) dif_pass<2>(buf, a.tw, twp, h, a.W, a.log2W, s, count);
-        else dif_pass<1>(buf, a.tw, twp, h, a.W, a.log2W, s, count);
-        off += (long long)(1 << ns) << (a.log2W - s - ns);
-        __syncthreads();
-    }
-    for (int b = 0; b < a.log2W; b += 3) {
-        const int ns = min(3, a.log2W - b);
-        const float2 *twp = a.twp ? a.twp + off : nullptr;
-        if (ns == 3) dit_pass<3>(buf, a.tw, twp, a.W, a.log2W, b, count);
-        else if (ns == 2) dit_pass<2>(buf, a.tw, twp, a.W, a.log2W, b, count);
-        else dit_pass<1>(buf, a.tw, twp, a.W, a.log2W, b, count);
-        off += (long long)(1 << ns) << b;
-        __syncthreads();
-    }
-}
-
-// Mean of the first (or last) pad_n weighted samples of row r.
-__device__ float edge_mean(const FilterArgs &a, const float *view, int r, bool left) {
-    float s = 0.f;
-    for (int k = 0; k < a.pad_n; k++) s += row_sample(a, view, r, left ? k : a.nu - 1 - k);
-    return s / (float)a.pad_n;
-}
-
-// LAYOUT: FDK_LAYOUT_ROWS, FDK_LAYOUT_TRANSPOSED, FDK_LAYOUT_MIRROR; OUT: float or __half
-template <int LAYOUT, typename OUT>
-__global__ void __launch_bounds__(256) filter_rows_kernel(FilterArgs a) {
-    extern __shared__ float2 buf[];
-    __shared__ float pads[4];
-    const int r1 = blockIdx.x;
-    const int r2 = a.nv - 1 - r1;
-    const int view = blockIdx.y;
-    const float *vsrc = a.src + (long long)view * a.src_vstride;
-    const int W = a.W;
-
-    if (threadIdx.x < 4) {
-        const int r = (threadIdx.x < 2) ? r1 : r2;
-        pads[threadIdx.x] = edge_mean(a, vsrc, r, (threadIdx.x & 1) == 0);
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < W; k += blockDim.x) {
-        const int c = k - a.off;
-        float x1, x2;
-        if (c < 0) {
-            x1 = pads[0]; x2 = pads[2];
-        } else if (c >= a.nu) {
-            x1 = pads[1]; x2 = pads[3];
-        } else {
-            x1 = row_sample(a, vsrc, r1, c);
-            x2 = row_sample(a, vsrc, r2, c);
-        }
-        buf[fsw(k)] = make_float2(x1, x2);
-    }
-    __syncthreads();
-
-    filter_fft(buf, a);
-
-    OUT *dst = reinterpret_cast<OUT *>(a.dst);
-    for (int u = threadIdx.x; u < a.nu; u += blockDim.x) {
-        const float2 y = buf[fsw(a.off + u)];
-        const OUT o1 = to_out<OUT>(a, y.x), o2 = to_out<OUT>(a, y.y);
-        if (LAYOUT == FDK_LAYOUT_ROWS) {
-            OUT *d = dst + (long long)view * a.dst_vstride;
-            d[(long long)r1 * a.dst_pitch + u] = o1;
-            if (r2 != r1) d[(long long)r2 * a.dst_pitch + u] = o2;
-        } else if (LAYOUT == FDK_LAYOUT_TRANSPOSED) {
-            OUT *d = dst + (long long)view * a.dst_vstride + (long long)u * a.dst_pitch;
-            d[r1] = o1;
-            if (r2 != r1) d[r2] = o2;
-        } else {  // mirror pairs: element (u, v) = (row v, row nv-1-v)
-            OUT *d = dst + (long long)view * a.dst_vstride + (long long)u * a.dst_pitch * 2;
-            d[2 * r1] = o1;
-            d[2 * r1 + 1] = o2;
-            if (r2 != r1) {
-                d[2 * r2] = o2;
-                d[2 * r2 + 1] = o1;
-            }
-        }
-    }
-}
-
-template <typename OUT>
-struct PairOf;
-template <>
-struct PairOf<float> {
-    using T = float2;
-    static __device__ __forceinline__ T make(float a, float b) { return make_float2(a, b); }
-};
-template <>
-struct PairOf<__half> {
-    using T = __half2;
-    static __device__ __forceinline__ T make(__half a, __half b) { return __halves2half2(a, b); }
+// Radices of a W-point transform: R1 over stride W / R1, then R2 (W > 256: 16) over stride W / 256,
+// then RL over contiguous points.
+template <int LOG2W>
+struct Fft {
+    static constexpr int W = 1 << LOG2W;
+    static constexpr int E = W < 16 ? W : 16;       // points per thread, the first radix
+    static constexpr int TPF = W / E;               // threads per transform
+    static constexpr bool MID = W > 256;            // a middle pass
+    static constexpr int RL = MID ? W / 256 : TPF;  // the last radix (1: no last pass)
+    // shared-memory slots of one transform: one float2 of padding per 16, so that the contiguous
+    // runs of the last pass (16 points a thread) and the strided ones of the others are all free
+    // of bank conflicts
+    static constexpr int PITCH = W + W / 16;
+    // CTAs per SM that the register budget is set for: 1024 threads of 64 registers
+    static constexpr int blocks(int g) { return 1024 / (TPF * g) < 16 ? 1024 / (TPF * g) : 16; }
 };
 
-// MIRROR layout, G row pairs (r, nv-1-r), r = G * blockIdx.x + g, per CTA; G * sizeof(pair) = 16.
-// NP = min(G, 4096 / W) pairs are transformed at once, so every 3-stage pass keeps all 512
-// threads busy (W / 8 groups per FFT).
-template <typename OUT, int G>
-__global__ void __launch_bounds__(512, 2) filter_mirror_kernel(FilterArgs a) {
-    using P = typename PairOf<OUT>::T;
-    static_assert(G * sizeof(P) == 16, "one 16-byte store per column and side");
-    extern __shared__ __align__(16) unsigned char fsm[];
-    const int NP = min(G, max(1, 4096 >> a.log2W));
-    float2 *buf = reinterpret_cast<float2 *>(fsm);                    // NP x W
-    P *stg = reinterpret_cast<P *>(fsm + sizeof(float2) * NP * a.W);  // [side][u][G]
-    __shared__ float pads[4 * G];
-    const int view = blockIdx.y, r0 = blockIdx.x * G;
-    const float *vsrc = a.src + (long long)view * a.src_vstride;
-    for (int g0 = 0; g0 < G; g0 += NP) {
-        if (threadIdx.x < 4 * NP) {
-            const int q = threadIdx.x >> 2, j = threadIdx.x & 3, r1 = r0 + g0 + q;
-            pads[threadIdx.x] = edge_mean(a, vsrc, j < 2 ? r1 : a.nv - 1 - r1, (j & 1) == 0);
+// Slot of point p.  Where p = i + q with i < d, d and 16 of which one divides the other, and q a
+// multiple of d, it is slot(i) + slot(q): the passes' slots are one address and constants.
+__host__ __device__ constexpr int slot(int p) { return p + (p >> 4); }
+
+// Row pairs (r, nv-1-r), r = G * blockIdx.x + g, g < G, of view blockIdx.y.
+template <int LOG2W, int G, bool GATHER>
+__global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) filter_kernel(const FilterArgs a) {
+    using F = Fft<LOG2W>;
+    constexpr int W = F::W, E = F::E, TPF = F::TPF, RL = F::RL, THREADS = TPF * G;
+    extern __shared__ __align__(16) float2 fsm[];
+    __shared__ float pads[G][4];
+    const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
+    const int r0 = blockIdx.x * G;
+    const int r1 = min(r0 + g, a.n_pairs - 1), r2 = a.nv - 1 - r1;  // pairs past the last repeat it, unstored
+    float2 *buf = fsm + g * F::PITCH;
+    // the threads of one transform meet without the rest of the CTA
+    auto meet = [&]() {
+        if constexpr (TPF <= 32) __syncwarp();
+        else if constexpr (G == 1) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(TPF) : "memory");
+    };
+
+    // samples t + m TPF of the padded rows
+    const long long view = blockIdx.y;
+    const float *p1 = a.src + view * a.src_vstride + (long long)r1 * a.src_pitch;
+    const float *p2 = a.src + view * a.src_vstride + (long long)r2 * a.src_pitch;
+    const float *w1 = a.cos ? a.cos + (long long)r1 * a.cos_pitch : nullptr;
+    const float *w2 = a.cos ? a.cos + (long long)r2 * a.cos_pitch : nullptr;
+    const int c0 = t - a.off;  // this thread's first column
+    float2 v[E];
+#pragma unroll
+    for (int m = 0; m < E; m++)
+        if ((unsigned)(c0 + m * TPF) < (unsigned)a.nu)
+            v[m] = make_float2(__ldg(p1 + c0 + m * TPF), __ldg(p2 + c0 + m * TPF));
+    if (a.cos) {
+#pragma unroll
+        for (int m = 0; m < E; m++)
+            if ((unsigned)(c0 + m * TPF) < (unsigned)a.nu)
+                v[m] = make_float2(v[m].x * __ldg(w1 + c0 + m * TPF), v[m].y * __ldg(w2 + c0 + m * TPF));
+    }
+    // the pads: means of the first and last pad_n weighted samples
+    for (int q = t; q < 4; q += TPF) {
+        const float *p = q < 2 ? p1 : p2, *w = q < 2 ? w1 : w2;
+        float s = 0.f;
+        for (int k = 0; k < a.pad_n; k++) {
+            const int c = (q & 1) ? a.nu - 1 - k : k;
+            float x = __ldg(p + c);
+            if (w) x *= __ldg(w + c);
+            s += x;
         }
-        __syncthreads();  // also ends the previous pairs' reads of buf
-        for (int k = threadIdx.x; k < (NP << a.log2W); k += blockDim.x) {
-            const int q = k >> a.log2W, c = (k & (a.W - 1)) - a.off;
-            const int r1 = r0 + g0 + q, r2 = a.nv - 1 - r1;
-            float x1, x2;
-            if (c < 0) {
-                x1 = pads[4 * q];
-                x2 = pads[4 * q + 2];
-            } else if (c >= a.nu) {
-                x1 = pads[4 * q + 1];
-                x2 = pads[4 * q + 3];
+        pads[g][q] = s / (float)a.pad_n;
+    }
+    meet();
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+        const int c = c0 + m * TPF;
+        if (c < 0) v[m] = make_float2(pads[g][0], pads[g][2]);
+        else if (c >= a.nu) v[m] = make_float2(pads[g][1], pads[g][3]);
+    }
+
+    // v[k] *= w_{n E}^(i k) (or its conjugate), i < n the thread's place in its block of a pass.
+    // plane: the pass's twiddles as float4 (k, k + 1) pairs, pair-major; gathered: entry i k of the
+    // pass's roots, which are every (W / n / E)-th of tw.
+    auto twiddle = [&](auto conj, const float2 *plane, int n, int i) {
+        constexpr bool CONJ = decltype(conj)::value;
+        if constexpr (GATHER) {
+#pragma unroll
+            for (int k = 1; k < E; k++) {
+                const int e = i * k * (TPF / n);  // < W
+                float2 w = __ldg(a.tw + (e & (W / 2 - 1)));
+                if (e >= W / 2) w = make_float2(-w.x, -w.y);
+                v[k] = cmul<CONJ>(v[k], w);
+            }
+        } else if constexpr (E >= 2) {
+            const float4 *q = reinterpret_cast<const float4 *>(plane) + i;
+#pragma unroll
+            for (int k = 0; k < E; k += 2) {
+                const float4 f = load_here(q + (k / 2) * n);
+                if (k) v[k] = cmul<CONJ>(v[k], make_float2(f.x, f.y));
+                v[k + 1] = cmul<CONJ>(v[k + 1], make_float2(f.z, f.w));
+            }
+        }
+    };
+    using Fwd = std::false_type;
+    using Inv = std::true_type;
+    float2 *outer = buf + slot(t);                               // points t + k TPF
+    float2 *middle = buf + slot((t / RL) * (E * RL)) + t % RL;  // points of the middle pass, RL apart
+    float2 *inner = buf + slot(t * E);                           // the last pass's run of points
+
+    dft<E, false>(v, 0);
+    if constexpr (TPF > 1) {
+        twiddle(Fwd{}, a.twp, TPF, t);
+#pragma unroll
+        for (int k = 0; k < E; k++) outer[slot(k * TPF)] = v[k];
+        meet();
+        if constexpr (F::MID) {
+#pragma unroll
+            for (int k = 0; k < E; k++) v[k] = middle[slot(k * RL)];
+            dft<E, false>(v, 0);
+            twiddle(Fwd{}, a.twp + W, RL, t % RL);
+#pragma unroll
+            for (int k = 0; k < E; k++) middle[slot(k * RL)] = v[k];
+            meet();
+        }
+#pragma unroll
+        for (int k = 0; k < E; k++) v[k] = inner[k];
+#pragma unroll
+        for (int b = 0; b < E; b += RL) dft<RL, false>(v, b);
+    }
+    if constexpr (E == 16) {  // four planes of float4
+        const float4 *h4 = reinterpret_cast<const float4 *>(a.hb) + t;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float4 h = __ldg(h4 + q * TPF);
+            v[4 * q] = make_float2(v[4 * q].x * h.x, v[4 * q].y * h.x);
+            v[4 * q + 1] = make_float2(v[4 * q + 1].x * h.y, v[4 * q + 1].y * h.y);
+            v[4 * q + 2] = make_float2(v[4 * q + 2].x * h.z, v[4 * q + 2].y * h.z);
+            v[4 * q + 3] = make_float2(v[4 * q + 3].x * h.w, v[4 * q + 3].y * h.w);
+        }
+    } else if constexpr (W > 1) {  // (a single sample is passed through)
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const float h = __ldg(a.hb + k);
+            v[k] = make_float2(v[k].x * h, v[k].y * h);
+        }
+    }
+    if constexpr (TPF > 1) {
+#pragma unroll
+        for (int b = 0; b < E; b += RL) dft<RL, true>(v, b);
+#pragma unroll
+        for (int k = 0; k < E; k++) inner[k] = v[k];
+        meet();
+        if constexpr (F::MID) {
+#pragma unroll
+            for (int k = 0; k < E; k++) v[k] = middle[slot(k * RL)];
+            twiddle(Inv{}, a.twp + W, RL, t % RL);
+            dft<E, true>(v, 0);
+#pragma unroll
+            for (int k = 0; k < E; k++) middle[slot(k * RL)] = v[k];
+            meet();
+        }
+#pragma unroll
+        for (int k = 0; k < E; k++) v[k] = outer[slot(k * TPF)];
+        twiddle(Inv{}, a.twp, TPF, t);
+    }
+    dft<E, true>(v, 0);
+
+    bool over = false;
+#pragma unroll
+    for (int k = 0; k < E; k++) v[k] = make_float2(v[k].x * a.out_scale, v[k].y * a.out_scale);
+    if (a.layout == FDK_LAYOUT_ROWS) {
+        // v[k] is sample t + k TPF: coalesced rows
+        const bool live = r0 + g < a.n_pairs;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const int u = t + k * TPF - a.off;
+            if (!live || u < 0 || u >= a.nu) continue;
+            const long long o1 = view * a.dst_vstride + (long long)r1 * a.dst_pitch + u;
+            const long long o2 = view * a.dst_vstride + (long long)r2 * a.dst_pitch + u;
+            if (a.half) {
+                over |= !(fabsf(v[k].x) <= 65504.f) || !(fabsf(v[k].y) <= 65504.f);
+                static_cast<__half *>(a.dst)[o1] = __float2half_rn(v[k].x);
+                if (r2 != r1) static_cast<__half *>(a.dst)[o2] = __float2half_rn(v[k].y);
             } else {
-                x1 = row_sample(a, vsrc, r1, c);
-                x2 = row_sample(a, vsrc, r2, c);
+                static_cast<float *>(a.dst)[o1] = v[k].x;
+                if (r2 != r1) static_cast<float *>(a.dst)[o2] = v[k].y;
             }
-            buf[(q << a.log2W) + fsw(k & (a.W - 1))] = make_float2(x1, x2);
+        }
+    } else {
+        // Columns: the G pairs' samples of one detector column are neighbours in the output, so they
+        // go through shared memory and out in runs of G.  Slot (u, g) is rotated within its column
+        // so that the 16 columns a half-warp writes fall into different banks.
+        constexpr int ROT = G >= 16 ? 1 : 16 / G;
+        __syncthreads();  // every transform of the CTA has read its last points
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const int u = t + k * TPF - a.off;
+            if (u >= 0 && u < a.nu) fsm[u * G + ((g + u / ROT) & (G - 1))] = v[k];
         }
         __syncthreads();
-        filter_fft(buf, a, NP);
-        for (int k = threadIdx.x; k < NP * a.nu; k += blockDim.x) {
-            const int q = k / a.nu, u = k - q * a.nu, g = g0 + q;
-            const float2 y = buf[(q << a.log2W) + fsw(a.off + u)];
-            const OUT o1 = to_out<OUT>(a, y.x), o2 = to_out<OUT>(a, y.y);
-            stg[u * G + g] = PairOf<OUT>::make(o1, o2);                     // element (u, r1)
-            stg[(a.nu + u) * G + (G - 1 - g)] = PairOf<OUT>::make(o2, o1);  // element (u, r2)
+        for (int i = threadIdx.x; i < a.nu * G; i += THREADS) {
+            const int u = i / G, q = i & (G - 1), ra = r0 + q, rb = a.nv - 1 - ra;
+            if (ra >= a.n_pairs) continue;
+            const float2 y = fsm[u * G + ((q + u / ROT) & (G - 1))];
+            if (a.half) over |= !(fabsf(y.x) <= 65504.f) || !(fabsf(y.y) <= 65504.f);
+            if (a.layout == FDK_LAYOUT_TRANSPOSED) {
+                const long long o = view * a.dst_vstride + (long long)u * a.dst_pitch;
+                if (a.half) {
+                    __half *d = static_cast<__half *>(a.dst) + o;
+                    d[ra] = __float2half_rn(y.x);
+                    if (rb != ra) d[rb] = __float2half_rn(y.y);
+                } else {
+                    float *d = static_cast<float *>(a.dst) + o;
+                    d[ra] = y.x;
+                    if (rb != ra) d[rb] = y.y;
+                }
+            } else {  // mirror pairs: element (u, v) = (row v, row nv-1-v)
+                const long long o = view * (a.dst_vstride / 2) + (long long)u * a.dst_pitch;
+                if (a.half) {
+                    __half2 *d = static_cast<__half2 *>(a.dst) + o;
+                    const __half x = __float2half_rn(y.x), z = __float2half_rn(y.y);
+                    if (a.pair_stores) {
+                        d[ra] = __halves2half2(x, z);
+                        d[rb] = __halves2half2(z, x);
+                    } else {
+                        __half *e = reinterpret_cast<__half *>(d);
+                        e[2 * ra] = x;
+                        e[2 * ra + 1] = z;
+                        e[2 * rb] = z;
+                        e[2 * rb + 1] = x;
+                    }
+                } else {
+                    float2 *d = static_cast<float2 *>(a.dst) + o;
+                    if (a.pair_stores) {
+                        d[ra] = y;
+                        d[rb] = make_float2(y.y, y.x);
+                    } else {
+                        float *e = reinterpret_cast<float *>(d);
+                        e[2 * ra] = y.x;
+                        e[2 * ra + 1] = y.y;
+                        e[2 * rb] = y.y;
+                        e[2 * rb + 1] = y.x;
+                    }
+                }
+            }
         }
     }
-    __syncthreads();
-    // side 0: elements v = r0 .. r0+G-1; side 1: v = nv-r0-G .. nv-1-r0 (the mirrors, ascending)
-    P *dst = reinterpret_cast<P *>(a.dst) + (long long)view * (a.dst_vstride / 2);
-    for (int i = threadIdx.x; i < 2 * a.nu; i += blockDim.x) {
-        const int side = i >= a.nu, u = side ? i - a.nu : i;
-        const int v0 = side ? a.nv - r0 - G : r0;
-        *reinterpret_cast<uint4 *>(dst + (long long)u * a.dst_pitch + v0) = *reinterpret_cast<const uint4 *>(stg + i * G);
-    }
+    if (a.overflow && over) atomicOr(a.overflow, 1u);
+}
+
+// f(std::integral_constant<int, log2W>) for the run-time length
+template <int L = 0, typename Fn>
+static int with_length(int log2W, Fn f) {
+    if constexpr (L > 12) return fail(FDK_ERR_INVALID_ARG, "filter length 2^%d", log2W);
+    else return log2W == L ? f(std::integral_constant<int, L>{}) : with_length<L + 1>(log2W, f);
 }
 
 int FilterTables::create(const double *H, int W_) {
     W = W_;
     log2W = 0;
     while ((1 << log2W) < W) log2W++;
-    std::vector<float2> t(W / 2);
-    for (int k = 0; k < W / 2; k++) {
-        const double ang = -2.0 * 3.14159265358979323846 * k / W;
-        t[k] = make_float2((float)std::cos(ang), (float)std::sin(ang));
-    }
+    auto root = [&](long long k, int n) {  // exp(-2 pi i k / n)
+        const double ang = -2.0 * 3.14159265358979323846 * (double)k / n;
+        return make_float2((float)std::cos(ang), (float)std::sin(ang));
+    };
+    std::vector<float2> t(std::max(1, W / 2));
+    for (int k = 0; k < W / 2; k++) t[k] = root(k, W);
     std::vector<float> h(W);
-    for (int p = 0; p < W; p++) {
-        int r = 0;
-        for (int b = 0; b < log2W; b++)
-            if (p & (1 << b)) r |= 1 << (log2W - 1 - b);
-        h[p] = (float)(H[r] / W);
-    }
-    // the group lists of every pass, in filter_fft's order (DIF passes, then DIT passes); each
-    // group's list padded to 2^ns entries and stored as 2^(ns-1) planes of pairs (pair k of
-    // group g at (k * groups + g) * 2)
+    for (int i = 0; i < W; i++) h[i] = (float)(H[filter_response_frequency(i, W)] / W);
+    // the passes' twiddles: w^(i k) for k < E as E / 2 planes of pairs, i fastest: first pass (n = W / E
+    // places, W-th roots), then the middle pass (n = W / 256 places, W/16-th roots)
     std::vector<float2> pt;
-    auto put_pass = [&](int groups, int GS, const std::vector<float2> &lists) {  // lists: groups x GS
-        for (int k = 0; k < GS / 2; k++)
-            for (int g = 0; g < groups; g++) {
-                pt.push_back(lists[(size_t)g * GS + 2 * k]);
-                pt.push_back(lists[(size_t)g * GS + 2 * k + 1]);
+    auto put = [&](int n, int E) {
+        for (int k = 0; k < E; k += 2)
+            for (int i = 0; i < n; i++) {
+                pt.push_back(root((long long)i * k, n * E));
+                pt.push_back(root((long long)i * (k + 1), n * E));
             }
     };
-    for (int s0 = 0; s0 < log2W; s0 += 3) {
-        const int ns = std::min(3, log2W - s0), GS = 1 << ns, low = log2W - s0 - ns;
-        std::vector<float2> lists((size_t)GS << low, make_float2(0.f, 0.f));
-        for (int g = 0; g < (1 << low); g++) {
-            int e = 0;
-            for (int st = 0; st < ns; st++)
-                for (int jt = 0; jt < (GS >> (st + 1)); jt++)
-                    lists[(size_t)g * GS + e++] = t[(g + (jt << low)) << (s0 + st)];
-        }
-        put_pass(1 << low, GS, lists);
-    }
-    for (int b0 = 0; b0 < log2W; b0 += 3) {
-        const int ns = std::min(3, log2W - b0), GS = 1 << ns;
-        std::vector<float2> lists((size_t)GS << b0, make_float2(0.f, 0.f));
-        for (int g = 0; g < (1 << b0); g++) {
-            int e = 0;
-            for (int st = 0; st < ns; st++)
-                for (int jt = 0; jt < (1 << st); jt++)
-                    lists[(size_t)g * GS + e++] = t[(g + (jt << b0)) << (log2W - 1 - b0 - st)];
-        }
-        put_pass(1 << b0, GS, lists);
-    }
-    FDK_CUDA(cudaMalloc(&tw, sizeof(float2) * (W / 2)));
+    if (W > 16) put(W / 16, 16);
+    if (W > 256) put(W / 256, 16);
+    if (pt.empty()) pt.push_back(make_float2(1.f, 0.f));
+    FDK_CUDA(cudaMalloc(&tw, sizeof(float2) * t.size()));
     FDK_CUDA(cudaMalloc(&hb, sizeof(float) * W));
     FDK_CUDA(cudaMalloc(&twp, sizeof(float2) * pt.size()));
     SetupStream ss;
     FDK_TRY(ss.open());
-    FDK_CUDA(cudaMemcpyAsync(tw, t.data(), sizeof(float2) * (W / 2), cudaMemcpyHostToDevice, ss.st));
+    FDK_CUDA(cudaMemcpyAsync(tw, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice, ss.st));
     FDK_CUDA(cudaMemcpyAsync(hb, h.data(), sizeof(float) * W, cudaMemcpyHostToDevice, ss.st));
     FDK_CUDA(cudaMemcpyAsync(twp, pt.data(), sizeof(float2) * pt.size(), cudaMemcpyHostToDevice, ss.st));
     return ss.finish("filter tables");
@@ -416,56 +423,37 @@ void FilterTables::release() {
     hb = nullptr;
 }
 
-template <typename OUT, int G>
-static int launch_mirror(const FilterArgs &a, int n_views, cudaStream_t st) {
-    using P = typename PairOf<OUT>::T;
-    const int np = std::min(G, std::max(1, 4096 >> a.log2W));
-    const size_t smem = sizeof(float2) * np * a.W + 2 * sizeof(P) * G * a.nu;
+template <int LOG2W, int G, bool GATHER>
+static int launch_group(const FilterArgs &a, int n_views, cudaStream_t st) {
+    using F = Fft<LOG2W>;
+    const int smem = (int)sizeof(float2) * std::max(F::TPF > 1 ? F::PITCH * G : 0, a.layout != FDK_LAYOUT_ROWS ? a.nu * G : 0);
     // per device and size, and needed at 48 KB too (the kernel also has static shared memory):
     // cheap, so set on every launch
-    FDK_CUDA(cudaFuncSetAttribute(filter_mirror_kernel<OUT, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    filter_mirror_kernel<OUT, G><<<dim3(a.nv / (2 * G), n_views), 512, smem, st>>>(a);
+    if (smem > 40 * 1024)
+        FDK_CUDA(cudaFuncSetAttribute(filter_kernel<LOG2W, G, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    filter_kernel<LOG2W, G, GATHER><<<dim3((unsigned)ceil_div(a.n_pairs, G), n_views), F::TPF * G, smem, st>>>(a);
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
 }
 
-static int launch_filter(const FilterArgs &a, int n_views, int layout, int dtype, cudaStream_t st) {
-    if (layout == FDK_LAYOUT_MIRROR) {
-        // grouped kernel when G pairs tile the rows and every 16-byte store is aligned
-        const int G = dtype == FDK_DTYPE_F32 ? 2 : 4;
-        const size_t pair = dtype == FDK_DTYPE_F32 ? 8 : 4;
-        const size_t smem = sizeof(float2) * std::max(a.W, std::min(G, 4096 / a.W) * a.W) + 2 * pair * G * a.nu;
-        if (a.nv % (2 * G) == 0 && ((uintptr_t)a.dst & 15) == 0 && (a.dst_pitch * pair) % 16 == 0 &&
-            (a.dst_vstride * (pair / 2)) % 16 == 0 && smem <= 200 * 1024) {
-            if (dtype == FDK_DTYPE_F32) return launch_mirror<float, 2>(a, n_views, st);
-            return launch_mirror<__half, 4>(a, n_views, st);
-        }
-    }
-    const dim3 grid((a.nv + 1) / 2, n_views);
-    const size_t smem = sizeof(float2) * a.W;
-    if (smem + sizeof(float) * 4 > 48 * 1024) {  // dynamic + static (pads) above the default limit
-        // opt in to more than 48 KB of dynamic shared memory (per device: set on every launch)
-        FDK_CUDA(cudaFuncSetAttribute(filter_rows_kernel<FDK_LAYOUT_ROWS, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        FDK_CUDA(cudaFuncSetAttribute(filter_rows_kernel<FDK_LAYOUT_TRANSPOSED, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        FDK_CUDA(cudaFuncSetAttribute(filter_rows_kernel<FDK_LAYOUT_MIRROR, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        FDK_CUDA(cudaFuncSetAttribute(filter_rows_kernel<FDK_LAYOUT_ROWS, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        FDK_CUDA(cudaFuncSetAttribute(filter_rows_kernel<FDK_LAYOUT_TRANSPOSED, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        FDK_CUDA(cudaFuncSetAttribute(filter_rows_kernel<FDK_LAYOUT_MIRROR, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    }
-#define FDK_LAUNCH(L, T) filter_rows_kernel<L, T><<<grid, 256, smem, st>>>(a)
-    if (dtype == FDK_DTYPE_F32) {
-        if (layout == FDK_LAYOUT_ROWS) FDK_LAUNCH(FDK_LAYOUT_ROWS, float);
-        else if (layout == FDK_LAYOUT_TRANSPOSED) FDK_LAUNCH(FDK_LAYOUT_TRANSPOSED, float);
-        else FDK_LAUNCH(FDK_LAYOUT_MIRROR, float);
-    } else {
-        if (layout == FDK_LAYOUT_ROWS) FDK_LAUNCH(FDK_LAYOUT_ROWS, __half);
-        else if (layout == FDK_LAYOUT_TRANSPOSED) FDK_LAUNCH(FDK_LAYOUT_TRANSPOSED, __half);
-        else FDK_LAUNCH(FDK_LAYOUT_MIRROR, __half);
-    }
-#undef FDK_LAUNCH
-    FDK_CUDA(cudaGetLastError());
-    return FDK_OK;
+// Transforms per CTA.  The column layouts write runs of G elements, so they take the largest CTA that
+// still fills the SM's 1024 resident threads evenly: 1024 threads at W = 4096 (G = 4, 32-byte runs of
+// FP32 pairs: 971 against 1139 us at 512 threads and G = 2, 32 views of 2048^2 to MIRROR FP32), 512
+// below, where G is 4 or more anyway (1500 x 1000 to MIRROR FP16 at 512 / 256 threads: 226 / 236 us).
+// ROWS stores are coalesced at any G, and smaller CTAs overlap each other's loads and transforms
+// better (48 views of 1536 x 1024 at 512 / 256 threads: 285 / 260 us).  A call whose CTAs would
+// not give every SM two takes the smallest group of whole warps, for more CTAs.
+static int launch_filter(const FilterArgs &a, int log2W, int n_views, cudaStream_t st) {
+    return with_length(log2W, [&](auto l) {
+        constexpr int L = decltype(l)::value, TPF = Fft<L>::TPF;
+        constexpr int cols = std::min((L == 12 ? 1024 : 512) / TPF, 64), rows = std::min(256 / TPF, 64);
+        constexpr int least = std::max(1, std::min(64 / TPF, 16));
+        const int g = a.layout == FDK_LAYOUT_ROWS ? rows : cols;
+        if (!a.twp) return launch_group<L, least, true>(a, n_views, st);
+        if (ceil_div(a.n_pairs, g) * n_views < 2 * 148) return launch_group<L, least, false>(a, n_views, st);
+        if (g == rows) return launch_group<L, rows, false>(a, n_views, st);
+        return launch_group<L, cols, false>(a, n_views, st);
+    });
 }
 
 // Shared by the FilterEngine handle, the cuFFT-plugin entry points and the reconstructor.
@@ -482,18 +470,20 @@ int filter_views(const float *src, int src_pitch, long long src_vstride, void *d
     a.hb = t.hb;
     a.nu = nu;
     a.nv = nv;
-    a.W = t.W;
-    a.log2W = t.log2W;
     a.off = (t.W - nu) >> 1;
     a.pad_n = pad_n;
+    a.n_pairs = (nv + 1) / 2;
     a.src_pitch = src_pitch;
     a.dst_pitch = dst_pitch;
     a.cos_pitch = cos_pitch;
     a.src_vstride = src_vstride;
     a.dst_vstride = dst_vstride;
+    a.layout = layout;
+    a.half = dtype == FDK_DTYPE_F16;
+    a.pair_stores = ((uintptr_t)dst & (a.half ? 3 : 7)) == 0 && dst_vstride % 2 == 0;
     a.out_scale = out_scale;
     a.overflow = overflow;
-    return launch_filter(a, n_views, layout, dtype, st);
+    return launch_filter(a, t.log2W, n_views, st);
 }
 
 static int check_filter_dims(int64_t nu, int64_t nv, int64_t W, int pad) {

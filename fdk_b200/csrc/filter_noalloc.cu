@@ -2,7 +2,7 @@
 // without any device allocation.
 //
 // fdk_filter_row_real32 allocates two small device tables per call (the FFT twiddles and the
-// bit-reversed, 1/W-scaled response) and frees them again.  Some callers cannot allocate device
+// reordered, 1/W-scaled response) and frees them again.  Some callers cannot allocate device
 // memory at that point: applications that reserve the whole device budget up front and hand
 // out memory themselves, and processing loops that must not call cudaMalloc/cudaFree because
 // those calls can synchronise the device and stall every other stream.  For them this entry
@@ -32,19 +32,20 @@ namespace fdk {
 
 constexpr int kNoAllocMaxW = 4096;
 
-// W/2 float2 twiddles followed by W floats of the bit-reversed response: 4096 * 8 bytes.
+// W/2 float2 twiddles followed by W floats of the reordered response: 4096 * 8 bytes.
 static __device__ __align__(256) float2 g_filter_scratch[kNoAllocMaxW];
 
-// tw[k] = exp(-2 pi i k / W) (FP64 sincospi, rounded), hb[p] = H[bitrev(p)] / W.
-__global__ void build_filter_tables_kernel(const float *__restrict__ H, int W, int log2W, float2 *tw, float *hb) {
+// tw[k] = exp(-2 pi i k / W) (FP64 sincospi, rounded), hb[i] = H / W in the order of the transform's
+// registers (filter_response_frequency).
+__global__ void build_filter_tables_kernel(const float *__restrict__ H, int W, float2 *tw, float *hb) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < W; k += gridDim.x * blockDim.x) {
         if (k < W / 2) {
             double s, c;
             sincospi(-2.0 * (double)k / (double)W, &s, &c);
             tw[k] = make_float2((float)c, (float)s);
         }
-        const int r = (int)(__brev((unsigned)k) >> (32 - log2W));
-        hb[k] = H[r] / (float)W;
+        const int f = filter_response_frequency(k, W);
+        hb[k] = H[f] / (float)W;
     }
 }
 
@@ -84,7 +85,7 @@ extern "C" int fdk_filter_row_real32_noalloc(const fdk_dataref *src, fdk_dataref
     while ((1 << t.log2W) < W) t.log2W++;
     t.tw = scratch;
     t.hb = reinterpret_cast<float *>(scratch + W / 2);
-    build_filter_tables_kernel<<<(W + 255) / 256, 256, 0, cudaStreamLegacy>>>(filter->data, W, t.log2W, t.tw, t.hb);
+    build_filter_tables_kernel<<<(W + 255) / 256, 256, 0, cudaStreamLegacy>>>(filter->data, W, t.tw, t.hb);
     FDK_CUDA(cudaGetLastError());
     FDK_TRY(filter_views(src->data, src->pitch, (long long)src->pitch * src->height, dst->data, dst->pitch,
                          (long long)dst->pitch * dst->height, nullptr, 0, t, src->width, src->height, 3, src->depth,

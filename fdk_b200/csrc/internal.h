@@ -12,13 +12,24 @@ void projection_matrix(const fdk_geometry &g, double a, double *m);
 // Device tables of one filter length (filter.cu).
 struct FilterTables {
     int W = 0, log2W = 0;
-    float2 *tw = nullptr;
-    float2 *twp = nullptr;  // per FFT pass and group, the group's twiddles (optional)
-    float *hb = nullptr;
+    float2 *tw = nullptr;   // W/2 twiddles exp(-2 pi i k / W)
+    float2 *twp = nullptr;  // the FFT passes' twiddles in the order the threads read them (optional)
+    float *hb = nullptr;    // H / W, entry i at frequency filter_response_frequency(i, W)
     // the copies go through a private set-up stream that the call waits for (bounded)
     int create(const double *H, int W_);
     void release();
 };
+
+// Frequency of entry i of FilterTables::hb.  The row filter's transform leaves thread t of W / 16 with
+// 16 points p = 16 t + k in digit-reversed order (radices 16, 16 for W > 256, then the rest); the
+// table holds them as four planes of four points of every thread.  W < 32 is one thread's.
+__host__ __device__ inline int filter_response_frequency(int i, int W) {
+    if (W < 32) return i;
+    const int threads = W / 16, p = 16 * (i / 4 % threads) + 4 * (i / (4 * threads)) + i % 4;
+    if (W <= 256) return p / threads + 16 * (p % threads);
+    const int last = W / 256;
+    return p / threads + 16 * (p % threads / last) + 256 * (p % last);
+}
 
 // Fused cosine weight + pad + ramp filter + crop + layout store (filter.cu).
 int filter_views(const float *src, int src_pitch, long long src_vstride, void *dst, int dst_pitch,

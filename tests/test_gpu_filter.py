@@ -103,3 +103,32 @@ def test_mirror_kernel_at_the_48k_shared_memory_boundary(nu, nv):
     assert np.array_equal(m[..., 0], t) and np.array_equal(m[..., 1], t[:, :, ::-1])
     hh = h.float().cpu().numpy() / scale
     assert max_rel(hh[..., 0], t) <= 1e-3
+
+
+@pytest.mark.parametrize("nu", [1, 3, 6, 15, 16, 31, 40, 64, 127, 128, 255, 256, 511, 600, 1023, 1100, 2047, 2048])
+@pytest.mark.parametrize("nv,views", [(1, 1), (7, 3), (37, 40)])
+def test_every_length_and_group(nu, nv, views):
+    """Every transform length (W = 2 .. 4096), one row (its own mirror), an odd row count, and few and many
+    transforms per CTA, in every layout against the FP64 oracle.  Tolerances: those of the tests above (FP32
+    transforms of up to 12 index bits each way; FP16 outputs round to 2^-11)."""
+    import torch
+
+    pad = min(4, nu)
+    rng = np.random.default_rng(nu * 100 + nv)
+    src = (rng.standard_normal((views, nv, nu)) + 2.0).astype(np.float32)
+    cos = rng.uniform(0.9, 1.0, (nv, nu)).astype(np.float32)
+    H = O.filter_design("hann", nu)
+    want = np.stack([O.filter_view(v, H, cos, pad_n=pad, transpose=True) for v in src])
+    eng = F.FilterEngine(cos, H.astype(np.float32), pad_edge=pad)
+    d = torch.from_numpy(src).cuda()
+    for layout, shape in ((F.LAYOUT_ROWS, (nv, nu)), (F.LAYOUT_TRANSPOSED, (nu, nv)), (F.LAYOUT_MIRROR, (nu, nv, 2))):
+        for dtype, torch_dtype, tol in ((F.DTYPE_F32, torch.float32, 3e-6), (F.DTYPE_F16, torch.float16, 1e-3)):
+            out = torch.full((views, *shape), 7.0, dtype=torch_dtype, device="cuda")
+            eng.run_device(d.data_ptr(), out.data_ptr(), views, layout, dtype)
+            got = out.double().cpu().numpy()
+            if layout == F.LAYOUT_ROWS:
+                got = got.transpose(0, 2, 1)
+            if layout == F.LAYOUT_MIRROR:
+                assert max_rel(got[..., 1], want[:, :, ::-1]) <= tol
+                got = got[..., 0]
+            assert max_rel(got, want) <= tol, (layout, dtype)
