@@ -187,3 +187,69 @@ def test_field_of_view_weights_beat_plain_fdk_inside_the_field_of_view():
     print(ev)
     assert ev["learned_better_frac"] == 1.0
     assert ev["fov_mse_reduction"] >= 0.17, ev
+
+
+@pytest.mark.parametrize("nx,ny,nz,nu,nv,views", [
+    (40, 40, 40, 48, 32, 3), (33, 50, 21, 70, 33, 2), (64, 64, 64, 5, 7, 1), (17, 19, 23, 40, 1, 2),
+    (30, 34, 1, 64, 65, 2), (2, 3, 64, 31, 31, 4)])
+def test_forward_projector_of_a_linear_volume(nx, ny, nz, nu, nv, views):
+    """A volume linear in the voxel indices is reproduced by trilinear samples, so every pixel is known in FP64:
+    the sum over the ray's samples.  Odd sizes, one row, one slice, few rays.  Tolerance: FP32 positions are off by about 1e-4 of the volume's extent; a ray
+    whose length is a whole number of steps to 1e-2 may take one sample more or less."""
+    import torch
+
+    p = small_param(64, nu, nv, views)
+    p.nx, p.ny, p.nz = nx, ny, nz
+    p.dx = p.dy = p.dz = 256.0 / max(nx, ny, nz)
+    z, y, x = (torch.arange(n, device="cuda", dtype=torch.float32) for n in (nz, ny, nx))
+    cx, cy, cz, c0 = 1.0 / nx, 2.0 / ny, 3.0 / nz, 1.0
+    vol = (c0 + cx * x[None, None, :] + cy * y[None, :, None] + cz * z[:, None, None]).contiguous()
+    out = torch.full((views, nv, nu), -1.0, device="cuda")
+    g = p.to_c()
+    check(lib().fdk_forward_project(C.byref(g), vol.data_ptr(), 0, views, out.data_ptr(), None))
+    got = out.double().cpu().numpy()
+    u = (np.arange(nu) - (nu - 1) / 2) * p.du
+    v = ((nv - 1) / 2 - np.arange(nv)) * p.dv
+    step = p.dx
+    half = (np.array([nx, ny, nz]) - 1) / 2 * step
+    for i, a in enumerate(p.angles):
+        c, s = np.cos(-a), np.sin(-a)
+        far = p.SID - p.SOD
+        o = np.array([p.SOD * s, -p.SOD * c, 0.0])
+        d = np.stack([np.broadcast_to(u * c - far * s, (nv, nu)), np.broadcast_to(u * s + far * c, (nv, nu)),
+                      np.broadcast_to(v[:, None], (nv, nu))], -1) - o
+        d /= np.linalg.norm(d, axis=-1, keepdims=True)
+        with np.errstate(divide="ignore", invalid="ignore"):
+            lo, hi = (-half - o) / d, (half - o) / d
+        near, end = np.fmax.reduce(np.fmin(lo, hi), -1), np.fmin.reduce(np.fmax(lo, hi), -1)
+        length = np.maximum(end - near, 0) / step
+        k = np.ceil(length)
+        t = near + (k - 1) / 2 * step  # the samples' mean position
+        pos = [o[0] / step + (nx - 1) / 2 + d[..., 0] / step * t, (ny - 1) / 2 - (o[1] + d[..., 1] * t) / step,
+               (nz - 1) / 2 - (o[2] + d[..., 2] * t) / step]
+        want = np.where(k > 0, k * step * (c0 + cx * pos[0] + cy * pos[1] + cz * pos[2]), 0)
+        slack = 7.0 * step * (np.abs(length - np.round(length)) < 1e-2)  # the largest voxel, one sample
+        off = np.abs(got[i] - want)
+        assert (off <= 2e-4 * max(np.abs(want).max(), step) + slack).all(), off.max()
+
+
+@pytest.mark.parametrize("nx,ny,nz,nu,nv", [(50, 50, 50, 65, 65), (45, 60, 33, 120, 35), (1030, 1030, 1030, 2070, 2070)])
+def test_forward_projector_routes_agree(nx, ny, nz, nu, nv):
+    """One view here has too few rays for the reordered copy of the volume and reads the volume as it is, two
+    views read the copy (through 64-bit offsets above 2^30 voxels): the same arithmetic, so the same bits."""
+    import torch
+
+    p = small_param(64, nu, nv, 2)
+    p.nx, p.ny, p.nz = nx, ny, nz
+    p.dx = p.dy = p.dz = 256.0 / max(nx, ny, nz)
+    least = (2 if nx < 1000 else 8) * nx * ny  # rays that take the copy
+    assert nu * nv < least <= 2 * nu * nv
+    gen = torch.Generator(device="cuda").manual_seed(nx)
+    vol = torch.rand((nz, ny, nx), device="cuda", generator=gen)
+    both, one = torch.empty((2, nv, nu), device="cuda"), torch.empty((2, nv, nu), device="cuda")
+    g = p.to_c()
+    check(lib().fdk_forward_project(C.byref(g), vol.data_ptr(), 0, 2, both.data_ptr(), None))
+    for i in range(2):
+        check(lib().fdk_forward_project(C.byref(g), vol.data_ptr(), i, 1, one[i].data_ptr(), None))
+    assert torch.equal(both, one)
+    assert float(both.abs().max()) > 0
