@@ -35,20 +35,6 @@ constexpr int kNoAllocMaxW = 4096;
 // W/2 float2 twiddles followed by W floats of the reordered response: 4096 * 8 bytes.
 static __device__ __align__(256) float2 g_filter_scratch[kNoAllocMaxW];
 
-// tw[k] = exp(-2 pi i k / W) (FP64 sincospi, rounded), hb[i] = H / W in the order of the transform's
-// registers (filter_response_frequency).
-__global__ void build_filter_tables_kernel(const float *__restrict__ H, int W, float2 *tw, float *hb) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < W; k += gridDim.x * blockDim.x) {
-        if (k < W / 2) {
-            double s, c;
-            sincospi(-2.0 * (double)k / (double)W, &s, &c);
-            tw[k] = make_float2((float)c, (float)s);
-        }
-        const int f = filter_response_frequency(k, W);
-        hb[k] = H[f] / (float)W;
-    }
-}
-
 // The array's device address on the current device.  A host-side lookup, repeated per call.
 static int scratch_address(float2 **out) {
     void *p = nullptr;
@@ -85,8 +71,7 @@ extern "C" int fdk_filter_row_real32_noalloc(const fdk_dataref *src, fdk_dataref
     while ((1 << t.log2W) < W) t.log2W++;
     t.tw = scratch;
     t.hb = reinterpret_cast<float *>(scratch + W / 2);
-    build_filter_tables_kernel<<<(W + 255) / 256, 256, 0, cudaStreamLegacy>>>(filter->data, W, t.tw, t.hb);
-    FDK_CUDA(cudaGetLastError());
+    FDK_TRY(filter_tables_on_device(filter->data, t, cudaStreamLegacy));
     FDK_TRY(filter_views(src->data, src->pitch, (long long)src->pitch * src->height, dst->data, dst->pitch,
                          (long long)dst->pitch * dst->height, nullptr, 0, t, src->width, src->height, 3, src->depth,
                          FDK_LAYOUT_ROWS, FDK_DTYPE_F32, cudaStreamLegacy));

@@ -20,6 +20,10 @@ struct FilterTables {
     void release();
 };
 
+// Fill t's device tables (tw and twp where not null, and hb) for response H (device, W taps) on st
+// (filter.cu).
+int filter_tables_on_device(const float *H, const FilterTables &t, cudaStream_t st);
+
 // Frequency of entry i of FilterTables::hb.  The row filter's transform leaves thread t of W / 16 with
 // 16 points p = 16 t + k in digit-reversed order (radices 16, 16 for W > 256, then the rest); the
 // table holds them as four planes of four points of every thread.  W < 32 is one thread's.
