@@ -8,13 +8,17 @@
 // inverse transform.  Pairing r with nv-1-r is what lets one CTA emit the backprojection's
 // mirror-pair layout directly.
 //
-// FFT: W / 16 threads hold the W points of a row pair in registers, 16 each, and run at most three
-// passes a direction (W = 16 x 16 x W/256; 4096 = 16^3), a radix-16 transform in registers each.
+// FFT: radix-2 decimation in frequency (natural -> bit-reversed order), multiply by H, radix-2
+// decimation in time back.  W / 16 threads hold the W points of a row pair in registers, 16 each, and
+// run the stages four at a time: the 16 points that differ in four adjacent index bits form a closed
+// group (W = 16 x 16 x W/256, 4096 = 16^3).
 // The samples go from global memory straight into the first pass's registers and from the last
 // pass's registers out again, the spectrum is multiplied by H between the forward and the inverse
 // half of the innermost pass, and so a row pair crosses shared memory four times in all.  Bound:
 // shared-memory wavefronts and FP32 issue about equally (per 512 points and warp some 460
-// wavefronts and 1100 FP32 instructions at W = 4096).
+// wavefronts and 1200 FP32 instructions at W = 4096).  Plain butterflies cost an eighth more
+// arithmetic than radix-16 ones with their constants folded (32 views of 2048^2 to MIRROR FP32:
+// 997 against 973 us) and keep the outputs, bit for bit, those of a stage-by-stage transform.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -47,93 +51,76 @@ struct FilterArgs {
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-// a * w, or a * conj(w)
+// a * w, or a * conj(w): one product of each sum rounded, the other fused, written out so that every
+// place rounds alike
 template <bool CONJ>
 __device__ __forceinline__ float2 cmul(float2 a, float2 w) {
-    if (CONJ) return make_float2(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
-    return make_float2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+    if (CONJ) return make_float2(__fmaf_rn(a.x, w.x, __fmul_rn(a.y, w.y)), __fmaf_rn(a.y, w.x, -__fmul_rn(a.x, w.y)));
+    return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)), __fmaf_rn(a.x, w.y, __fmul_rn(a.y, w.x)));
 }
 
 // A table load that stays where it is written.  The forward and the inverse half read the same
 // twiddles; as plain read-only loads the compiler merges the two and keeps 32 to 64 registers alive
 // from one half to the other, as spills to local memory (300 bytes a thread at W = 4096, which
 // missed L1 and made two thirds of the kernel's L2 traffic: 1469 against 1139 us for 32 views of
-// 2048^2 to MIRROR FP32, before the CTA size was chosen).
+// 2048^2 to MIRROR FP32, with radix-16 butterflies and 512-thread CTAs).
 __device__ __forceinline__ float4 load_here(const float4 *p) {
     float4 f;
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(p) : "memory");
     return f;
 }
 
-// 4-point transform of v[b], v[b + s], v[b + 2s], v[b + 3s] in place, exp(-2 pi i / 4) or, INV, its conjugate
-template <bool INV, int N>
-__device__ __forceinline__ void dft4(float2 (&v)[N], int b, int s) {
-    const float2 t0 = cadd(v[b], v[b + 2 * s]), t1 = csub(v[b], v[b + 2 * s]);
-    const float2 t2 = cadd(v[b + s], v[b + 3 * s]), t3 = csub(v[b + s], v[b + 3 * s]);
-    const float2 r = INV ? make_float2(-t3.y, t3.x) : make_float2(t3.y, -t3.x);  // +-i t3
-    v[b] = cadd(t0, t2);
-    v[b + s] = cadd(t1, r);
-    v[b + 2 * s] = csub(t0, t2);
-    v[b + 3 * s] = csub(t1, r);
-}
-
-// R-point transform of v[b .. b + R-1], natural order in and out (the final reordering is a renaming
-// of registers).
-template <int R, bool INV, int N>
-__device__ __forceinline__ void dft(float2 (&v)[N], int b) {
-    constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508977f, h = 0.70710678118654752f;
-    if constexpr (R == 2) {
-        const float2 x = v[b], y = v[b + 1];
-        v[b] = cadd(x, y);
-        v[b + 1] = csub(x, y);
-    } else if constexpr (R == 4) {
-        dft4<INV>(v, b, 1);
-    } else if constexpr (R == 8) {  // 4 x 2
-        dft4<INV>(v, b, 2);
-        dft4<INV>(v, b + 1, 2);
-        v[b + 3] = cmul<INV>(v[b + 3], make_float2(h, -h));
-        v[b + 5] = INV ? make_float2(-v[b + 5].y, v[b + 5].x) : make_float2(v[b + 5].y, -v[b + 5].x);
-        v[b + 7] = cmul<INV>(v[b + 7], make_float2(-h, -h));
-        float2 o[8];
+// Stages in registers.  A group of R points has R/2 twiddles in its first decimation-in-frequency
+// stage, then R/4, and so on: entry j of the stage of half-width h serves the butterflies j mod h.  `w(h, j)`
+// gives it; decimation in time runs the same stages backwards with the conjugates.
+template <int R, int N, typename Tw>
+__device__ __forceinline__ void dif(float2 (&v)[N], int b, Tw w) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            o[k] = cadd(v[b + 2 * k], v[b + 2 * k + 1]);
-            o[k + 4] = csub(v[b + 2 * k], v[b + 2 * k + 1]);
+    for (int h = R / 2; h; h >>= 1)
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            if (j & h) continue;
+            const float2 x = v[b + j], y = v[b + j + h];
+            v[b + j] = cadd(x, y);
+            v[b + j + h] = w(std::false_type{}, csub(x, y), h, j & (h - 1));
         }
-#pragma unroll
-        for (int k = 0; k < 8; k++) v[b + k] = o[k];
-    } else if constexpr (R == 16) {  // 4 x 4
-#pragma unroll
-        for (int q = 0; q < 4; q++) dft4<INV>(v, b + q, 4);
-        // v[b + q + 4 k] *= w16^(q k)
-        v[b + 5] = cmul<INV>(v[b + 5], make_float2(c1, -s1));
-        v[b + 6] = cmul<INV>(v[b + 6], make_float2(h, -h));
-        v[b + 7] = cmul<INV>(v[b + 7], make_float2(s1, -c1));
-        v[b + 9] = cmul<INV>(v[b + 9], make_float2(h, -h));
-        v[b + 10] = INV ? make_float2(-v[b + 10].y, v[b + 10].x) : make_float2(v[b + 10].y, -v[b + 10].x);
-        v[b + 11] = cmul<INV>(v[b + 11], make_float2(-h, -h));
-        v[b + 13] = cmul<INV>(v[b + 13], make_float2(s1, -c1));
-        v[b + 14] = cmul<INV>(v[b + 14], make_float2(-h, -h));
-        v[b + 15] = cmul<INV>(v[b + 15], make_float2(-c1, s1));
-#pragma unroll
-        for (int k = 0; k < 4; k++) dft4<INV>(v, b + 4 * k, 1);
-        float2 o[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) o[k] = v[b + 4 * (k & 3) + (k >> 2)];
-#pragma unroll
-        for (int k = 0; k < 16; k++) v[b + k] = o[k];
-    }
 }
+template <int R, int N, typename Tw>
+__device__ __forceinline__ void dit(float2 (&v)[N], int b, Tw w) {
+#pragma unroll
+    for (int h = 1; h < R; h <<= 1)
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            if (j & h) continue;
+            const float2 x = v[b + j], u = w(std::true_type{}, v[b + j + h], h, j & (h - 1));
+            v[b + j] = cadd(x, u);
+            v[b + j + h] = csub(x, u);
+        }
+}
+// The stages of the last bits (contiguous points): twiddles exp(-2 pi i j / 2h), constants.
+struct Roots {
+    template <typename Conj>
+    __device__ __forceinline__ float2 operator()(Conj, float2 a, int h, int j) const {
+        constexpr float c[8] = {1.f, 0.92387953251128674f, 0.70710678118654752f, 0.38268343236508977f,
+                                0.f, -0.38268343236508977f, -0.70710678118654752f, -0.92387953251128674f};
+        constexpr float s[8] = {0.f, -0.38268343236508977f, -0.70710678118654752f, -0.92387953251128674f,
+                                -1.f, -0.92387953251128674f, -0.70710678118654752f, -0.38268343236508977f};
+        const int k = j * (8 / h);
+        if (k == 0) return a;
+        if (k == 4) return Conj::value ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+        return cmul<Conj::value>(a, make_float2(c[k], s[k]));
+    }
+};
 
-// Radices of a W-point transform: R1 over stride W / R1, then R2 (W > 256: 16) over stride W / 256,
-// then RL over contiguous points.
+// Passes of a W-point transform: 16 points over stride W / 16, then (W > 256) 16 over stride W / 256, then
+// RL contiguous ones.
 template <int LOG2W>
 struct Fft {
     static constexpr int W = 1 << LOG2W;
-    static constexpr int E = W < 16 ? W : 16;       // points per thread, the first radix
+    static constexpr int E = W < 16 ? W : 16;       // points per thread, and of the first pass
     static constexpr int TPF = W / E;               // threads per transform
     static constexpr bool MID = W > 256;            // a middle pass
-    static constexpr int RL = MID ? W / 256 : TPF;  // the last radix (1: no last pass)
+    static constexpr int RL = MID ? W / 256 : TPF;  // points of the last pass (1: none)
     // shared-memory slots of one transform: one float2 of padding per 16, so that the contiguous
     // runs of the last pass (16 points a thread) and the strided ones of the others are all free
     // of bank conflicts
@@ -176,11 +163,11 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) fi
     for (int m = 0; m < E; m++)
         if ((unsigned)(c0 + m * TPF) < (unsigned)a.nu)
             v[m] = make_float2(__ldg(p1 + c0 + m * TPF), __ldg(p2 + c0 + m * TPF));
-    if (a.cos) {
+    if (a.cos) {  // rounded products (here and with H): not fused into the first stage's sums
 #pragma unroll
         for (int m = 0; m < E; m++)
             if ((unsigned)(c0 + m * TPF) < (unsigned)a.nu)
-                v[m] = make_float2(v[m].x * __ldg(w1 + c0 + m * TPF), v[m].y * __ldg(w2 + c0 + m * TPF));
+                v[m] = make_float2(__fmul_rn(v[m].x, __ldg(w1 + c0 + m * TPF)), __fmul_rn(v[m].y, __ldg(w2 + c0 + m * TPF)));
     }
     // the pads: means of the first and last pad_n weighted samples
     for (int q = t; q < 4; q += TPF) {
@@ -202,46 +189,42 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) fi
         else if (c >= a.nu) v[m] = make_float2(pads[g][1], pads[g][3]);
     }
 
-    // v[k] *= w_{n E}^(i k) (or its conjugate), i < n the thread's place in its block of a pass.
-    // plane: the pass's twiddles as float4 (k, k + 1) pairs, pair-major; gathered: entry i k of the
-    // pass's roots, which are every (W / n / E)-th of tw.
-    auto twiddle = [&](auto conj, const float2 *plane, int n, int i) {
-        constexpr bool CONJ = decltype(conj)::value;
+    // The twiddles of a pass: 8 + 4 + 2 + 1 of the first to the last stage of its four, for the thread's place
+    // i < n in a block (n: the pass's stride).  plane: as float4 pairs, pair-major; gathered: entry j of the
+    // stage of half-width h is root (i + j n) 8/h of the pass's, which are every (TPF / n)-th of tw.
+    float2 tq[16];
+    auto load_twiddles = [&](const float2 *plane, int n, int i) {
         if constexpr (GATHER) {
 #pragma unroll
-            for (int k = 1; k < E; k++) {
-                const int e = i * k * (TPF / n);  // < W
-                float2 w = __ldg(a.tw + (e & (W / 2 - 1)));
-                if (e >= W / 2) w = make_float2(-w.x, -w.y);
-                v[k] = cmul<CONJ>(v[k], w);
-            }
-        } else if constexpr (E >= 2) {
+            for (int h = E / 2; h; h >>= 1)
+#pragma unroll
+                for (int j = 0; j < h; j++) tq[E - 2 * h + j] = __ldg(a.tw + (i + j * n) * (E / 2 / h) * (TPF / n));
+        } else {
             const float4 *q = reinterpret_cast<const float4 *>(plane) + i;
 #pragma unroll
-            for (int k = 0; k < E; k += 2) {
-                const float4 f = load_here(q + (k / 2) * n);
-                if (k) v[k] = cmul<CONJ>(v[k], make_float2(f.x, f.y));
-                v[k + 1] = cmul<CONJ>(v[k + 1], make_float2(f.z, f.w));
+            for (int k = 0; k < 8; k++) {
+                const float4 f = load_here(q + k * n);
+                tq[2 * k] = make_float2(f.x, f.y);
+                tq[2 * k + 1] = make_float2(f.z, f.w);
             }
         }
     };
-    using Fwd = std::false_type;
-    using Inv = std::true_type;
+    auto loaded = [&](auto conj, float2 x, int h, int j) { return cmul<decltype(conj)::value>(x, tq[E - 2 * h + j]); };
     float2 *outer = buf + slot(t);                               // points t + k TPF
     float2 *middle = buf + slot((t / RL) * (E * RL)) + t % RL;  // points of the middle pass, RL apart
     float2 *inner = buf + slot(t * E);                           // the last pass's run of points
 
-    dft<E, false>(v, 0);
     if constexpr (TPF > 1) {
-        twiddle(Fwd{}, a.twp, TPF, t);
+        load_twiddles(a.twp, TPF, t);
+        dif<E>(v, 0, loaded);
 #pragma unroll
         for (int k = 0; k < E; k++) outer[slot(k * TPF)] = v[k];
         meet();
         if constexpr (F::MID) {
 #pragma unroll
             for (int k = 0; k < E; k++) v[k] = middle[slot(k * RL)];
-            dft<E, false>(v, 0);
-            twiddle(Fwd{}, a.twp + W, RL, t % RL);
+            load_twiddles(a.twp + W, RL, t % RL);
+            dif<E>(v, 0, loaded);
 #pragma unroll
             for (int k = 0; k < E; k++) middle[slot(k * RL)] = v[k];
             meet();
@@ -249,45 +232,49 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) fi
 #pragma unroll
         for (int k = 0; k < E; k++) v[k] = inner[k];
 #pragma unroll
-        for (int b = 0; b < E; b += RL) dft<RL, false>(v, b);
+        for (int b = 0; b < E; b += RL) dif<RL>(v, b, Roots{});
+    } else {
+        dif<E>(v, 0, Roots{});
     }
     if constexpr (E == 16) {  // four planes of float4
         const float4 *h4 = reinterpret_cast<const float4 *>(a.hb) + t;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const float4 h = __ldg(h4 + q * TPF);
-            v[4 * q] = make_float2(v[4 * q].x * h.x, v[4 * q].y * h.x);
-            v[4 * q + 1] = make_float2(v[4 * q + 1].x * h.y, v[4 * q + 1].y * h.y);
-            v[4 * q + 2] = make_float2(v[4 * q + 2].x * h.z, v[4 * q + 2].y * h.z);
-            v[4 * q + 3] = make_float2(v[4 * q + 3].x * h.w, v[4 * q + 3].y * h.w);
+            v[4 * q] = make_float2(__fmul_rn(v[4 * q].x, h.x), __fmul_rn(v[4 * q].y, h.x));
+            v[4 * q + 1] = make_float2(__fmul_rn(v[4 * q + 1].x, h.y), __fmul_rn(v[4 * q + 1].y, h.y));
+            v[4 * q + 2] = make_float2(__fmul_rn(v[4 * q + 2].x, h.z), __fmul_rn(v[4 * q + 2].y, h.z));
+            v[4 * q + 3] = make_float2(__fmul_rn(v[4 * q + 3].x, h.w), __fmul_rn(v[4 * q + 3].y, h.w));
         }
     } else if constexpr (W > 1) {  // (a single sample is passed through)
 #pragma unroll
         for (int k = 0; k < E; k++) {
             const float h = __ldg(a.hb + k);
-            v[k] = make_float2(v[k].x * h, v[k].y * h);
+            v[k] = make_float2(__fmul_rn(v[k].x, h), __fmul_rn(v[k].y, h));
         }
     }
     if constexpr (TPF > 1) {
 #pragma unroll
-        for (int b = 0; b < E; b += RL) dft<RL, true>(v, b);
+        for (int b = 0; b < E; b += RL) dit<RL>(v, b, Roots{});
 #pragma unroll
         for (int k = 0; k < E; k++) inner[k] = v[k];
         meet();
         if constexpr (F::MID) {
 #pragma unroll
             for (int k = 0; k < E; k++) v[k] = middle[slot(k * RL)];
-            twiddle(Inv{}, a.twp + W, RL, t % RL);
-            dft<E, true>(v, 0);
+            load_twiddles(a.twp + W, RL, t % RL);
+            dit<E>(v, 0, loaded);
 #pragma unroll
             for (int k = 0; k < E; k++) middle[slot(k * RL)] = v[k];
             meet();
         }
 #pragma unroll
         for (int k = 0; k < E; k++) v[k] = outer[slot(k * TPF)];
-        twiddle(Inv{}, a.twp, TPF, t);
+        load_twiddles(a.twp, TPF, t);
+        dit<E>(v, 0, loaded);
+    } else {
+        dit<E>(v, 0, Roots{});
     }
-    dft<E, true>(v, 0);
 
     bool over = false;
 #pragma unroll
@@ -391,18 +378,17 @@ int FilterTables::create(const double *H, int W_) {
     for (int k = 0; k < W / 2; k++) t[k] = root(k, W);
     std::vector<float> h(W);
     for (int i = 0; i < W; i++) h[i] = (float)(H[filter_response_frequency(i, W)] / W);
-    // the passes' twiddles: w^(i k) for k < E as E / 2 planes of pairs, i fastest: first pass (n = W / E
-    // places, W-th roots), then the middle pass (n = W / 256 places, W/16-th roots)
+    // the passes' twiddles: 8 + 4 + 2 + 1 per place i < n of a pass of stride n, as 8 planes of pairs, i
+    // fastest: entry j of the stage of half-width h is root (i + j n) 8/h of the 16 n
     std::vector<float2> pt;
-    auto put = [&](int n, int E) {
-        for (int k = 0; k < E; k += 2)
-            for (int i = 0; i < n; i++) {
-                pt.push_back(root((long long)i * k, n * E));
-                pt.push_back(root((long long)i * (k + 1), n * E));
-            }
+    auto put = [&](int n) {
+        const size_t at = pt.size();
+        pt.resize(at + 16 * (size_t)n, make_float2(0.f, 0.f));
+        for (int e = 0; e < 15; e++)
+            for (int i = 0; i < n; i++) pt[at + ((size_t)(e / 2) * n + i) * 2 + e % 2] = root(filter_twiddle(e, i, n), 16 * n);
     };
-    if (W > 16) put(W / 16, 16);
-    if (W > 256) put(W / 256, 16);
+    if (W > 16) put(W / 16);
+    if (W > 256) put(W / 256);
     if (pt.empty()) pt.push_back(make_float2(1.f, 0.f));
     FDK_CUDA(cudaMalloc(&tw, sizeof(float2) * t.size()));
     FDK_CUDA(cudaMalloc(&hb, sizeof(float) * W));
@@ -426,11 +412,11 @@ __global__ void filter_tables_kernel(const float *__restrict__ H, int W, float2 
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < W; k += gridDim.x * blockDim.x) {
         if (tw && k < W / 2) tw[k] = root(k, W);
         if (twp && W > 16) {  // entry k of the first pass's planes, then of the middle pass's
-            const int n = W / 16, i = k / 2 % n, m = k / 2 / n * 2 + (k & 1);
-            twp[k] = root((long long)i * m, W);
+            const int n = W / 16;
+            twp[k] = root(filter_twiddle(k / 2 / n * 2 + (k & 1), k / 2 % n, n), W);
             if (W > 256 && k < W / 16) {
-                const int q = W / 256, j = k / 2 % q, r = k / 2 / q * 2 + (k & 1);
-                twp[W + k] = root((long long)j * r, W / 16);
+                const int m = W / 256;
+                twp[W + k] = root(filter_twiddle(k / 2 / m * 2 + (k & 1), k / 2 % m, m), W / 16);
             }
         }
         hb[k] = H[filter_response_frequency(k, W)] / (float)W;
@@ -467,7 +453,8 @@ static int launch_group(const FilterArgs &a, int n_views, cudaStream_t st) {
 
 // Transforms per CTA.  The column layouts write runs of G elements, so they take the largest CTA that
 // still fills the SM's 1024 resident threads evenly: 1024 threads at W = 4096 (G = 4, 32-byte runs of
-// FP32 pairs: 971 against 1139 us at 512 threads and G = 2, 32 views of 2048^2 to MIRROR FP32), 512
+// FP32 pairs: 971 against 1139 us at 512 threads and G = 2, 32 views of 2048^2 to MIRROR FP32; these and the
+// next figures with radix-16 butterflies, 2% to 4% below the present ones), 512
 // below, where G is 4 or more anyway (1500 x 1000 to MIRROR FP16 at 512 / 256 threads: 226 / 236 us).
 // ROWS stores are coalesced at any G, and smaller CTAs overlap each other's loads and transforms
 // better (48 views of 1536 x 1024 at 512 / 256 threads: 285 / 260 us).  A call whose CTAs would
@@ -683,7 +670,7 @@ int fdk_filter_row_real32(const fdk_dataref *src, fdk_dataref *dst, const fdk_da
     FDK_TRY(check_filter_dims(src->width, src->height, W, 3));
     // The tables are built on the device in a workspace of the library's pool: copying the response to
     // the host, three allocations and the copies back cost more than the filter (48 views of
-    // 1536 x 1024: 1073 us of which 240 in the filter kernel, 257 so).
+    // 1536 x 1024: 1073 us of which 240 in the filter kernel; 268 us so).
     FilterTables t;
     t.W = W;
     while ((1 << t.log2W) < W) t.log2W++;

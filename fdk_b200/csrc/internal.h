@@ -25,14 +25,24 @@ struct FilterTables {
 int filter_tables_on_device(const float *H, const FilterTables &t, cudaStream_t st);
 
 // Frequency of entry i of FilterTables::hb.  The row filter's transform leaves thread t of W / 16 with
-// 16 points p = 16 t + k in digit-reversed order (radices 16, 16 for W > 256, then the rest); the
-// table holds them as four planes of four points of every thread.  W < 32 is one thread's.
+// points p = 16 t + k, k < 16, in bit-reversed order; the table holds them as four planes of four
+// points of every thread.  W < 32 is one thread's.
 __host__ __device__ inline int filter_response_frequency(int i, int W) {
-    if (W < 32) return i;
-    const int threads = W / 16, p = 16 * (i / 4 % threads) + 4 * (i / (4 * threads)) + i % 4;
-    if (W <= 256) return p / threads + 16 * (p % threads);
-    const int last = W / 256;
-    return p / threads + 16 * (p % threads / last) + 256 * (p % last);
+    const int threads = W / 16;
+    int p = W < 32 ? i : 16 * (i / 4 % threads) + 4 * (i / (4 * threads)) + i % 4, f = 0;
+    for (int b = 1; b < W; b <<= 1, p >>= 1) f = 2 * f + (p & 1);
+    return f;
+}
+
+// Twiddle e < 15 of place i in a pass of stride n: 8 of the first of its four stages, then 4, 2, 1; as a
+// power of exp(-2 pi i / 16 n).
+__host__ __device__ inline int filter_twiddle(int e, int i, int n) {
+    int h = 8;
+    while (h && e >= h) {
+        e -= h;
+        h >>= 1;
+    }
+    return h ? (i + e * n) * (8 / h) : 0;
 }
 
 // Fused cosine weight + pad + ramp filter + crop + layout store (filter.cu).
