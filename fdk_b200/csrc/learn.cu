@@ -11,409 +11,20 @@
 //   y  = x + o / s                  residual: zero W3, b3 give plain FDK
 // Parameters FP32 (layout W1[32][9], b1[32], W2[32][32][9], b2[32], W3[32][9], b3); activations
 // are kept in shared memory as BF16 (forward) and recomputed in the backward pass, so no
-// activation tensor touches HBM.
+// activation tensor touches HBM.  The network's kernels are in nn_tc.cuh.
 //
 // Training kernels: exact adjoint of the staged backprojection (scatter with the gather's
 // bilinear weights and bounds, accumulated per view in a shared-memory box), the volume MSE
 // and its gradient, Adam, Poisson transmission noise, an ellipsoid voxelizer, and the
 // ROWS -> MIRROR layout change that feeds the backprojection.
-#include <cuda_bf16.h>
-
 #include <mutex>
 #include <vector>
 
 #include "common.h"
 #include "internal.h"
+#include "nn_tc.cuh"
 
 namespace fdk {
-
-constexpr int kCh = 32, kK = 9, kHalo = 4;
-constexpr int kW1 = 0, kB1 = kW1 + kCh * kK, kW2 = kB1 + kCh, kB2 = kW2 + kCh * kCh * kK, kW3 = kB2 + kCh,
-              kB3 = kW3 + kCh * kK, kNParam = kB3 + 1;
-constexpr int kMaxLen = 256;  // row length limit (the backward kernel holds ~176 KB of shared memory)
-
-// --------------------------------------------------------------------------------------------
-// Network kernels.  One CTA of 256 threads works on one row at a time (persistent over rows).
-// The convolutions are register-blocked: in the channel phases thread t owns 4 consecutive
-// positions (pg = t % 64) x 8 channels (q = t / 64, uniform within a warp), so each float4
-// weight load (a warp-wide broadcast) feeds 16 FMAs and one 12-value activation window feeds
-// all 9 taps.  Activation rows carry a zero halo: buffer index = position + 4, and every entry
-// past the row's end stays zero, so no tap needs a bounds test.
-// --------------------------------------------------------------------------------------------
-constexpr int kThreads = 256;
-constexpr int kBuf = kMaxLen + 2 * kHalo + 8;  // 272 f32 per scalar row buffer (x, d3)
-constexpr int kPitchA = 268;                    // bf16 per activation row (8-byte aligned rows)
-constexpr int kPitchD = 268;                    // f32 per dz2 row (16-byte aligned rows)
-constexpr int kPitchZ = 260;                    // f32 per dz1 row (16-byte aligned rows)
-
-struct NnWeights {
-    float w2f[kCh * kK * kCh];  // W2 as [ci][k][c]: the 8 output channels of one (ci, k) are contiguous
-    float w1[kCh * kK], b1[kCh], b2[kCh], w3[kCh * kK], b3[4];
-};
-
-struct NnFwdShared {
-    NnWeights w;
-    float x[kBuf];                        // s * x with halo
-    float part[4][kMaxLen];               // layer-3 partial sums of the 4 channel groups
-    __nv_bfloat16 a1[kCh][kPitchA];       // relu(layer 1), BF16
-    __nv_bfloat16 a2[kCh][kPitchA];       // relu(layer 2), BF16
-};
-
-__device__ __forceinline__ float bf_lo(unsigned u) { return __uint_as_float(u << 16); }
-__device__ __forceinline__ float bf_hi(unsigned u) { return __uint_as_float(u & 0xFFFF0000u); }
-
-// 12 consecutive f32 from a 16-byte aligned address
-__device__ __forceinline__ void ld_f12(const float *p, float (&v)[12]) {
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const float4 t = reinterpret_cast<const float4 *>(p)[i];
-        v[4 * i] = t.x;
-        v[4 * i + 1] = t.y;
-        v[4 * i + 2] = t.z;
-        v[4 * i + 3] = t.w;
-    }
-}
-
-// 4n consecutive BF16 (as f32) from an 8-byte aligned address
-template <int N>
-__device__ __forceinline__ void ld_bf(const __nv_bfloat16 *p, float (&v)[N]) {
-    static_assert(N % 4 == 0, "groups of 4");
-#pragma unroll
-    for (int i = 0; i < N / 4; i++) {
-        const uint2 u = reinterpret_cast<const uint2 *>(p)[i];
-        v[4 * i] = bf_lo(u.x);
-        v[4 * i + 1] = bf_hi(u.x);
-        v[4 * i + 2] = bf_lo(u.y);
-        v[4 * i + 3] = bf_hi(u.y);
-    }
-}
-
-// 4 values -> BF16 (round to nearest even) at an 8-byte aligned address
-__device__ __forceinline__ void st_bf4(__nv_bfloat16 *p, const float (&v)[4]) {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-    uint2 u;
-    u.x = *reinterpret_cast<const unsigned *>(&lo);
-    u.y = *reinterpret_cast<const unsigned *>(&hi);
-    *reinterpret_cast<uint2 *>(p) = u;
-}
-
-__device__ void nn_load_weights(NnWeights &w, float *w2b, const float *params) {
-    for (int i = threadIdx.x; i < kCh * kCh * kK; i += kThreads) {
-        const int c = i / (kCh * kK), ci = (i / kK) % kCh, k = i % kK;  // params W2[c][ci][k]
-        const float v = params[kW2 + i];
-        w.w2f[(ci * kK + k) * kCh + c] = v;
-        if (w2b) w2b[(c * kK + k) * kCh + ci] = v;
-    }
-    for (int i = threadIdx.x; i < kCh * kK; i += kThreads) {
-        w.w1[i] = params[kW1 + i];
-        w.w3[i] = params[kW3 + i];
-    }
-    for (int i = threadIdx.x; i < kCh; i += kThreads) {
-        w.b1[i] = params[kB1 + i];
-        w.b2[i] = params[kB2 + i];
-    }
-    if (threadIdx.x == 0) w.b3[0] = params[kB3];
-}
-
-// a1[c][p] = relu(b1[c] + sum_k W1[c][k] xs[p + k - 4]) for this thread's 4 positions x 8 channels
-__device__ __forceinline__ void nn_layer1(const NnWeights &w, const float *xb, __nv_bfloat16 (*a1)[kPitchA], int pg,
-                                          int q, int L) {
-    const int p0 = 4 * pg;
-    float xw[12];
-    ld_f12(xb + p0, xw);  // positions p0 - 4 .. p0 + 7
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int c = 8 * q + i;
-        float z[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) z[j] = w.b1[c];
-#pragma unroll
-        for (int k = 0; k < kK; k++) {
-            const float wk = w.w1[c * kK + k];
-#pragma unroll
-            for (int j = 0; j < 4; j++) z[j] = fmaf(wk, xw[j + k], z[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) z[j] = (p0 + j < L) ? fmaxf(z[j], 0.f) : 0.f;
-        st_bf4(&a1[c][p0 + kHalo], z);
-    }
-}
-
-// a2[c][p] = relu(b2[c] + sum_ci sum_k W2[c][ci][k] a1[ci][p + k - 4])
-__device__ __forceinline__ void nn_layer2(const NnWeights &w, const __nv_bfloat16 (*a1)[kPitchA],
-                                          __nv_bfloat16 (*a2)[kPitchA], int pg, int q, int L) {
-    const int p0 = 4 * pg;
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = w.b2[8 * q + i];
-#pragma unroll 2
-    for (int ci = 0; ci < kCh; ci++) {
-        float a[12];
-        ld_bf<12>(&a1[ci][p0], a);
-#pragma unroll
-        for (int k = 0; k < kK; k++) {
-            const float4 wa = *reinterpret_cast<const float4 *>(&w.w2f[(ci * kK + k) * kCh + 8 * q]);
-            const float4 wb = *reinterpret_cast<const float4 *>(&w.w2f[(ci * kK + k) * kCh + 8 * q + 4]);
-            const float wv[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(wv[i], a[j + k], acc[i][j]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        float r[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) r[j] = (p0 + j < L) ? fmaxf(acc[i][j], 0.f) : 0.f;
-        st_bf4(&a2[8 * q + i][p0 + kHalo], r);
-    }
-}
-
-__global__ void __launch_bounds__(kThreads, 2) nn_forward_kernel(const float *__restrict__ params, const float *x,
-                                                                float *y, int L, long long rows, float s) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    NnFwdShared &sm = *reinterpret_cast<NnFwdShared *>(smraw);
-    const int t = threadIdx.x, pg = t % 64, q = t / 64;
-    nn_load_weights(sm.w, nullptr, params);
-    for (int i = t; i < kCh * kPitchA; i += kThreads) {
-        (&sm.a1[0][0])[i] = __float2bfloat16(0.f);
-        (&sm.a2[0][0])[i] = __float2bfloat16(0.f);
-    }
-    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-        __syncthreads();
-        for (int i = t; i < kBuf; i += kThreads) {
-            const int p = i - kHalo;
-            sm.x[i] = (p >= 0 && p < L) ? x[r * L + p] * s : 0.f;
-        }
-        __syncthreads();
-        nn_layer1(sm.w, sm.x, sm.a1, pg, q, L);
-        __syncthreads();
-        nn_layer2(sm.w, sm.a1, sm.a2, pg, q, L);
-        __syncthreads();
-        {  // layer 3, partial over this thread's 8 channels
-            float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int c = 8 * q + i;
-                float a[12];
-                ld_bf<12>(&sm.a2[c][4 * pg], a);
-#pragma unroll
-                for (int k = 0; k < kK; k++) {
-                    const float wk = sm.w.w3[c * kK + k];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) o[j] = fmaf(wk, a[j + k], o[j]);
-                }
-            }
-            *reinterpret_cast<float4 *>(&sm.part[q][4 * pg]) = make_float4(o[0], o[1], o[2], o[3]);
-        }
-        __syncthreads();
-        if (t < L) {
-            const float o = sm.w.b3[0] + ((sm.part[0][t] + sm.part[1][t]) + (sm.part[2][t] + sm.part[3][t]));
-            y[r * L + t] = x[r * L + t] + o / s;
-        }
-    }
-}
-
-// --------------------------------------------------------------------------------------------
-// backward: persistent CTAs (one per SM); each row's activations are recomputed in shared
-// memory, and the parameter gradients stay in registers for the CTA's whole life:
-//   dW2[c][ci][k]  thread (warp w: c = 4w..4w+3, lane: ci), 36 accumulators
-//   dW3[c][k], dW1[ci][k]  lane = channel, warp = a 32-position range, 9 accumulators each
-//   db1, db2 (8 per thread, its channel group), db3
-// and are added to global memory once at the end.
-// --------------------------------------------------------------------------------------------
-struct NnBackShared {
-    NnWeights w;
-    float w2b[kCh * kK * kCh];        // W2 as [c][k][ci]: the 8 input channels of one (c, k) are contiguous
-    float x[kBuf];                    // s * x with halo
-    float d3[kBuf];                   // dL/do = dL/dy / s with halo
-    float dz2[kCh][kPitchD];          // dL/dz2 with halo
-    float dz1[kCh][kPitchZ];          // dL/dz1, positions 0 .. 255
-    __nv_bfloat16 a1[kCh][kPitchA];
-    __nv_bfloat16 a2[kCh][kPitchA];
-};
-
-__global__ void __launch_bounds__(kThreads, 1) nn_backward_kernel(const float *__restrict__ params, const float *x,
-                                                                 const float *dy, float *dparams, int L,
-                                                                 long long rows, float s) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    NnBackShared &sm = *reinterpret_cast<NnBackShared *>(smraw);
-    const int t = threadIdx.x, pg = t % 64, q = t / 64, p0 = 4 * pg, lane = t & 31, wp = t >> 5;
-    nn_load_weights(sm.w, sm.w2b, params);
-    for (int i = t; i < kCh * kPitchA; i += kThreads) {
-        (&sm.a1[0][0])[i] = __float2bfloat16(0.f);
-        (&sm.a2[0][0])[i] = __float2bfloat16(0.f);
-    }
-    for (int i = t; i < kCh * kPitchD; i += kThreads) (&sm.dz2[0][0])[i] = 0.f;
-
-    float gw2[4][kK], gw3[kK], gw1[kK], gb1[8], gb2[8], gb3 = 0.f;
-#pragma unroll
-    for (int k = 0; k < kK; k++) {
-        gw3[k] = gw1[k] = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; i++) gw2[i][k] = 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) gb1[i] = gb2[i] = 0.f;
-
-    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-        __syncthreads();
-        for (int i = t; i < kBuf; i += kThreads) {
-            const int p = i - kHalo;
-            const bool in = p >= 0 && p < L;
-            sm.x[i] = in ? x[r * L + p] * s : 0.f;
-            const float d = in ? dy[r * L + p] / s : 0.f;  // y = x + o / s
-            sm.d3[i] = d;
-            gb3 += d;
-        }
-        __syncthreads();
-        nn_layer1(sm.w, sm.x, sm.a1, pg, q, L);
-        __syncthreads();
-        nn_layer2(sm.w, sm.a1, sm.a2, pg, q, L);
-        __syncthreads();
-        {  // dz2[c][p] = [a2 > 0] sum_k W3[c][k] d3[p - k + 4]
-            float dw[12];
-            ld_f12(sm.d3 + p0, dw);  // positions p0 - 4 .. p0 + 7
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int c = 8 * q + i;
-                float m[4];
-                ld_bf<4>(&sm.a2[c][p0 + kHalo], m);
-                float g[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int k = 0; k < kK; k++) {
-                    const float wk = sm.w.w3[c * kK + k];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) g[j] = fmaf(wk, dw[j - k + 8], g[j]);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    g[j] = m[j] > 0.f ? g[j] : 0.f;
-                    gb2[i] += g[j];
-                }
-                *reinterpret_cast<float4 *>(&sm.dz2[c][p0 + kHalo]) = make_float4(g[0], g[1], g[2], g[3]);
-            }
-        }
-        // dW3[c][k] += sum_p d3[p] a2[c][p + k - 4]   (lane = c, warp = positions 32 wp ..)
-#pragma unroll 1
-        for (int m = 0; m < 4; m++) {
-            const int pb = 32 * wp + 8 * m;
-            if (pb >= L) break;
-            float a[16];
-            ld_bf<16>(&sm.a2[lane][pb], a);
-            const float4 d0 = *reinterpret_cast<const float4 *>(&sm.d3[pb + kHalo]);
-            const float4 d1 = *reinterpret_cast<const float4 *>(&sm.d3[pb + kHalo + 4]);
-            const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-#pragma unroll
-                for (int k = 0; k < kK; k++) gw3[k] = fmaf(d[j], a[j + k], gw3[k]);
-        }
-        __syncthreads();
-        {  // dz1[ci][p] = [a1 > 0] sum_c sum_k W2[c][ci][k] dz2[c][p - k + 4]
-            float acc[8][4];
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-#pragma unroll 2
-            for (int c = 0; c < kCh; c++) {
-                float dw[12];
-                ld_f12(&sm.dz2[c][p0], dw);
-#pragma unroll
-                for (int k = 0; k < kK; k++) {
-                    const float4 wa = *reinterpret_cast<const float4 *>(&sm.w2b[(c * kK + k) * kCh + 8 * q]);
-                    const float4 wb = *reinterpret_cast<const float4 *>(&sm.w2b[(c * kK + k) * kCh + 8 * q + 4]);
-                    const float wv[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-#pragma unroll
-                        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(wv[i], dw[j - k + 8], acc[i][j]);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int ci = 8 * q + i;
-                float m[4];
-                ld_bf<4>(&sm.a1[ci][p0 + kHalo], m);
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    acc[i][j] = m[j] > 0.f ? acc[i][j] : 0.f;
-                    gb1[i] += acc[i][j];
-                }
-                *reinterpret_cast<float4 *>(&sm.dz1[ci][p0]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-            }
-        }
-        // dW2[c][ci][k] += sum_p dz2[c][p] a1[ci][p + k - 4]   (c = 4 wp + i, lane = ci)
-#pragma unroll 1
-        for (int pb = 0; pb < L; pb += 8) {
-            float a[16];
-            ld_bf<16>(&sm.a1[lane][pb], a);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 d0 = *reinterpret_cast<const float4 *>(&sm.dz2[4 * wp + i][pb + kHalo]);
-                const float4 d1 = *reinterpret_cast<const float4 *>(&sm.dz2[4 * wp + i][pb + kHalo + 4]);
-                const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-#pragma unroll
-                    for (int k = 0; k < kK; k++) gw2[i][k] = fmaf(d[j], a[j + k], gw2[i][k]);
-            }
-        }
-        __syncthreads();
-        // dW1[ci][k] += sum_p dz1[ci][p] xs[p + k - 4]   (lane = ci, warp = positions 32 wp ..)
-#pragma unroll 1
-        for (int m = 0; m < 4; m++) {
-            const int pb = 32 * wp + 8 * m;
-            if (pb >= L) break;
-            float xw[16];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 v = *reinterpret_cast<const float4 *>(&sm.x[pb + 4 * i]);
-                xw[4 * i] = v.x;
-                xw[4 * i + 1] = v.y;
-                xw[4 * i + 2] = v.z;
-                xw[4 * i + 3] = v.w;
-            }
-            const float4 g0 = *reinterpret_cast<const float4 *>(&sm.dz1[lane][pb]);
-            const float4 g1 = *reinterpret_cast<const float4 *>(&sm.dz1[lane][pb + 4]);
-            const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-#pragma unroll
-                for (int k = 0; k < kK; k++) gw1[k] = fmaf(g[j], xw[j + k], gw1[k]);
-        }
-    }
-
-    // one global add per accumulator (db sums reduced over the warp's lanes first)
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int k = 0; k < kK; k++) atomicAdd(dparams + kW2 + ((4 * wp + i) * kCh + lane) * kK + k, gw2[i][k]);
-#pragma unroll
-    for (int k = 0; k < kK; k++) {
-        atomicAdd(dparams + kW3 + lane * kK + k, gw3[k]);
-        atomicAdd(dparams + kW1 + lane * kK + k, gw1[k]);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-        for (int o = 16; o; o >>= 1) {
-            gb1[i] += __shfl_xor_sync(0xFFFFFFFFu, gb1[i], o);
-            gb2[i] += __shfl_xor_sync(0xFFFFFFFFu, gb2[i], o);
-        }
-    for (int o = 16; o; o >>= 1) gb3 += __shfl_xor_sync(0xFFFFFFFFu, gb3, o);
-    if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            atomicAdd(dparams + kB1 + 8 * q + i, gb1[i]);
-            atomicAdd(dparams + kB2 + 8 * q + i, gb2[i]);
-        }
-        atomicAdd(dparams + kB3, gb3);
-    }
-}
 
 // --------------------------------------------------------------------------------------------
 // Adam (Kingma & Ba), bias-corrected
@@ -533,7 +144,7 @@ __global__ void rows_to_mirror_kernel(const float *__restrict__ src, float2 *__r
 // volume MSE: vol in the backprojection's [x][y][z] layout, truth [z][y][x];
 // res[z][y][x] = 2 (vol - truth) / N, sum of squared errors in *sse
 // --------------------------------------------------------------------------------------------
-__device__ double g_sse;  // fdk_volume_mse's accumulator
+__device__ double g_sse[2];  // fdk_volume_mse's accumulator; the network kernels' error word, for the same copy
 
 __global__ void mse_kernel(const float *__restrict__ vol, const float *__restrict__ truth, float *res, int nx, int ny,
                            int nz, double *sse) {
@@ -549,6 +160,7 @@ __global__ void mse_kernel(const float *__restrict__ vol, const float *__restric
     }
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(sse, acc);
+    if (blockIdx.x == 0 && threadIdx.x == 0) sse[1] = (double)atomicExch(&nn::g_nn_err, 0u);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -748,13 +360,12 @@ int fdk_nn_forward(const float *params, const float *x, float *y, int64_t rows, 
     clear_error();
     FDK_CHECK_ARG(params && x && y, "NULL argument");
     FDK_CHECK_ARG(len >= kK && len <= kMaxLen && rows > 0, "row length must be 9..%d", kMaxLen);
-    const size_t smem = sizeof(NnFwdShared);
-    FDK_CUDA(cudaFuncSetAttribute(nn_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FDK_CUDA(cudaFuncSetAttribute(nn::forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nn::Fwd::BYTES));
     int sms = 0, dev = 0;
     FDK_CUDA(cudaGetDevice(&dev));
     FDK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int blocks = (int)std::min<long long>(rows, 2 * sms);  // two resident CTAs per SM
-    nn_forward_kernel<<<blocks, kThreads, smem, (cudaStream_t)stream>>>(params, x, y, len, rows, scale);
+    const int blocks = (int)std::min<long long>(ceil_div(rows, nn::rows_per_step(len)), 2 * sms);  // two resident CTAs per SM
+    nn::forward_kernel<<<blocks, nn::THREADS, nn::Fwd::BYTES, (cudaStream_t)stream>>>(params, x, y, len, rows, scale);
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
     FDK_ABI_END
@@ -766,14 +377,14 @@ int fdk_nn_backward(const float *params, const float *x, const float *dy, float 
     clear_error();
     FDK_CHECK_ARG(params && x && dy && dparams, "NULL argument");
     FDK_CHECK_ARG(len >= kK && len <= kMaxLen && rows > 0, "row length must be 9..%d", kMaxLen);
-    const size_t smem = sizeof(NnBackShared);
-    FDK_CUDA(cudaFuncSetAttribute(nn_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FDK_CUDA(cudaFuncSetAttribute(nn::backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nn::Bwd::BYTES));
     int sms = 0, dev = 0;
     FDK_CUDA(cudaGetDevice(&dev));
     FDK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int blocks = (int)std::min<long long>(rows, sms);
+    const int blocks = (int)std::min<long long>(ceil_div(rows, nn::rows_per_step(len)), sms);
     FDK_CUDA(cudaMemsetAsync(dparams, 0, sizeof(float) * kNParam, (cudaStream_t)stream));
-    nn_backward_kernel<<<blocks, kThreads, smem, (cudaStream_t)stream>>>(params, x, dy, dparams, len, rows, scale);
+    nn::backward_kernel<<<blocks, nn::Bwd::THREADS, nn::Bwd::BYTES, (cudaStream_t)stream>>>(params, x, dy, dparams, len, rows,
+                                                                                          scale);
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
     FDK_ABI_END
@@ -832,11 +443,16 @@ int fdk_volume_mse(const float *dev_vol_xyz, const float *dev_truth, float *dev_
     std::lock_guard<std::mutex> lock(mu);
     double *d_sse = nullptr;
     FDK_CUDA(cudaGetSymbolAddress((void **)&d_sse, g_sse));
-    FDK_CUDA(cudaMemsetAsync(d_sse, 0, sizeof(double), st));
+    FDK_CUDA(cudaMemsetAsync(d_sse, 0, 2 * sizeof(double), st));
     mse_kernel<<<148 * 8, 256, 0, st>>>(dev_vol_xyz, dev_truth, dev_res, nx, ny, nz, d_sse);
     FDK_CUDA(cudaGetLastError());
-    FDK_CUDA(cudaMemcpyAsync(sse_host, d_sse, sizeof(double), cudaMemcpyDeviceToHost, st));
+    double got[2] = {};
+    FDK_CUDA(cudaMemcpyAsync(got, d_sse, sizeof(got), cudaMemcpyDeviceToHost, st));
     FDK_CUDA(cudaStreamSynchronize(st));
+    *sse_host = got[0];
+    if (got[1] != 0)
+        return fail(FDK_ERR_DEVICE_CHECK, "a network kernel's pipeline wait timed out on the device (error word %u)",
+                    (unsigned)got[1]);
     return FDK_OK;
     FDK_ABI_END
 }

@@ -380,6 +380,8 @@ int fdk_voxelize(const fdk_geometry *g, const double *ell, int32_t n_ell, float 
 /* ROWS views (n x nv x nu) -> MIRROR f32 pairs (n x nu x nv x 2), the staged backprojection's input. */
 int fdk_rows_to_mirror(const float *dev_rows, void *dev_mirror, int64_t n_views, int32_t nu, int32_t nv,
                        void *stream);
+/* (fdk_volume_mse, synchronous, also reports FDK_ERR_DEVICE_CHECK once if a bounded pipeline wait of
+ * fdk_nn_forward or fdk_nn_backward ran out on the device since its last call.) */
 /* Sum of squared errors of a backprojection volume ([x][y][z], as fdk_bp_volume_device of a full slab
  * pair) against truth ([z][y][x]) into *sse_host; dev_res (may be NULL) = 2 (vol - truth) / N, [z][y][x]. */
 int fdk_volume_mse(const float *dev_vol_xyz, const float *dev_truth, float *dev_res, int32_t nx, int32_t ny,

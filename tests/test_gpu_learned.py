@@ -253,3 +253,36 @@ def test_forward_projector_routes_agree(nx, ny, nz, nu, nv):
         check(lib().fdk_forward_project(C.byref(g), vol.data_ptr(), i, 1, one[i].data_ptr(), None))
     assert torch.equal(both, one)
     assert float(both.abs().max()) > 0
+
+
+@pytest.mark.parametrize("L,rows", [(9, 1), (9, 61), (10, 38), (60, 9), (61, 8), (84, 7), (124, 3), (126, 5), (127, 2), (128, 3),
+                                    (129, 1), (200, 2), (252, 4), (255, 3), (256, 1), (256, 300)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_network_kernels_over_lengths(L, rows, offset):
+    """Rows that share a step of 256 positions, rows that fill one tile or two, a last step that is not full,
+    more steps than CTAs, and parameters on 4-byte boundaries, against the FP64 network with the same BF16
+    activations.  Tolerance 2^-8: an FP32 activation next to the middle of two BF16 values may round to the
+    other one, one step of 2^-8 of it, and nothing else is above 1e-6."""
+    import torch
+
+    rng = np.random.default_rng(L * 1000 + rows)
+    s = 0.25
+    params = (rng.standard_normal(N.NPARAM) * 0.1).astype(np.float32)
+    x = rng.standard_normal((rows, L)).astype(np.float32) * 4
+    dy = rng.standard_normal((rows, L)).astype(np.float32)
+    dp = torch.empty(N.NPARAM + offset, device="cuda")[offset:]
+    dp.copy_(torch.from_numpy(params))
+    dx, ddy = (torch.from_numpy(a).cuda() for a in (x, dy))
+    y, g = torch.full_like(dx, 7.0), torch.full_like(dp, 7.0)
+    check(lib().fdk_nn_forward(dp.data_ptr(), dx.data_ptr(), y.data_ptr(), rows, L, s, None))
+    check(lib().fdk_nn_backward(dp.data_ptr(), dx.data_ptr(), ddy.data_ptr(), g.data_ptr(), rows, L, s, None))
+    torch.cuda.synchronize()
+    y_ref, _ = N.forward(params, x, s, round_bf16=True)
+    g_ref = N.backward(params, x, dy, s, round_bf16=True)
+    assert np.abs(y.double().cpu().numpy() - y_ref).max() <= 2.0 ** -8 * np.abs(y_ref).max()
+    got = g.double().cpu().numpy()
+    at = 0
+    for name, n in (("W1", 288), ("b1", 32), ("W2", 9216), ("b2", 32), ("W3", 288), ("b3", 1)):
+        a, b = got[at:at + n], g_ref[at:at + n]
+        assert np.linalg.norm(a - b) <= 2.0 ** -8 * max(np.linalg.norm(b), 1e-3 * np.linalg.norm(g_ref)), name
+        at += n
