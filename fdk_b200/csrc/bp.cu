@@ -511,21 +511,13 @@ int read_volume(fdk_bp *h, float *host) {
     return FDK_OK;
 }
 
-// z bands: up to kMaxBands launches per batch (FDK_BP_BANDS lowers the cap) when each still
-// gives every CTA of the persistent grid at least 8 tiles (the split costs nothing measurable
-// then).  Boundaries fall on whole `unit`s of slices: the staged kernel's tile height R, or a
-// common multiple of it and the quarter-turn kernel's once that kernel is set up; each boundary
-// is the whole unit nearest an even split of the slices.
-void set_bands(fdk_bp *h, int unit) {
+// Cuts the slab into nb z bands.  Boundaries fall on whole `unit`s of slices: the staged kernel's tile
+// height R, or a common multiple of it and the quarter-turn kernel's once that kernel is set up; each
+// boundary is the whole unit nearest an even split of the slices.
+void cut_bands(fdk_bp *h, int nb, int unit) {
     const int R = h->precision == FDK_BP_MIXED ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
     const long long depth = (long long)h->top.depth;
-    const long long cols = ceil_div((long long)h->top.width, 16) * ceil_div((long long)h->top.height, 16);
-    const int tiles_z = (int)ceil_div(depth, R);
-    const int units = (int)ceil_div(depth, unit);
-    const char *cap = getenv("FDK_BP_BANDS");
-    const int max_bands = cap ? std::max(1, std::min(kMaxBands, atoi(cap))) : kMaxBands;
-    int nb = std::min(max_bands, units);
-    while (nb > 1 && cols * (tiles_z / nb) < 8ll * h->plan.tma_ctas) nb--;
+    const int tiles_z = (int)ceil_div(depth, R), units = (int)ceil_div(depth, unit);
     h->n_bands = nb;
     for (int k = 0; k <= nb; k++) {
         h->band_z[k] = std::min<long long>((long long)k * units / nb * unit, depth);
@@ -540,6 +532,53 @@ void set_bands(fdk_bp *h, int unit) {
             }
             break;
         }
+}
+
+// Most bands of a batch: kMaxBands (FDK_BP_BANDS lowers the cap), none empty.
+int most_bands(const fdk_bp *h, int unit) {
+    const char *cap = getenv("FDK_BP_BANDS");
+    const int max_bands = cap ? std::max(1, std::min(kMaxBands, atoi(cap))) : kMaxBands;
+    return std::min(max_bands, (int)ceil_div((long long)h->top.depth, unit));
+}
+
+// Bands of a handle whose batches are not known (BackProjectionFDK calls): as many as leave every CTA
+// of the persistent grid at least 8 tiles a launch (the split costs nothing measurable then).
+void set_bands(fdk_bp *h, int unit) {
+    const int R = h->precision == FDK_BP_MIXED ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
+    const long long cols = ceil_div((long long)h->top.width, 16) * ceil_div((long long)h->top.height, 16);
+    const int tiles_z = (int)ceil_div((long long)h->top.depth, R);
+    int nb = most_bands(h, unit);
+    while (nb > 1 && cols * (tiles_z / nb) < 8ll * h->plan.tma_ctas) nb--;
+    cut_bands(h, nb, unit);
+}
+
+// Bands of a reconstructor, which flushes up to `views` views before the volume is read: the cut with
+// the shortest backprojection and copy of the last band, the only one that no backprojection hides.
+// A band's persistent launch takes whole waves of tiles, so the cut decides how full they are.
+// Estimates: the kernels' measured rates and 50 GB/s to the host, 8 us a launch.  Against "8 tiles a
+// CTA", from host memory to host memory: 512^3 FP32 (5 bands of 7 to 9 waves, before 7 of 6 that held 5.3)
+// 54.1 -> 50.4 ms, 256^3 MIXED from 256 views (8 bands, before 1) 4.25 -> 3.87 ms; 2048^3 keeps 16.
+void plan_bands(fdk_bp *h, int unit, long long views) {
+    const bool mixed = h->precision == FDK_BP_MIXED, quarter = h->sym_rot != 0;
+    const int R = quarter ? (mixed ? SymCfg<HalfLerp>::R : SymCfg<float2>::R) : mixed ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
+    const long long w = (long long)h->top.width, d = (long long)h->top.height;
+    const long long cols = quarter ? ceil_div((w + 1) / 2, 16) * ceil_div((d + 1) / 2, 16) : ceil_div(w, 16) * ceil_div(d, 16);
+    const int ctas = quarter ? h->sym_ctas : h->plan.tma_ctas;
+    const double rate = mixed ? 2.7e12 : quarter ? 1.7e12 : 1.25e12;  // voxel updates a second
+    const double wave = (quarter ? 4.0 : 1.0) * 256 * 2 * R * views * ctas / rate;
+    double best = 1e300;
+    int nb = 1;
+    for (int n = 1; n <= most_bands(h, unit); n++) {
+        cut_bands(h, n, unit);
+        double t = 16e-6 * n + (double)(h->band_z[n] - h->band_z[n - 1]) * 2 * w * d * 4 / 50e9;
+        for (int k = 0; k < n; k++)
+            t += wave * (double)ceil_div(cols * ceil_div(h->band_z[k + 1] - h->band_z[k], (long long)R), (long long)ctas);
+        if (t < best) {
+            best = t;
+            nb = n;
+        }
+    }
+    cut_bands(h, nb, unit);
 }
 
 // The fast kernels need circular-orbit matrices: rows 0 and 2 without a z term.
@@ -1117,6 +1156,21 @@ int fdk_bp_check_internal(fdk_bp *h) {
     return check_device_error(h);
 }
 
+// Bands for a reconstructor's batches (plan_bands), once its kernels are chosen and before the first
+// launch.  views: the most that a flush backprojects.  Internal to the library (recon.cu).
+int fdk_bp_plan_bands_internal(fdk_bp *h, long long views) {
+    FDK_CHECK_ARG(h && views > 0, "NULL handle or no views");
+    if (!h->plan.tma_ok || !h->sym || h->launches > 0) return FDK_OK;
+    const bool mixed = h->precision == FDK_BP_MIXED;
+    const int R = mixed ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
+    const int Rq = mixed ? SymCfg<HalfLerp>::R : SymCfg<float2>::R;
+    int unit = R;
+    if (h->sym_rot)
+        while (unit % Rq) unit += R;  // whole tiles of both kernels
+    plan_bands(h, unit, views);
+    return FDK_OK;
+}
+
 // z bands of a batch (1 where the kernel has none).  Internal to the library (recon.cu).
 int fdk_bp_band_count_internal(const fdk_bp *h) { return h ? h->n_bands : 1; }
 
@@ -1135,8 +1189,7 @@ int fdk_bp_sym_setup_internal(fdk_bp *h, const float *mats, int n_proj, int *rot
     if (mode == "0") return FDK_OK;
     if (h->precision == FDK_BP_FP32_EXACT || !h->plan.tma_ok || !h->sym) return FDK_OK;
     if (h->precision == FDK_BP_MIXED && mode != "1") return FDK_OK;
-    // the set-up moves the z band boundaries: only before the first launch (or after a reset),
-    // so that no readback waits on a band event of launches over the old boundaries
+    // only before the first launch (or after a reset): the z band boundaries follow the kernel (plan_bands)
     if (h->launches > 0) return FDK_OK;
     const BpFastPlan &p = h->plan;
     if (p.x0 != 0 || p.y0 != 0 || p.nxs != p.nys || p.nxs != h->nx || h->nx != h->ny || (p.nxs & 1) || n_proj % 4)
@@ -1161,11 +1214,6 @@ int fdk_bp_sym_setup_internal(fdk_bp *h, const float *mats, int n_proj, int *rot
     DeviceGuard dg(h->device);
     FDK_TRY(dg.status);
     FDK_TRY(mixed ? sym_prepare<HalfLerp>(h->sym_ctas, h->device) : sym_prepare<float2>(h->sym_ctas, h->device));
-    // bands on whole tiles of both kernels (set up before the first launch)
-    const int Rt = mixed ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
-    int unit = Rt;
-    while (unit % R) unit += Rt;
-    set_bands(h, unit);
     h->sym_rot = r;
     *rot = r;
     return FDK_OK;
