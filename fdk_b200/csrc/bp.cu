@@ -12,6 +12,7 @@
 #include <cmath>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "bp_exact.cuh"
@@ -397,13 +398,20 @@ int launch_bp(fdk_bp *h, const void *dev_proj, int layout, int transpose, const 
         a.nys = (int)h->top.height;
         a.nzz = h->sym ? (int)(h->D / 2) : (int)h->top.depth;
         a.D = h->D;
-        a.transpose = transpose;
         const dim3 grid((unsigned)ceil_div(a.nzz, 32), (unsigned)ceil_div(a.nys, 8), a.nxs);
         if (kb == 0) {
-            if (h->sym && transpose) bp_exact_kernel<true, true><<<grid, dim3(32, 8), 0, st>>>(a);
-            else if (h->sym) bp_exact_kernel<true, false><<<grid, dim3(32, 8), 0, st>>>(a);
-            else if (transpose) bp_exact_kernel<false, true><<<grid, dim3(32, 8), 0, st>>>(a);
-            else bp_exact_kernel<false, false><<<grid, dim3(32, 8), 0, st>>>(a);
+            const bool wide = (size_t)width * height >= (1ull << 30) - width;
+            auto go = [&](auto sym, auto tr) {
+                constexpr bool S = decltype(sym)::value, T = decltype(tr)::value;
+                if (wide) bp_exact_kernel<S, T, unsigned long long><<<grid, dim3(32, 8), 0, st>>>(a);
+                else bp_exact_kernel<S, T, unsigned><<<grid, dim3(32, 8), 0, st>>>(a);
+            };
+            using Yes = std::true_type;
+            using No = std::false_type;
+            if (h->sym && transpose) go(Yes{}, Yes{});
+            else if (h->sym) go(Yes{}, No{});
+            else if (transpose) go(No{}, Yes{});
+            else go(No{}, No{});
             FDK_CUDA(cudaGetLastError());
             h->launches++;
         }

@@ -156,3 +156,26 @@ def test_fast_rejects_non_circular_matrices():
     bp = F.BackProjectionFDK(16, 16, 32, n, n, n, F.BoxT(0, 0, 0, n, n, 8), F.BoxT(0, 0, 8, n, n, 8), "fp32")
     with pytest.raises(F.FdkError):
         bp.BP(1, random_views(4, 16, 16), 16, 16, mats, 4)
+
+
+def test_exact_views_of_4_gb():
+    """A view of more than 2^30 samples is addressed with 64-bit offsets: the same bits as a crop of it.  The matrix
+    has w = 1 and dyadic u and v, so that moving the detector's origin by whole rows changes no rounding."""
+    import torch
+
+    n, width, rows, crop = 24, 32768, 32800, 256
+    tail = random_views(1, crop, width, seed=3)
+    big = torch.zeros((1, rows, width), device="cuda")
+    big[:, rows - crop:] = torch.from_numpy(tail).cuda()
+    small = torch.from_numpy(tail).cuda()
+
+    def run(views, height, u0):
+        m = np.array([[2.0, 0.25, 0, u0, 0.5, 16.0, 64.25, 100.5, 0, 0, 0, 1.0]], np.float32)
+        bp = F.BackProjectionFDK(width, height, 1, n, n, n, F.BoxT(0, 0, 0, n, n, n), F.BoxT(0, 0, 0, 0, 0, 0))
+        bp.BP_device(views.data_ptr(), F.LAYOUT_TRANSPOSED, m, 1)
+        vol = bp.GetVolumeData().copy()
+        bp.close()
+        return vol
+
+    got, want = run(big, rows, rows - crop + 130.5), run(small, crop, 130.5)
+    assert np.array_equal(got, want) and np.abs(want).max() > 0
