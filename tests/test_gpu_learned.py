@@ -286,3 +286,34 @@ def test_network_kernels_over_lengths(L, rows, offset):
         a, b = got[at:at + n], g_ref[at:at + n]
         assert np.linalg.norm(a - b) <= 2.0 ** -8 * max(np.linalg.norm(b), 1e-3 * np.linalg.norm(g_ref)), name
         at += n
+
+
+@pytest.mark.parametrize("nx,ny,nz,n_ell", [(1, 1, 1, 3), (31, 33, 5, 12), (64, 35, 40, 30), (130, 20, 66, 64), (40, 40, 40, 0)])
+def test_voxelizer_vs_fp64(nx, ny, nz, n_ell):
+    """Voxels against the FP64 formula in numpy, ellipsoids with voxel centres exactly on their surface, flat and
+    point-like ones and an axis of 0 among them.  A voxel may only differ where q is within 1e-12 of 1 (the order
+    of FP64 sums)."""
+    import torch
+
+    from fdk_b200.phantom import random_ellipsoids
+
+    p = small_param(64, 64, 64, 4)
+    p.nx, p.ny, p.nz = nx, ny, nz
+    p.dx, p.dy, p.dz = 1.0, 1.25, 0.75
+    e = random_ellipsoids(nx + n_ell, max(n_ell, 1), 0.5 * max(nx, ny, nz))
+    if n_ell > 6:
+        e[0, :3], e[0, 3:6], e[0, 6:15] = 0.0, 4.0, np.eye(3).ravel()
+        e[1, 3], e[2, 3:6], e[3, 5] = 1e-3, 1e-3, 0.0
+    e = np.ascontiguousarray(e[:max(n_ell, 1)])
+    out = torch.full((nz, ny, nx), 9.0, device="cuda")
+    check(lib().fdk_voxelize(C.byref(p.to_c()), e.ctypes.data, n_ell, out.data_ptr(), None))
+    z, y, x = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+    P = np.stack([(x - (nx - 1) / 2) * p.dx, -(y - (ny - 1) / 2) * p.dy, -(z - (nz - 1) / 2) * p.dz], -1)
+    want, close = np.zeros(P.shape[:3]), np.zeros(P.shape[:3], bool)
+    for k in range(n_ell):
+        with np.errstate(divide="ignore", invalid="ignore"):
+            q = (((P - e[k, :3]) @ e[k, 6:15].reshape(3, 3)) ** 2 / e[k, 3:6] ** 2).sum(-1)
+        want += np.where(q <= 1.0, e[k, 15], 0.0)
+        close |= np.abs(q - 1) < 1e-12
+    got = out.cpu().numpy()
+    assert (np.abs(got - want) <= 1e-6)[~close].all() and np.isfinite(got).all()
