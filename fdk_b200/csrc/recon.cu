@@ -305,74 +305,22 @@ std::vector<int64_t> consecutive(int64_t first, int64_t n) {
     return v;
 }
 
-// Order in which the n views of one push are taken: pos[i] is the place of the i-th view taken.  As
-// they come, unless the reconstructor pairs views into quarter-turn quadruples and its batches hold 128
-// views or more (smaller ones are a caller's choice of order and memory): then the views whose three
-// partners are in the push come first, `group` orbits from each quarter of the scan at a time, so that
-// every batch, the quarter-size first one too, holds whole orbits.  (A scan of 512 views pushed at once
-// in batches of 512 starts with views 0 .. 127, without any partner, and leaves the others one partner
-// short: 512^3 FP32 from host memory took 62.8 ms, all of it in the staged kernel, and 54.1 in this
-// order.)
-std::vector<long long> take_order(const fdk_recon *h, const int64_t *ids, int64_t n, int group) {
-    std::vector<long long> pos(n);
-    for (int64_t i = 0; i < n; i++) pos[i] = i;
-    if (!h->sym_rot || h->batch < 128 || n < 4) return pos;
-    const int64_t q = h->g.n_proj / 4;
-    // by (orbit, quarter, place); the k-th views of an orbit's four quarters make a quadruple
-    std::vector<std::array<long long, 3>> e(n);
-    for (int64_t i = 0; i < n; i++) e[i] = {ids[i] % q, ids[i] / q, i};
-    std::sort(e.begin(), e.end());
-    std::vector<std::array<long long, 4>> quads;
-    std::vector<char> paired(n, 0);
-    for (size_t i = 0; i < e.size();) {
-        std::vector<long long> by_q[4];
-        size_t j = i;
-        for (; j < e.size() && e[j][0] == e[i][0]; j++) by_q[e[j][1]].push_back(e[j][2]);
-        const size_t nq = std::min({by_q[0].size(), by_q[1].size(), by_q[2].size(), by_q[3].size()});
-        for (size_t k = 0; k < nq; k++) {
-            quads.push_back({by_q[0][k], by_q[1][k], by_q[2][k], by_q[3][k]});
-            for (const auto &l : by_q) paired[l[k]] = 1;
-        }
-        i = j;
-    }
-    size_t at = 0;
-    for (size_t c = 0; c < quads.size(); c += group)
-        for (int m = 0; m < 4; m++)
-            for (size_t k = c; k < std::min(quads.size(), c + group); k++) pos[at++] = quads[k][m];
-    for (int64_t i = 0; i < n; i++)
-        if (!paired[i]) pos[at++] = i;
-    return pos;
-}
-
-// Views next to one another in the caller's memory from pos[i] on, at most `most`.
-int run_length(const std::vector<long long> &pos, long long i, long long most) {
-    int r = 1;
-    while (r < most && i + r < (long long)pos.size() && pos[i + r] == pos[i] + r) r++;
-    return r;
-}
-
 // Host views through the copy ring: chunks of up to h->chunk views, each copied into a ring slot
 // on the copy stream and filtered on the compute stream; returns once the last copy has landed.
 int push_host(fdk_recon *h, const float *host_views, const int64_t *ids, int64_t n) {
     const long long frame = h->g.nu * h->g.nv;
     const int cap = h->chunk;
-    const std::vector<long long> pos = take_order(h, ids, n, std::max(1, cap / 4));
-    std::vector<int64_t> taken(n);
-    for (int64_t i = 0; i < n; i++) taken[i] = ids[pos[i]];
     cudaEvent_t last = nullptr;
     for (long long c = 0; c < n; c += cap) {
         const int m = (int)std::min<long long>(cap, n - c);
         const int k = h->slot;
         h->slot = (k + 1) % (int)h->d_raw.size();
         FDK_CUDA(cudaStreamWaitEvent(h->copy, h->raw_free[k], 0));
-        for (int i = 0, r; i < m; i += r) {
-            r = run_length(pos, c + i, m - i);
-            FDK_CUDA(cudaMemcpyAsync(h->d_raw[k] + i * frame, host_views + pos[c + i] * frame, sizeof(float) * frame * r,
-                                     cudaMemcpyHostToDevice, h->copy));
-        }
+        FDK_CUDA(cudaMemcpyAsync(h->d_raw[k], host_views + c * frame, sizeof(float) * frame * m,
+                                 cudaMemcpyHostToDevice, h->copy));
         FDK_CUDA(cudaEventRecord(h->raw_ready[k], h->copy));
         FDK_CUDA(cudaStreamWaitEvent(h->compute, h->raw_ready[k], 0));
-        FDK_TRY(process_chunk(h, h->d_raw[k], taken.data() + c, m, h->raw_free[k], true));
+        FDK_TRY(process_chunk(h, h->d_raw[k], ids + c, m, h->raw_free[k], true));
         last = h->raw_ready[k];
     }
     // the caller may reuse host_views once its last copy has landed
@@ -607,12 +555,9 @@ int fdk_recon_push_folder(fdk_recon *h, const char *folder, int64_t first, int64
 int push_device_ids(fdk_recon *h, const float *dev_views, const int64_t *ids, int64_t n) {
     const long long frame = h->g.nu * h->g.nv;
     const int cap = h->precision == FDK_BP_FP32_EXACT ? std::min(h->batch, 32) : h->batch;
-    const std::vector<long long> pos = take_order(h, ids, n, std::max(1, h->batch / 4));
-    std::vector<int64_t> taken(n);
-    for (int64_t i = 0; i < n; i++) taken[i] = ids[pos[i]];
-    for (long long c = 0, m; c < n; c += m) {
-        m = run_length(pos, c, cap);
-        FDK_TRY(process_chunk(h, dev_views + pos[c] * frame, taken.data() + c, (int)m, nullptr, false));
+    for (long long c = 0; c < n; c += cap) {
+        const int m = (int)std::min<long long>(cap, n - c);
+        FDK_TRY(process_chunk(h, dev_views + c * frame, ids + c, m, nullptr, false));
     }
     return FDK_OK;
 }
