@@ -289,6 +289,7 @@ struct fdk_bp {
     // the reconstructor's MIXED launches read through the compact boxes (every tile fits them)
     bool lerp_compact = false;
     bool lerp_compact_ok = false;  // the compact kernel runs at the same grid
+    bool tall_tiles = false;       // FP32: the staged kernel takes its taller tiles (TallFloat2)
     ListRec *h_list = nullptr, *d_list = nullptr;
     cudaEvent_t list_ev[kListRing] = {};
     bool list_used[kListRing] = {};
@@ -321,6 +322,30 @@ int take_timer(fdk_bp *h, std::pair<cudaEvent_t, cudaEvent_t> &t) {
     FDK_CUDA(cudaEventCreate(&t.first));
     FDK_CUDA(cudaEventCreate(&t.second));
     return FDK_OK;
+}
+
+// FP32: the staged kernel's taller tiles where the slab gives every CTA of its grid at least four of them.
+// Tall / short there: 1522 / 1434 GUPS at 256^3 (7 tiles a CTA), 1889 / 1756 at 512^3; below it the short
+// tiles are up to 1.23x the faster (133 against 150 us, 86 x 51 x 58 slices from 22 views).
+int choose_tiles(fdk_bp *h) {
+    int ctas = 0;
+    FDK_TRY(tma_prepare<TallFloat2>(ctas, h->device));
+    const BpFastPlan &p = h->plan;
+    h->tall_tiles = ceil_div(p.nxs, 16) * ceil_div(p.nys, 16) * ceil_div(p.nzz, TmaCfg<TallFloat2>::R) >= 4ll * ctas;
+    if (h->tall_tiles) h->plan.tma_ctas = ctas;
+    return FDK_OK;
+}
+
+// Tile height of the handle's staged kernel.
+int staged_rows(const fdk_bp *h) {
+    if (h->precision == FDK_BP_MIXED) return TmaCfg<HalfLerp>::R;
+    return h->tall_tiles ? TmaCfg<TallFloat2>::R : TmaCfg<float2>::R;
+}
+
+template <typename... A>
+int launch_staged_f32(const fdk_bp *h, A... a) {
+    return h->tall_tiles ? bp_tma_launch<TallFloat2>(h->plan, h->d_vol, h->d_comp, a...)
+                         : bp_tma_launch<float2>(h->plan, h->d_vol, h->d_comp, a...);
 }
 
 // Backproject n views already resident on the device.
@@ -428,8 +453,8 @@ int launch_bp(fdk_bp *h, const void *dev_proj, int layout, int transpose, const 
                     FDK_TRY(bp_tma_launch<HalfLerp>(h->plan, h->d_vol, h->d_comp, lv, d_mats, host_mats, n, st,
                                                     lerp_sc, h->band_tz[k], h->band_tz[k + 1]));
                 else
-                    FDK_TRY(bp_tma_launch<float2>(h->plan, h->d_vol, h->d_comp, dev_proj, d_mats, host_mats, n, st,
-                                                  acc_scale, h->band_tz[k], h->band_tz[k + 1]));
+                    FDK_TRY(launch_staged_f32(h, dev_proj, d_mats, host_mats, n, st, acc_scale, h->band_tz[k],
+                                              h->band_tz[k + 1]));
                 h->launches++;
                 FDK_CUDA(cudaEventRecord(h->band_done[k], st));
             }
@@ -523,7 +548,7 @@ int read_volume(fdk_bp *h, float *host) {
 // height R, or a common multiple of it and the quarter-turn kernel's once that kernel is set up; each
 // boundary is the whole unit nearest an even split of the slices.
 void cut_bands(fdk_bp *h, int nb, int unit) {
-    const int R = h->precision == FDK_BP_MIXED ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
+    const int R = staged_rows(h);
     const long long depth = (long long)h->top.depth;
     const int tiles_z = (int)ceil_div(depth, R), units = (int)ceil_div(depth, unit);
     h->n_bands = nb;
@@ -552,7 +577,7 @@ int most_bands(const fdk_bp *h, int unit) {
 // Bands of a handle whose batches are not known (BackProjectionFDK calls): as many as leave every CTA
 // of the persistent grid at least 8 tiles a launch (the split costs nothing measurable then).
 void set_bands(fdk_bp *h, int unit) {
-    const int R = h->precision == FDK_BP_MIXED ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
+    const int R = staged_rows(h);
     const long long cols = ceil_div((long long)h->top.width, 16) * ceil_div((long long)h->top.height, 16);
     const int tiles_z = (int)ceil_div((long long)h->top.depth, R);
     int nb = most_bands(h, unit);
@@ -564,15 +589,16 @@ void set_bands(fdk_bp *h, int unit) {
 // the shortest backprojection and copy of the last band, the only one that no backprojection hides.
 // A band's persistent launch takes whole waves of tiles, so the cut decides how full they are.
 // Estimates: the kernels' measured rates and 50 GB/s to the host, 8 us a launch.  Against "8 tiles a
-// CTA", from host memory to host memory: 512^3 FP32 (5 bands of 7 to 9 waves, before 7 of 6 that held 5.3)
-// 54.1 -> 50.4 ms, 256^3 MIXED from 256 views (8 bands, before 1) 4.25 -> 3.87 ms; 2048^3 keeps 16.
-void plan_bands(fdk_bp *h, int unit, long long views) {
-    const bool mixed = h->precision == FDK_BP_MIXED, quarter = h->sym_rot != 0;
-    const int R = quarter ? (mixed ? SymCfg<HalfLerp>::R : SymCfg<float2>::R) : mixed ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
+// CTA", 256^3 MIXED from 256 views, host memory to host memory (8 bands, before 1): 4.25 -> 3.87 ms;
+// 512^3 FP32 with the quarter-turn kernel (5 bands of 7 to 9 waves, before 7 of 6 that held 5.3): 54.1 -> 50.4
+// ms; 2048^3 keeps 16.
+void plan_bands(fdk_bp *h, int unit, long long views, bool quarter) {
+    const bool mixed = h->precision == FDK_BP_MIXED;
+    const int R = quarter ? (mixed ? SymCfg<HalfLerp>::R : SymCfg<float2>::R) : staged_rows(h);
     const long long w = (long long)h->top.width, d = (long long)h->top.height;
     const long long cols = quarter ? ceil_div((w + 1) / 2, 16) * ceil_div((d + 1) / 2, 16) : ceil_div(w, 16) * ceil_div(d, 16);
     const int ctas = quarter ? h->sym_ctas : h->plan.tma_ctas;
-    const double rate = mixed ? 2.7e12 : quarter ? 1.7e12 : 1.25e12;  // voxel updates a second
+    const double rate = mixed ? 2.7e12 : 1.75e12;  // voxel updates a second
     const double wave = (quarter ? 4.0 : 1.0) * 256 * 2 * R * views * ctas / rate;
     double best = 1e300;
     int nb = 1;
@@ -793,6 +819,7 @@ int fdk_bp_create(fdk_bp **out, int32_t proj_width, int32_t proj_height, int32_t
             if (h->plan.tma_ok) {
                 s = precision == FDK_BP_MIXED ? tma_prepare<HalfLerp>(h->plan.tma_ctas, device)
                                               : tma_prepare<float2>(h->plan.tma_ctas, device);
+                if (s == FDK_OK && precision != FDK_BP_MIXED) s = choose_tiles(h);
                 if (s == FDK_OK && precision == FDK_BP_MIXED) {
                     int c = 0;
                     s = tma_prepare<HalfLerpCompact>(c, device);
@@ -812,7 +839,7 @@ int fdk_bp_create(fdk_bp **out, int32_t proj_width, int32_t proj_height, int32_t
     h->band_z[0] = 0;
     h->band_z[1] = (long long)t.depth;
     if (s == FDK_OK && h->plan.tma_ok && sym)
-        set_bands(h, precision == FDK_BP_MIXED ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R);
+        set_bands(h, staged_rows(h));
     for (int k = 0; k < kMaxBands && s == FDK_OK; k++)
         ck(cudaEventCreateWithFlags(&h->band_done[k], cudaEventDisableTiming), "event");
     for (int i = 0; i < 2 && s == FDK_OK; i++)
@@ -1165,17 +1192,18 @@ int fdk_bp_check_internal(fdk_bp *h) {
 }
 
 // Bands for a reconstructor's batches (plan_bands), once its kernels are chosen and before the first
-// launch.  views: the most that a flush backprojects.  Internal to the library (recon.cu).
-int fdk_bp_plan_bands_internal(fdk_bp *h, long long views) {
+// launch.  views: the most that a flush backprojects; quarter: batches may take the quarter-turn kernel.
+// Internal to the library (recon.cu).
+int fdk_bp_plan_bands_internal(fdk_bp *h, long long views, bool quarter) {
     FDK_CHECK_ARG(h && views > 0, "NULL handle or no views");
     if (!h->plan.tma_ok || !h->sym || h->launches > 0) return FDK_OK;
     const bool mixed = h->precision == FDK_BP_MIXED;
-    const int R = mixed ? TmaCfg<HalfLerp>::R : TmaCfg<float2>::R;
+    const int R = staged_rows(h);
     const int Rq = mixed ? SymCfg<HalfLerp>::R : SymCfg<float2>::R;
     int unit = R;
-    if (h->sym_rot)
+    if (quarter)
         while (unit % Rq) unit += R;  // whole tiles of both kernels
-    plan_bands(h, unit, views);
+    plan_bands(h, unit, views, quarter);
     return FDK_OK;
 }
 
@@ -1191,7 +1219,7 @@ int fdk_bp_sym_setup_internal(fdk_bp *h, const float *mats, int n_proj, int *rot
     FDK_CHECK_ARG(h && mats && rot, "NULL argument");
     *rot = 0;
     h->sym_rot = 0;
-    // FDK_BP_SYM: unset = FP32 only (where it measured faster), 1 = FP32 and MIXED, 0 = off
+    // FDK_BP_SYM: unset = FP32 only, 1 = FP32 and MIXED, 0 = off
     const char *env = getenv("FDK_BP_SYM");
     const std::string mode = env ? env : "";
     if (mode == "0") return FDK_OK;
@@ -1346,8 +1374,8 @@ int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const fl
                                                              h->band_tz[k + 1])
                         : lv ? bp_tma_launch<HalfLerp>(h->plan, h->d_vol, h->d_comp, pv, d_mats + m0, host_mats + m0,
                                                      ns, st, lerp_sc, h->band_tz[k], h->band_tz[k + 1])
-                        : bp_tma_launch<float2>(h->plan, h->d_vol, h->d_comp, pv, d_mats + m0, host_mats + m0, ns,
-                                                st, acc_scale, h->band_tz[k], h->band_tz[k + 1]));
+                        : launch_staged_f32(h, pv, d_mats + m0, host_mats + m0, ns, st, acc_scale, h->band_tz[k],
+                                            h->band_tz[k + 1]));
                 h->launches++;
                 continue;
             }
@@ -1368,8 +1396,8 @@ int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const fl
                           : lv ? bp_tma_launch<HalfLerp>(h->plan, h->d_vol, h->d_comp, lv, d_mats, host_mats, ns, st,
                                                        lerp_sc, h->band_tz[k], h->band_tz[k + 1], &vl, &dev->views,
                                                        n_slots)
-                          : bp_tma_launch<float2>(h->plan, h->d_vol, h->d_comp, views, d_mats, host_mats, ns, st,
-                                                  acc_scale, h->band_tz[k], h->band_tz[k + 1], &vl, &dev->views, n_slots);
+                          : launch_staged_f32(h, views, d_mats, host_mats, ns, st, acc_scale, h->band_tz[k],
+                                              h->band_tz[k + 1], &vl, &dev->views, n_slots);
             FDK_TRY(release_list(h, e, st));
             FDK_TRY(r);
             h->launches++;

@@ -9,6 +9,7 @@
 // store.
 #pragma once
 #include "common.h"
+#include "tma_common.cuh"
 
 namespace fdk {
 
@@ -34,14 +35,6 @@ __device__ __forceinline__ float dot_ijkw(const float4 m, const float4 p) {
     s = fma_rz(m.y, p.y, s);
     s = fma_rz(m.z, p.z, s);
     return s;
-}
-
-// Whole part and fraction of x in [0, 2^22): x + 2^23 rounded toward zero holds the whole part in its
-// low bits (floorf and the conversion to int run at a quarter of the FP32 rate).
-__device__ __forceinline__ unsigned whole_part(float x, float &fraction) {
-    const float r = __fadd_rz(x, 8388608.f);
-    fraction = x - (r - 8388608.f);
-    return __float_as_uint(r) - 0x4B000000u;
 }
 
 // What one view has in common for a warp (32 z of one column): computed by the view's lane.

@@ -56,11 +56,18 @@ struct TmaCfg;
 // 512-view batches), though the loop's registers did not change.  A layout with two detector
 // columns per 8-byte element (read by 64-bit loads) measured slower than that FP16 gather: 2133
 // against 2257 GUPS (its doubled boxes halved the views per stage and the kernel spilled).
+// FP32 with voxel and mirror in packed registers (512-view batches, R 12 / 16): 1434 / 1522 GUPS at 256^3,
+// 1756 / 1889 at 512^3, 1579 / 1830 at 2048^3 (scalar arithmetic at R 12: 1257); R 8 1565, R 16 with three
+// stages 1537 at 512^3.  Where the slab holds few tiles the lower tile fills the chip better: 86 x 51 x 58 slices
+// from 22 views 133 / 150 us, so TallFloat2 takes R 16 and bp.cu chooses (tall_tiles).
 #ifndef FDK_TMA_MIXED_R
 #define FDK_TMA_MIXED_R 16
 #endif
 #ifndef FDK_TMA_FP32_R
 #define FDK_TMA_FP32_R 12
+#endif
+#ifndef FDK_TMA_FP32_TALL_R
+#define FDK_TMA_FP32_TALL_R 16
 #endif
 #ifndef FDK_TMA_FP32_S
 #define FDK_TMA_FP32_S 2
@@ -72,6 +79,11 @@ struct TmaCfg<float2> {
     static constexpr int BH = 40;
     static constexpr int NV = 4;
     static constexpr int S = FDK_TMA_FP32_S;
+};
+struct __align__(8) TallFloat2 : float2 {};
+template <>
+struct TmaCfg<TallFloat2> : TmaCfg<float2> {
+    static constexpr int R = FDK_TMA_FP32_TALL_R;
 };
 
 // MIXED views in the interpolation layout: element (u, v) holds e = E(v) 2^-k and d = (E(v+1) -
@@ -291,7 +303,7 @@ __device__ __forceinline__ void fold_lerp_meta(const float (&m)[12], float za, u
     for (int q = 0; q < 12; q++) md.m[q] = f[q];
 }
 
-// One view's contribution to a thread's column: R voxel pairs.
+// One view's contribution to a thread's column, MIXED views in the interpolation layout: R voxel pairs.
 template <typename E>
 __device__ __forceinline__ void column_view(const TmaMeta &md_s, unsigned box, const E *gview, float x, float y,
                                             float zf0, int nu, int nv, float wscale, float (&am)[TmaCfg<E>::R],
@@ -376,6 +388,17 @@ __device__ __forceinline__ void column_view(const TmaMeta &md_s, unsigned box, c
         }
         return;
     }
+}
+
+// The same for FP32 views: voxel and mirror are the two halves of a packed sum (acc).
+template <typename E>
+__device__ __forceinline__ void column_view_f32(const TmaMeta &md_s, unsigned box, const E *gview, float x, float y,
+                                                float zf0, int nu, int nv, float wscale,
+                                                f32x2 (&acc)[TmaCfg<E>::R]) {
+    using C = TmaCfg<E>;
+    constexpr int R = C::R;
+    const MetaRegs md = load_meta(md_s);
+    const float *m = md.m;
     const float w = fmaf(m[8], x, fmaf(m[9], y, m[11]));
     const float rw = __fdividef(1.0f, w);
     const float U = fmaf(m[0], x, fmaf(m[1], y, m[3])) * rw;
@@ -386,41 +409,50 @@ __device__ __forceinline__ void column_view(const TmaMeta &md_s, unsigned box, c
     const float fuf = floorf(U);
     const float fu = U - fuf;
     const int u0 = (int)fuf;
-    const float wa = (1.f - fu) * wt, wb = fu * wt;
+    const float wb = fu * wt;
+    const f32x2 wa2 = pack2f((1.f - fu) * wt, (1.f - fu) * wt), wb2 = pack2f(wb, wb), minus = pack2f(-1.f, -1.f);
+    // the sample's four pairs of detector column u0, row vi: the u-lerps, then the v-lerp
+    auto sample = [&](f32x2 e0, f32x2 e1, f32x2 e2, f32x2 e3, float fv) {
+        const f32x2 c0 = fma2f(e2, wb2, mul2f(e0, wa2)), c1 = fma2f(e3, wb2, mul2f(e1, wa2));
+        return fma2f(pack2f(fv, fv), fma2f(c0, minus, c1), c0);
+    };
+    if (md.staged) {
+        // byte address of row vi in the box, the bits of vi + 2^23 taken off at once (mod 2^32)
+        const unsigned row = box + (unsigned)((u0 - md.u_lo) * C::BW - md.v_lo) * 8u - 0x4B000000u * 8u;
+        if (md.interior) {
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                const float v = fmaf(B, (float)k, A), r = __fadd_rz(v, 8388608.f);
+                const unsigned a = row + __float_as_uint(r) * 8u;
+                acc[k] = add2f(acc[k], sample(lds2f(a), lds2f(a + 8), lds2f(a + C::BW * 8), lds2f(a + C::BW * 8 + 8),
+                                              v - (r - 8388608.f)));
+            }
+            return;
+        }
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            const float v = fmaf(B, (float)k, A), vr = (float)(nv - 1) - v;
+            const bool mv = v >= 0.f && v < (float)(nv - 1), rv = vr >= 0.f && vr < (float)(nv - 1);
+            if (!(mv || rv)) continue;
+            const float vf = fminf(__fadd_rz(v, 8388608.f) - 8388608.f, (float)(nv - 2));  // 0 <= v <= nv - 1 here
+            const unsigned a = row + __float_as_uint(vf + 8388608.f) * 8u;
+            float sm, sr;
+            unpack2f(sample(lds2f(a), lds2f(a + 8), lds2f(a + C::BW * 8), lds2f(a + C::BW * 8 + 8), v - vf), sm, sr);
+            acc[k] = add2f(acc[k], pack2f(mv ? sm : 0.f, rv ? sr : 0.f));
+        }
+        return;
+    }
+    const f32x2 *g = reinterpret_cast<const f32x2 *>(gview) + (long long)u0 * nv;
 #pragma unroll
     for (int k = 0; k < R; k++) {
-        const float v = fmaf(B, (float)k, A);
-        bool mv = true, rv = true;
-        float vf;
-        if (!(md.staged && md.interior)) {
-            const float vr = (float)(nv - 1) - v;
-            mv = v >= 0.f && v < (float)(nv - 1);
-            rv = vr >= 0.f && vr < (float)(nv - 1);
-            if (!(mv || rv)) continue;
-            vf = fminf(floorf(v), (float)(nv - 2));
-        } else {
-            vf = floorf(v);
-        }
-        const int vi = (int)vf;
-        const float fv = v - vf;
-        float2 e0, e1, e2, e3;
-        if (md.staged) {
-            const unsigned a = box + (unsigned)(((u0 - md.u_lo) * C::BW + (vi - md.v_lo)) * 8);
-            e0 = lds64f(a);
-            e1 = lds64f(a + 8);
-            e2 = lds64f(a + C::BW * 8);
-            e3 = lds64f(a + C::BW * 8 + 8);
-        } else {
-            const float2 *g0 = reinterpret_cast<const float2 *>(gview) + (long long)u0 * nv + vi;
-            e0 = __ldg(g0);
-            e1 = __ldg(g0 + 1);
-            e2 = __ldg(g0 + nv);
-            e3 = __ldg(g0 + nv + 1);
-        }
-        const float c0x = fmaf(e2.x, wb, e0.x * wa), c0y = fmaf(e2.y, wb, e0.y * wa);
-        const float c1x = fmaf(e3.x, wb, e1.x * wa), c1y = fmaf(e3.y, wb, e1.y * wa);
-        if (mv) am[k] += fmaf(fv, c1x - c0x, c0x);
-        if (rv) ar[k] += fmaf(fv, c1y - c0y, c0y);
+        const float v = fmaf(B, (float)k, A), vr = (float)(nv - 1) - v;
+        const bool mv = v >= 0.f && v < (float)(nv - 1), rv = vr >= 0.f && vr < (float)(nv - 1);
+        if (!(mv || rv)) continue;
+        const float vf = fminf(floorf(v), (float)(nv - 2));
+        const f32x2 *p = g + (int)vf;
+        float sm, sr;
+        unpack2f(sample(__ldg(p), __ldg(p + 1), __ldg(p + nv), __ldg(p + nv + 1), v - vf), sm, sr);
+        acc[k] = add2f(acc[k], pack2f(mv ? sm : 0.f, rv ? sr : 0.f));
     }
 }
 
@@ -621,8 +653,12 @@ __global__ void __launch_bounds__(288, FDK_TMA_MIN_BLOCKS)
         const float zf0 = (float)(a.z0 + zt);
         if (col_ok) prefetch_column<R>(a.vol, a.comp, ((long long)xi * a.nys + yi) * a.D, a.D, zt);
         float am[R], ar[R];
+        f32x2 acc[is_lerp_v<E> ? 1 : R];  // FP32: voxel and mirror in one register pair
 #pragma unroll
-        for (int k = 0; k < R; k++) am[k] = ar[k] = 0.f;
+        for (int k = 0; k < R; k++) {
+            am[k] = ar[k] = 0.f;
+            if constexpr (!is_lerp_v<E>) acc[k] = 0;
+        }
         for (int c = 0; c < n_chunks; c++, it++) {
             const int s = it % S;
             const unsigned ph = (unsigned)(it / S) & 1u;
@@ -635,14 +671,21 @@ __global__ void __launch_bounds__(288, FDK_TMA_MIN_BLOCKS)
                     const int view = c * NV + l;
                     if (view >= a.n_proj) break;
                     const long long slot = a.list_slot ? __ldg(a.list_slot + view) : view;
-                    column_view<E>(meta[s * NV + l], boxes + (s * NV + l) * BOX, proj + slot * frame, x, y, zf0, a.nu,
-                                   a.nv, a.wscale, am, ar);
+                    if constexpr (is_lerp_v<E>)
+                        column_view<E>(meta[s * NV + l], boxes + (s * NV + l) * BOX, proj + slot * frame, x, y, zf0, a.nu,
+                                       a.nv, a.wscale, am, ar);
+                    else
+                        column_view_f32(meta[s * NV + l], boxes + (s * NV + l) * BOX, proj + slot * frame, x, y, zf0, a.nu,
+                                        a.nv, a.wscale, acc);
                 }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty0 + 8 * s);
         }
         if (col_ok) {
+            if constexpr (!is_lerp_v<E>)
+#pragma unroll
+                for (int k = 0; k < R; k++) unpack2f(acc[k], am[k], ar[k]);
             const float sc = (a.scale ? *a.scale : 1.0f) / a.wscale;
             write_back<R>(a.vol, a.comp, ((long long)xi * a.nys + yi) * a.D, a.D, zt, min(R, a.nzz - zt), sc, am,
                           ar);

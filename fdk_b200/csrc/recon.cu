@@ -68,6 +68,7 @@ struct fdk_recon {
     int ramp = 0;
     std::vector<int> bviews[2];
     int sym_rot = 0;  // quarter-turn kernel's column map (0: not available for this scan)
+    int pair_least = 0;  // views of a batch that have to pair for it to take that kernel (fdk_recon_create)
     double filter_ms = 0;
     long long views = 0;
     long long filter_launches = 0;   // kernel launches of the filter since creation or reset
@@ -91,7 +92,7 @@ long long fdk_bp_launches_internal(const fdk_bp *h);
 int fdk_bp_bp_device_mats_internal(fdk_bp *h, const void *dev_proj, int32_t layout, const float *dev_mats,
                                    int32_t n_proj, const float *host_mats, void *stream, int32_t band);
 int fdk_bp_band_count_internal(const fdk_bp *h);
-int fdk_bp_plan_bands_internal(fdk_bp *h, long long views);
+int fdk_bp_plan_bands_internal(fdk_bp *h, long long views, bool quarter);
 int fdk_bp_check_internal(fdk_bp *h);
 
 namespace {
@@ -160,7 +161,7 @@ int launch_batch(fdk_recon *h, int b, int n, int band) {
                                               h->mats.data() + 12 * first, h->compute, band);
     }
     std::vector<int> s_slot, s_view, q_slot, q_view;
-    if (h->sym_rot) {
+    if (h->sym_rot && n >= h->pair_least) {
         const int q = (int)(h->g.n_proj / 4);
         // (orbit, quarter, slot), grouped by orbit: complete quadruples take one slot per quarter
         std::vector<std::array<int, 3>> e(n);
@@ -186,7 +187,12 @@ int launch_batch(fdk_recon *h, int b, int n, int band) {
                 }
             i = j;
         }
-    } else {
+    }
+    if (!h->sym_rot || (int)q_view.size() < std::max(1, h->pair_least)) {
+        s_slot.clear();
+        s_view.clear();
+        q_slot.clear();
+        q_view.clear();
         for (int i = 0; i < n; i++) {
             s_slot.push_back(i);
             s_view.push_back(vw[i]);
@@ -454,12 +460,23 @@ int fdk_recon_create_slab(fdk_recon **out, const fdk_geometry *g, int64_t top_z,
         if (s == FDK_OK && h->d_scale) s = fdk_bp_set_acc_scale_internal(h->bp, h->d_scale);
         // the quarter-turn kernel where the scan and the grid have the symmetry
         if (s == FDK_OK) s = fdk_bp_sym_setup_internal(h->bp, h->mats.data(), (int)g->n_proj, &h->sym_rot);
+        // The quarter-turn kernel on request (FDK_BP_SYM=1), else where it is the faster one: a batch of 256
+        // paired views or more on a grid of up to 256 (1662 against 1522 GUPS at 256^3).  The staged kernel
+        // is ahead below that (256^3 from 128 and 32 views: 1343 and 1092 against 1224 and 671).  On larger
+        // grids it is near or ahead (2048^3 1830 against 1779 GUPS, 512^3 1889 against 1937 from 512 views
+        // and 1719 against 1551 from 128) and needs no order of views: a 512^3 scan from host memory takes
+        // 41.7 ms with it and 46.7 paired.
+        const char *sym_env = std::getenv("FDK_BP_SYM");
+        if (sym_env && std::string(sym_env) == "1") h->pair_least = 0;
+        else h->pair_least = g->nx <= 256 ? 256 : batch + 1;
         // MIXED: the staged kernel reads each batch converted to the interpolation layout
         if (s == FDK_OK && precision == FDK_BP_MIXED) s = fdk_bp_reserve_lerp_internal(h->bp, h->batch);
         if (s == FDK_OK && precision == FDK_BP_MIXED)
             s = fdk_bp_choose_lerp_box_internal(h->bp, h->mats.data(), (int)g->n_proj);
         // a flush runs the held batch and the filling one
-        if (s == FDK_OK) s = fdk_bp_plan_bands_internal(h->bp, std::min<long long>(g->n_proj, 2ll * batch));
+        if (s == FDK_OK)
+            s = fdk_bp_plan_bands_internal(h->bp, std::min<long long>(g->n_proj, 2ll * batch),
+                                           h->sym_rot && h->pair_least <= batch);
     }
     if (s == FDK_OK) s = wait_stream(h->compute, h->sync_ev[0], "fdk_recon_create");  // set-up copies landed
     if (s != FDK_OK) {

@@ -8,6 +8,58 @@
 
 namespace fdk {
 
+// Whole part and fraction of x in [0, 2^22): x + 2^23 rounded toward zero holds the whole part in its
+// low bits (floorf and the conversion to int run at a quarter of the FP32 rate).
+__device__ __forceinline__ unsigned whole_part(float x, float &fraction) {
+    const float r = __fadd_rz(x, 8388608.f);
+    fraction = x - (r - 8388608.f);
+    return __float_as_uint(r) - 0x4B000000u;
+}
+
+// Pairs of FP32 values in one 64-bit register: a voxel and its mirror take the same weights, so the
+// backprojection's arithmetic is one packed instruction for both, each half rounded as by itself.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2f(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2f(f32x2 a, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+}
+__device__ __forceinline__ f32x2 add2f(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2f_rz(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2f(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2f(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 lds2f(unsigned addr) {
+    f32x2 r;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(r) : "r"(addr));
+    return r;
+}
+
+// 1 / x, the quotient of __fdividef(1, x) where x and 1 / x are normal numbers, without its scaling of others.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 constexpr long long kWaitLimit = 1ll << 26;
 // Sleep between a producer warp's polls of a stage's empty barrier (tuning macro; 0 = spin).  The
 // MIXED staged kernel at 2048^3 measured the same with 256 ns (3167 against 3171 GUPS): try_wait

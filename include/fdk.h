@@ -299,10 +299,11 @@ int fdk_recon_flush(fdk_recon *h);
 int fdk_recon_filter_kind(fdk_recon *h, int32_t *kind);
 /* The backprojection this reconstructor runs: 0 the reference arithmetic (FP32_EXACT), 1 the
  * staged kernel, 2 the staged kernel plus the quarter-turn kernel: views whose partners
- * v + N/4, v + N/2, v + 3N/4 (mod N) are in the same batch are backprojected four at a time
+ * v + N/4, v + N/2, v + 3N/4 (mod N) are in the same batch may be backprojected four at a time
  * with one address computation (a circular scan of N % 4 == 0 views about a square, centred
- * grid).  FP32 uses it by default; MIXED only when the environment sets FDK_BP_SYM=1 (its
- * staged kernel measured faster); FDK_BP_SYM=0 turns it off.  No counterpart in the reference. */
+ * grid).  FP32 sets it up by default and uses it for the batches where it measured faster (256 paired
+ * views or more, on grids of up to 256 x 256 columns); FDK_BP_SYM=1 uses it for every batch that
+ * pairs, in FP32 and MIXED, FDK_BP_SYM=0 never.  No counterpart in the reference. */
 int fdk_recon_bp_kernel(fdk_recon *h, int32_t *kind);
 /* Wait (bounded by timeout_ms; <= 0 means 10 minutes) until every pushed view is backprojected. */
 int fdk_recon_sync(fdk_recon *h, int64_t timeout_ms);

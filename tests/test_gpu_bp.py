@@ -148,6 +148,20 @@ def test_fast_border_views(precision, kernel, nu, nv, monkeypatch):
     assert e <= (1e-5 if precision == "fp32" else 1e-3), e
 
 
+@pytest.mark.parametrize("half", [176, 190, 193])  # 1100, 1200 and 1300 tiles of 16 slices; ragged in both heights
+def test_fp32_tile_heights(half):
+    """FP32 tiles of 12 and of 16 slices, against FP32_EXACT.  A detector coordinate is off by at most four roundings
+    of the detector's size; a sample of white noise moves by 2.2 of its own size per pixel (rms)."""
+    n, nu, nv, views = 160, 40, 44, 5
+    p = small_param(n, nu, nv, views)
+    p.nz = 2 * half
+    top, bot = [0, 0, 0, n, n, half], [0, 0, half, n, n, half]
+    filt, mats = random_views(views, nu, nv, seed=half), p.proj_matrices()
+    got, want = (run_bp(k, p, top, bot, [filt], [mats]) for k in ("fp32", "fp32_exact"))
+    m = knife_edge_mask(p, top, bot[5])
+    assert rel_l2(got[m], want[m]) <= 4 * 2.0 ** -24 * nv * 2.2
+
+
 def test_fast_rejects_non_circular_matrices():
     n = 16
     p = small_param(n, 16, 16, 4)
