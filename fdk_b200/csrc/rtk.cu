@@ -17,6 +17,7 @@
 //    views (width not a multiple of 4 floats, base not 16-byte aligned) or when the environment
 //    sets FDK_RTK_KERNEL=l1.
 #include <string>
+#include <type_traits>
 
 #include "common.h"
 #include "tma_common.cuh"
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(256) rtk_bp_kernel(const float *__restrict__ v
 #pragma unroll
         for (int kk = 0; kk < kRtkR; kk++) {
             const float fk = (float)(k0 + kk);
-            const float rw = __fdividef(1.0f, fmaf(m[10], fk, Z));
+            const float rw = rcp_approx(fmaf(m[10], fk, Z));
             const float u = fmaf(m[2], fk, X) * rw, v = fmaf(m[6], fk, Y) * rw;
             float s = 0.f;
             if (u >= 0.f && u < wm1 && v >= 0.f && v < hm1) {
@@ -159,24 +160,49 @@ __device__ __forceinline__ void rtk_tile_box(const float *m, float xa, float xb,
     if (umin >= 1.f && umax < (float)(W - 2) && vmin >= 1.f && vmax < (float)(H - 2)) md.flags |= kInterior;
 }
 
+// A texel and its right neighbour, and the pair below, of the staged box (a shared-memory address, rows of BW
+// floats) or of the global view; `at`: the element's offset.
+struct RtkBox {
+    unsigned base;
+    static constexpr int row = rtkt::BW;
+    __device__ __forceinline__ void quad(int at, float (&t)[4]) const {
+        const unsigned a = base + 4u * at;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t[0]) : "r"(a));
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t[1]) : "r"(a + 4));
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t[2]) : "r"(a + 4 * row));
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t[3]) : "r"(a + 4 * row + 4));
+    }
+};
+struct RtkGlobal {
+    const float *base;
+    int row;
+    __device__ __forceinline__ void quad(long long at, float (&t)[4]) const {
+        const float *p = base + at;
+        t[0] = __ldg(p);
+        t[1] = __ldg(p + 1);
+        t[2] = __ldg(p + row);
+        t[3] = __ldg(p + row + 1);
+    }
+};
+
 // One view's contribution to a thread's run of R voxels along z at column (X, Y, Z) (the
-// matrix rows evaluated at z = 0).  src: the staged box (pitch BW, origin (u_lo, v_lo)) or the
-// global view (pitch W, origin 0).  CHECK: the per-sample bounds rule of RtkSUBPIXEL and the
-// run's end at nz; without it the caller guarantees both.  ZFREE: u and w are the column's.
-// The arithmetic of every sample is that of rtk_bp_kernel, so results are bit-identical.
-template <bool CHECK, bool ZFREE>
-__device__ __forceinline__ void rtk_view(const float *m, float X, float Y, float Z, int k0, int nk,
-                                         const float *src, int pitch, int u_lo, int v_lo, float wm1, float hm1,
-                                         float (&acc)[rtkt::R]) {
+// matrix rows evaluated at z = 0).  src: the staged box (origin (u_lo, v_lo)) or the global view (origin
+// 0).  CHECK: the per-sample bounds rule of RtkSUBPIXEL and the run's end at nz; without it the caller
+// guarantees both.  ZFREE: u and w are the column's.  The arithmetic of every sample is that of
+// rtk_bp_kernel, so results are bit-identical.
+template <bool CHECK, bool ZFREE, typename Src>
+__device__ __forceinline__ void rtk_view(const float *m, float X, float Y, float Z, int k0, int nk, const Src &src,
+                                         int u_lo, int v_lo, float wm1, float hm1, float (&acc)[rtkt::R]) {
     constexpr int R = rtkt::R;
+    using At = std::conditional_t<std::is_same<Src, RtkBox>::value, int, long long>;
     const float fk0 = (float)k0;  // one conversion per run; the slices add small exact integers
     if constexpr (ZFREE) {
-        const float rw = __fdividef(1.0f, Z);  // fmaf(0, k, Z) == Z
+        const float rw = rcp_approx(Z);         // fmaf(0, k, Z) == Z
         const float u = X * rw;                 // fmaf(0, k, X) == X
         if (!(u >= 0.f && u < wm1)) return;     // every sample of the column is zero
         const float iu = floorf(u);
         const float du = u - iu;
-        const float *col = src + ((int)iu - u_lo) - v_lo * pitch;
+        const At col = (int)iu - u_lo - (At)v_lo * src.row;
 #pragma unroll
         for (int kk = 0; kk < R; kk++) {
             const float fk = fk0 + (float)kk;  // == (float)(k0 + kk): integers below 2^24
@@ -185,28 +211,35 @@ __device__ __forceinline__ void rtk_view(const float *m, float X, float Y, float
             if (!CHECK || (kk < nk && v >= 0.f && v < hm1)) {
                 const float iv = floorf(v);
                 const float dv = v - iv;
-                const float *p0 = col + (int)iv * pitch;
-                const float *p1 = p0 + pitch;
-                const float e0 = fmaf(du, p0[1] - p0[0], p0[0]);
-                const float e1 = fmaf(du, p1[1] - p1[0], p1[0]);
+                float t[4];
+                src.quad(col + (At)(int)iv * src.row, t);
+                const float e0 = fmaf(du, t[1] - t[0], t[0]);
+                const float e1 = fmaf(du, t[3] - t[2], t[2]);
                 sv = fmaf(dv, e1 - e0, e0);
             }
             acc[kk] = fmaf(sv * rw, rw, acc[kk]);
         }
     } else {
+        // u and v as a packed pair, their whole parts by packed additions rounded toward zero: with
+        // floorf and conversions a sample's five quarter-rate instructions take 40 of its clocks.
+        const f32x2 mz = pack2f(m[2], m[6]), XY = pack2f(X, Y), minus = pack2f(-1.f, -1.f);
+        const f32x2 big = pack2f(8388608.f, 8388608.f), less = pack2f(-8388608.f, -8388608.f);
 #pragma unroll
         for (int kk = 0; kk < R; kk++) {
             const float fk = fk0 + (float)kk;  // == (float)(k0 + kk): integers below 2^24
-            const float rw = __fdividef(1.0f, fmaf(m[10], fk, Z));
-            const float u = fmaf(m[2], fk, X) * rw, v = fmaf(m[6], fk, Y) * rw;
-            float sv = 0.f;
+            const float rw = rcp_approx(fmaf(m[10], fk, Z));
+            const f32x2 uv = mul2f(fma2f(mz, pack2f(fk, fk), XY), pack2f(rw, rw));
+            float u, v, sv = 0.f;
+            unpack2f(uv, u, v);
             if (!CHECK || (kk < nk && u >= 0.f && u < wm1 && v >= 0.f && v < hm1)) {
-                const float iu = floorf(u), iv = floorf(v);
-                const float du = u - iu, dv = v - iv;
-                const float *p0 = src + ((int)iv - v_lo) * pitch + ((int)iu - u_lo);
-                const float *p1 = p0 + pitch;
-                const float e0 = fmaf(du, p0[1] - p0[0], p0[0]);
-                const float e1 = fmaf(du, p1[1] - p1[0], p1[0]);
+                const f32x2 r = add2f_rz(uv, big);
+                float ru, rv, du, dv, t[4];
+                unpack2f(r, ru, rv);
+                unpack2f(fma2f(add2f(r, less), minus, uv), du, dv);
+                const At iu = __float_as_int(ru) - (0x4B000000 + u_lo), iv = __float_as_int(rv) - (0x4B000000 + v_lo);
+                src.quad(iv * src.row + iu, t);
+                const float e0 = fmaf(du, t[1] - t[0], t[0]);
+                const float e1 = fmaf(du, t[3] - t[2], t[2]);
                 sv = fmaf(dv, e1 - e0, e0);
             }
             acc[kk] = fmaf(sv * rw, rw, acc[kk]);
@@ -215,8 +248,9 @@ __device__ __forceinline__ void rtk_view(const float *m, float X, float Y, float
 }
 
 // CTAs per SM the register budget is set for (tuning macro).  Measured on 512^3 from 32 views of
-// 512^2: 2 CTAs (96 registers) 910 / 654 GUPS circular / tilted, 3 CTAs (72 registers, no
-// spills) 966 / 671 GUPS; the L1 kernel 602 / 602.
+// 512^2: 2 CTAs 910 / 654 GUPS circular / tilted, 3 CTAs 966 / 671, the L1 kernel 602 / 602; with the
+// packed coordinates of tilted views, 400^3 from 32 views of 512^2 tilted: 2, 3, 4 CTAs 2347, 2298, 2359 us
+// (scalar 2813).
 #ifndef FDK_RTK_MIN_BLOCKS
 #define FDK_RTK_MIN_BLOCKS 3
 #endif
@@ -324,18 +358,18 @@ __global__ void __launch_bounds__(rtkt::THREADS, FDK_RTK_MIN_BLOCKS)
                     const float Z = fmaf(m[8], fi, fmaf(m[9], fj, m[11]));
                     const bool zfree = md.flags & kZFree;
                     if (md.flags & kStaged) {
-                        const float *box = reinterpret_cast<const float *>(smem + (s * NV + l) * BOX);
+                        const RtkBox box{boxes + (unsigned)((s * NV + l) * BOX)};
                         if ((md.flags & kInterior) && nk == R) {
-                            if (zfree) rtk_view<false, true>(m, X, Y, Z, k0, nk, box, BW, md.u_lo, md.v_lo, wm1, hm1, acc);
-                            else rtk_view<false, false>(m, X, Y, Z, k0, nk, box, BW, md.u_lo, md.v_lo, wm1, hm1, acc);
+                            if (zfree) rtk_view<false, true>(m, X, Y, Z, k0, nk, box, md.u_lo, md.v_lo, wm1, hm1, acc);
+                            else rtk_view<false, false>(m, X, Y, Z, k0, nk, box, md.u_lo, md.v_lo, wm1, hm1, acc);
                         } else {
-                            if (zfree) rtk_view<true, true>(m, X, Y, Z, k0, nk, box, BW, md.u_lo, md.v_lo, wm1, hm1, acc);
-                            else rtk_view<true, false>(m, X, Y, Z, k0, nk, box, BW, md.u_lo, md.v_lo, wm1, hm1, acc);
+                            if (zfree) rtk_view<true, true>(m, X, Y, Z, k0, nk, box, md.u_lo, md.v_lo, wm1, hm1, acc);
+                            else rtk_view<true, false>(m, X, Y, Z, k0, nk, box, md.u_lo, md.v_lo, wm1, hm1, acc);
                         }
                     } else {
-                        const float *pv = a.proj + p * frame;
-                        if (zfree) rtk_view<true, true>(m, X, Y, Z, k0, nk, pv, a.W, 0, 0, wm1, hm1, acc);
-                        else rtk_view<true, false>(m, X, Y, Z, k0, nk, pv, a.W, 0, 0, wm1, hm1, acc);
+                        const RtkGlobal view{a.proj + p * frame, a.W};
+                        if (zfree) rtk_view<true, true>(m, X, Y, Z, k0, nk, view, 0, 0, wm1, hm1, acc);
+                        else rtk_view<true, false>(m, X, Y, Z, k0, nk, view, 0, 0, wm1, hm1, acc);
                     }
                 }
             }
