@@ -66,6 +66,35 @@ def test_bp_adjoint_dot_product():
     assert abs(a - b) <= 1e-4 * abs(a), (a, b)
 
 
+@pytest.mark.parametrize("n,nu,nv,views", [(50, 20, 20, 9), (24, 56, 52, 12), (16, 80, 76, 5), (34, 19, 45, 17)])
+def test_bp_adjoint_slices_per_row(n, nu, nv, views):
+    """Several slices per detector row, several rows per slice, odd sizes, views past a multiple of 8.  A detector
+    coordinate of either kernel is off by at most four roundings of the detector's size, which moves a sample of
+    white noise by 2.2 of its own size per pixel (rms); the sum over the volume is held to four of its deviations."""
+    import torch
+
+    p = small_param(n, nu, nv, views)
+    rng = np.random.default_rng(n)
+    rows = torch.from_numpy(rng.standard_normal((views, nv, nu)).astype(np.float32)).cuda()
+    r = torch.from_numpy(rng.standard_normal((n, n, n)).astype(np.float32)).cuda()
+    mats = p.proj_matrices()
+    top, bot = (F.BoxT(0, 0, 0, n, n, n), F.BoxT(0, 0, 0, 0, 0, 0))
+    bp = F.BackProjectionFDK(nv, nu, 32, n, n, n, top, bot)
+    views_t = rows.transpose(1, 2).contiguous()
+    bp.BP_device(views_t.data_ptr(), F.LAYOUT_TRANSPOSED, mats, views)
+    vol = bp.GetVolumeData().reshape(-1).astype(np.float64).copy()
+    bp.close()
+    grad = torch.zeros_like(rows)
+    d_mats = torch.from_numpy(mats.reshape(-1)).cuda()
+    g = p.to_c()
+    check(lib().fdk_bp_adjoint(C.byref(g), r.data_ptr(), d_mats.data_ptr(), views, grad.data_ptr(), None))
+    torch.cuda.synchronize()
+    a = float((vol * r.cpu().numpy().reshape(-1).astype(np.float64)).sum())
+    b = float((rows.double() * grad.double()).sum())
+    rel = 2 * 4 * 2.0 ** -24 * max(nu, nv) * 2.2
+    assert abs(a - b) <= 4 * rel * float(np.linalg.norm(vol)), (a, b)
+
+
 def test_network_kernels_vs_cpu_oracle():
     import torch
 
