@@ -47,6 +47,11 @@ __device__ __forceinline__ f32x2 fma2f(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+__device__ __forceinline__ f32x2 fma2f_rz_ftz(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rz.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 __device__ __forceinline__ f32x2 lds2f(unsigned addr) {
     f32x2 r;
     asm volatile("ld.shared.b64 %0, [%1];" : "=l"(r) : "r"(addr));
