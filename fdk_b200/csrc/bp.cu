@@ -174,17 +174,32 @@ __global__ void to_lerp_kernel(const __half2 *__restrict__ src, HalfLerp *__rest
     const int k = (M > 0.f && M < 65536.f) ? ilogbf(M) + 1 : 0;  // M is an FP16 magnitude: -23 <= k <= 16
     const float se = pow2i(-k), sd = pow2i(14 - k);
     if (blockIdx.x == 0 && threadIdx.x == 0) *out_scale = (acc_scale ? *acc_scale : 1.0f) * pow2i(k);
-    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-        const __half2 *s = src + r * nv;
-        HalfLerp *d = dst + r * nv;
-        for (int v = threadIdx.x; v < nv; v += blockDim.x) {
-            const float2 e0 = __half22float2(s[v]);
-            const float2 e1 = v + 1 < nv ? __half22float2(s[v + 1]) : e0;
-            HalfLerp o;
-            o.e = __floats2half2_rn(e0.x * se, e0.y * se);
-            o.d = __floats2half2_rn((e1.x - e0.x) * sd, (e1.y - e0.y) * sd);
-            d[v] = o;
+    // 4 pairs a thread and step: nv is a multiple of 4 (the 16-byte rule of the TMA rows).  64 views of
+    // 2048^2: 707 us a pair at a time, 658 so.
+    const int groups = nv / 4;
+    const long long stride = (long long)gridDim.x * blockDim.x, total = rows * groups;
+    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    int c = (int)(i % groups);  // the group's place in its row
+    const int step = (int)(stride % groups);
+    for (; i < total; i += stride) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+        const unsigned w[5] = {q.x, q.y, q.z, q.w,
+                               c + 1 < groups ? __ldg(reinterpret_cast<const unsigned *>(src) + 4 * i + 4) : q.w};
+        float2 e[5];
+#pragma unroll
+        for (int j = 0; j < 5; j++) e[j] = __half22float2(*reinterpret_cast<const __half2 *>(&w[j]));
+        __half2 o[8];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            o[2 * j] = __floats2half2_rn(e[j].x * se, e[j].y * se);
+            o[2 * j + 1] = __floats2half2_rn((e[j + 1].x - e[j].x) * sd, (e[j + 1].y - e[j].y) * sd);
         }
+        const unsigned *u = reinterpret_cast<const unsigned *>(o);
+        uint4 *d = reinterpret_cast<uint4 *>(dst) + 2 * i;
+        d[0] = make_uint4(u[0], u[1], u[2], u[3]);
+        d[1] = make_uint4(u[4], u[5], u[6], u[7]);
+        c += step;
+        if (c >= groups) c -= groups;
     }
 }
 
@@ -369,7 +384,8 @@ int convert_lerp(fdk_bp *h, const void *src, HalfLerp *dst, long long n_views, i
     absmax_half2_kernel<<<(int)std::min<long long>(ceil_div(pairs / 4 + 1, 256), 148 * 8), 256, 0, st>>>(
         static_cast<const __half2 *>(src), pairs, lerp_absmax(h, j));
     FDK_CUDA(cudaGetLastError());
-    to_lerp_kernel<<<(int)std::min<long long>(rows, 148 * 16), 256, 0, st>>>(
+    FDK_CHECK_ARG(h->plan.nv % 4 == 0, "rows of %d pairs are not whole 16-byte words", h->plan.nv);
+    to_lerp_kernel<<<(int)std::min<long long>(ceil_div(pairs / 4, 256), 148 * 8), 256, 0, st>>>(
         static_cast<const __half2 *>(src), dst, rows, h->plan.nv, lerp_absmax(h, j), acc_scale, lerp_scale(h, j));
     FDK_CUDA(cudaGetLastError());
     h->launches += 2;

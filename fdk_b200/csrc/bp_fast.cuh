@@ -290,11 +290,30 @@ __global__ void __launch_bounds__(256) bp_fast_kernel(BpFastArgs a) {
     }
 }
 
-// Adds the compensation term into the volume and clears it (before the volume is read).
-__global__ void fold_comp_kernel(float *vol, float *comp, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        vol[i] -= comp[i];
-        comp[i] = 0.f;
+// Adds the compensation term into the volume and clears it (before the volume is read).  HBM-bound: two
+// 16-byte loads of each array in flight a thread (2 GiB of each: 1.92 ms by single floats, 1.43, 6.0 TB/s).  Both
+// arrays start on a 16-byte boundary.
+__global__ void __launch_bounds__(256) fold_comp_kernel(float *__restrict__ vol, float *__restrict__ comp, long long n) {
+    const long long n4 = n / 4, stride = (long long)gridDim.x * blockDim.x;
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    float4 *v4 = reinterpret_cast<float4 *>(vol), *c4 = reinterpret_cast<float4 *>(comp);
+    const auto less = [](float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    long long i = t;
+    for (; i + stride < n4; i += 2 * stride) {
+        const float4 a = v4[i], b = v4[i + stride], c = c4[i], d = c4[i + stride];
+        v4[i] = less(a, c);
+        v4[i + stride] = less(b, d);
+        c4[i] = zero;
+        c4[i + stride] = zero;
+    }
+    if (i < n4) {
+        v4[i] = less(v4[i], c4[i]);
+        c4[i] = zero;
+    }
+    if (4 * n4 + t < n) {  // at most three
+        vol[4 * n4 + t] -= comp[4 * n4 + t];
+        comp[4 * n4 + t] = 0.f;
     }
 }
 
