@@ -134,8 +134,11 @@ struct Fft {
 __host__ __device__ constexpr int slot(int p) { return p + (p >> 4); }
 
 // Row pairs (r, nv-1-r), r = G * blockIdx.x + g, g < G, of view blockIdx.y.
-template <int LOG2W, int G, bool GATHER>
-__global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) filter_kernel(const FilterArgs a) {
+// FEW: for calls of few CTAs, which are one chain of latencies: all that the passes read from global memory is
+// asked for at the start and kept in registers (121 to 167 of them).  2 views of 33 rows to MIRROR FP16, rows of
+// 200, 1000 and 2048: 8.2, 10.3 and 10.4 us before, 6.3, 8.2 and 10.3 so.
+template <int LOG2W, int G, bool GATHER, bool FEW>
+__global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blocks(G)) filter_kernel(const FilterArgs a) {
     using F = Fft<LOG2W>;
     constexpr int W = F::W, E = F::E, TPF = F::TPF, RL = F::RL, THREADS = TPF * G;
     extern __shared__ __align__(16) float2 fsm[];
@@ -158,6 +161,27 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) fi
     const float *w1 = a.cos ? a.cos + (long long)r1 * a.cos_pitch : nullptr;
     const float *w2 = a.cos ? a.cos + (long long)r2 * a.cos_pitch : nullptr;
     const int c0 = t - a.off;  // this thread's first column
+    float4 early[2][8], hearly[4];  // FEW: the twiddles of the two loaded passes, the response
+    float ex[4], ew[4];             // and the samples of one pad
+    if constexpr (FEW) {
+        if (t < 4) {
+            const float *p = t < 2 ? p1 : p2, *w = t < 2 ? w1 : w2;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < a.pad_n) {
+                    const int c = (t & 1) ? a.nu - 1 - k : k;
+                    ex[k] = __ldg(p + c);
+                    if (w) ew[k] = __ldg(w + c);
+                }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            early[0][k] = load_here(reinterpret_cast<const float4 *>(a.twp) + t + k * TPF);
+            if constexpr (F::MID) early[1][k] = load_here(reinterpret_cast<const float4 *>(a.twp + W) + t % RL + k * RL);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) hearly[q] = load_here(reinterpret_cast<const float4 *>(a.hb) + t + q * TPF);
+    }
     float2 v[E];
 #pragma unroll
     for (int m = 0; m < E; m++)
@@ -170,7 +194,16 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) fi
                 v[m] = make_float2(__fmul_rn(v[m].x, __ldg(w1 + c0 + m * TPF)), __fmul_rn(v[m].y, __ldg(w2 + c0 + m * TPF)));
     }
     // the pads: means of the first and last pad_n weighted samples
-    for (int q = t; q < 4; q += TPF) {
+    if constexpr (FEW) {
+        if (t < 4) {
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < a.pad_n) s += w1 ? __fmul_rn(ex[k], ew[k]) : ex[k];
+            pads[g][t] = s / (float)a.pad_n;
+        }
+    }
+    for (int q = t; !FEW && q < 4; q += TPF) {
         const float *p = q < 2 ? p1 : p2, *w = q < 2 ? w1 : w2;
         float s = 0.f;
         for (int k = 0; k < a.pad_n; k++) {
@@ -199,6 +232,14 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) fi
             for (int h = E / 2; h; h >>= 1)
 #pragma unroll
                 for (int j = 0; j < h; j++) tq[E - 2 * h + j] = __ldg(a.tw + (i + j * n) * (E / 2 / h) * (TPF / n));
+        } else if constexpr (FEW) {
+            const bool mid = n != TPF;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float4 f = mid ? early[1][k] : early[0][k];
+                tq[2 * k] = make_float2(f.x, f.y);
+                tq[2 * k + 1] = make_float2(f.z, f.w);
+            }
         } else {
             const float4 *q = reinterpret_cast<const float4 *>(plane) + i;
 #pragma unroll
@@ -240,7 +281,7 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, Fft<LOG2W>::blocks(G)) fi
         const float4 *h4 = reinterpret_cast<const float4 *>(a.hb) + t;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            const float4 h = __ldg(h4 + q * TPF);
+            const float4 h = FEW ? hearly[q] : __ldg(h4 + q * TPF);
             v[4 * q] = make_float2(__fmul_rn(v[4 * q].x, h.x), __fmul_rn(v[4 * q].y, h.x));
             v[4 * q + 1] = make_float2(__fmul_rn(v[4 * q + 1].x, h.y), __fmul_rn(v[4 * q + 1].y, h.y));
             v[4 * q + 2] = make_float2(__fmul_rn(v[4 * q + 2].x, h.z), __fmul_rn(v[4 * q + 2].y, h.z));
@@ -438,15 +479,15 @@ void FilterTables::release() {
     hb = nullptr;
 }
 
-template <int LOG2W, int G, bool GATHER>
+template <int LOG2W, int G, bool GATHER, bool FEW = false>
 static int launch_group(const FilterArgs &a, int n_views, cudaStream_t st) {
     using F = Fft<LOG2W>;
     const int smem = (int)sizeof(float2) * std::max(F::TPF > 1 ? F::PITCH * G : 0, a.layout != FDK_LAYOUT_ROWS ? a.nu * G : 0);
     // per device and size, and needed at 48 KB too (the kernel also has static shared memory):
     // cheap, so set on every launch
     if (smem > 40 * 1024)
-        FDK_CUDA(cudaFuncSetAttribute(filter_kernel<LOG2W, G, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    filter_kernel<LOG2W, G, GATHER><<<dim3((unsigned)ceil_div(a.n_pairs, G), n_views), F::TPF * G, smem, st>>>(a);
+        FDK_CUDA(cudaFuncSetAttribute(filter_kernel<LOG2W, G, GATHER, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    filter_kernel<LOG2W, G, GATHER, FEW><<<dim3((unsigned)ceil_div(a.n_pairs, G), n_views), F::TPF * G, smem, st>>>(a);
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
 }
@@ -458,7 +499,8 @@ static int launch_group(const FilterArgs &a, int n_views, cudaStream_t st) {
 // below, where G is 4 or more anyway (1500 x 1000 to MIRROR FP16 at 512 / 256 threads: 226 / 236 us).
 // ROWS stores are coalesced at any G, and smaller CTAs overlap each other's loads and transforms
 // better (48 views of 1536 x 1024 at 512 / 256 threads: 285 / 260 us).  A call whose CTAs would
-// not give every SM two takes the smallest group of whole warps, for more CTAs.
+// not give every SM two takes the smallest group of whole warps, for more CTAs, and FEW from 128 points on
+// (below, a thread holds too few points for its planes).
 static int launch_filter(const FilterArgs &a, int log2W, int n_views, cudaStream_t st) {
     return with_length(log2W, [&](auto l) {
         constexpr int L = decltype(l)::value, TPF = Fft<L>::TPF;
@@ -466,7 +508,7 @@ static int launch_filter(const FilterArgs &a, int log2W, int n_views, cudaStream
         constexpr int least = std::max(1, std::min(64 / TPF, 16));
         const int g = a.layout == FDK_LAYOUT_ROWS ? rows : cols;
         if (!a.twp) return launch_group<L, least, true>(a, n_views, st);
-        if (ceil_div(a.n_pairs, g) * n_views < 2 * 148) return launch_group<L, least, false>(a, n_views, st);
+        if (ceil_div(a.n_pairs, g) * n_views < 2 * 148) return launch_group<L, least, false, (L >= 7)>(a, n_views, st);
         if (g == rows) return launch_group<L, rows, false>(a, n_views, st);
         return launch_group<L, cols, false>(a, n_views, st);
     });
