@@ -519,6 +519,7 @@ int filter_views(const float *src, int src_pitch, long long src_vstride, void *d
                  long long dst_vstride, const float *cos, int cos_pitch, const FilterTables &t, int nu,
                  int nv, int pad_n, int n_views, int layout, int dtype, cudaStream_t st, float out_scale,
                  unsigned int *overflow) {
+    FDK_CHECK_ARG(((uintptr_t)t.hb & 15) == 0 && ((uintptr_t)t.twp & 15) == 0, "filter tables must start on 16-byte boundaries");
     FilterArgs a;
     a.src = src;
     a.dst = dst;
@@ -716,11 +717,12 @@ int fdk_filter_row_real32(const fdk_dataref *src, fdk_dataref *dst, const fdk_da
     FilterTables t;
     t.W = W;
     while ((1 << t.log2W) < W) t.log2W++;
+    // The response first: W floats are whole 16-byte words (W >= 4), which the kernel reads both tables by.
     const size_t planes = (size_t)W + W / 16;
     Scratch tables;
-    FDK_TRY(tables.alloc(sizeof(float2) * planes + sizeof(float) * W, cudaStreamLegacy));
-    t.twp = static_cast<float2 *>(tables.p);
-    t.hb = reinterpret_cast<float *>(t.twp + planes);
+    FDK_TRY(tables.alloc(sizeof(float) * W + sizeof(float2) * planes, cudaStreamLegacy));
+    t.hb = static_cast<float *>(tables.p);
+    t.twp = reinterpret_cast<float2 *>(t.hb + W);
     FDK_TRY(filter_tables_on_device(filter->data, t, cudaStreamLegacy));
     FDK_TRY(filter_views(src->data, src->pitch, (long long)src->pitch * src->height, dst->data, dst->pitch,
                          (long long)dst->pitch * dst->height, nullptr, 0, t, src->width, src->height, 3, src->depth,

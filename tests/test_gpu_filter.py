@@ -132,3 +132,32 @@ def test_every_length_and_group(nu, nv, views):
                 assert max_rel(got[..., 1], want[:, :, ::-1]) <= tol
                 got = got[..., 0]
             assert max_rel(got, want) <= tol, (layout, dtype)
+
+
+@pytest.mark.parametrize("log2w", range(2, 13))
+@pytest.mark.parametrize("nv,views", [(1, 1), (7, 2), (37, 40)])
+def test_row_entry_points_over_every_length(log2w, nv, views):
+    """filter_row_real32 and its no-allocation form at every filter length they take (4 .. 4096), the shortest
+    and the longest rows of each, against the FP64 oracle.  Tolerance: that of the tests above (FP32 transforms
+    of up to 12 index bits each way)."""
+    import ctypes as C
+
+    import torch
+
+    from fdk_b200._lib import DataRef, check, lib
+
+    W = 1 << log2w
+    for nu in (max(3, W // 2 + 1), W):
+        rng = np.random.default_rng(W * 100 + nv)
+        H = O.filter_design("hann", W // 2)  # W taps
+        assert H.size == W
+        src = torch.from_numpy((rng.standard_normal((views, nv, nu)) + 2.0).astype(np.float32)).cuda()
+        filt = torch.from_numpy(H.astype(np.float32)).cuda()
+        want = np.stack([O.filter_view(v, H, None, pad_n=3) for v in src.cpu().numpy()])
+        out = torch.full_like(src, 7.0)
+        F.filter_row_real32(src, out, filt)
+        assert max_rel(out.cpu().numpy(), want) <= 3e-6
+        again = torch.full_like(src, 7.0)
+        ref = [C.byref(DataRef(t.data_ptr(), t.shape[-1], nv, views, t.shape[-1])) for t in (src, again)]
+        check(lib().fdk_filter_row_real32_noalloc(*ref, C.byref(DataRef(filt.data_ptr(), W, 1, 1, W))))
+        assert max_rel(again.cpu().numpy(), want) <= 3e-6
