@@ -13,6 +13,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "internal.h"
 #include "scratch.h"
 
 namespace fdk {
@@ -168,6 +169,7 @@ extern "C" int fdk_forward_project(const fdk_geometry *g, const float *dev_vol, 
     FDK_CHECK_ARG(g && dev_vol && dev_out, "NULL argument");
     FDK_CHECK_ARG(first >= 0 && n > 0 && first + n <= g->n_proj && n <= 65535, "view range out of bounds");
     FDK_CHECK_ARG(g->nu * g->nv < (1ll << 31), "detector too large");
+    FDK_TRY(check_geometry(g));
     cudaStream_t st = (cudaStream_t)stream;
     FprojArgs a;
     a.vol = dev_vol;

@@ -29,7 +29,7 @@ void set_error(const char *fmt, ...) {
 void clear_error() { g_last_error.clear(); }
 const char *last_error() { return g_last_error.c_str(); }
 
-static int check_geometry(const fdk_geometry *g) {
+int check_geometry(const fdk_geometry *g) {
     FDK_CHECK_ARG(g != nullptr, "geometry is NULL");
     FDK_CHECK_ARG(g->nx > 0 && g->ny > 0 && g->nz > 0, "volume size must be positive");
     FDK_CHECK_ARG(g->nu > 0 && g->nv > 0, "detector size must be positive");

@@ -9,6 +9,10 @@ namespace fdk {
 // FP64 3x4 projection matrix of CalculateProjMat for view angle a (geometry.cpp).
 void projection_matrix(const fdk_geometry &g, double a, double *m);
 
+// FDK_ERR_INVALID_ARG for a geometry without positive sizes, pitches and view count, SOD below SID and a known
+// window (geometry.cpp).  The kernels that take a geometry rely on it.
+int check_geometry(const fdk_geometry *g);
+
 // Device tables of one filter length (filter.cu).
 struct FilterTables {
     int W = 0, log2W = 0;

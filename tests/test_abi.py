@@ -61,3 +61,18 @@ def test_no_device_is_an_error_not_a_crash():
     assert rc in (-2, -6) and not h.value
     with pytest.raises(F.FdkError):
         F.Reconstructor(F.config("c1"), "mixed")
+
+
+NO_MEMORY = 16  # a device pointer that nothing may follow
+
+
+@pytest.mark.skipif(F.device_count() > 0, reason="must not reach a GPU")
+@pytest.mark.parametrize("field,value", [(f, v) for f in ("nx", "ny", "nz", "nu", "nv") for v in (0, -1)] +
+                         [(f, v) for f in ("dx", "dy", "dz", "du", "dv") for v in (0.0, -1.0, float("nan"))] +
+                         [("sod", 1500.0), ("sod", 2000.0), ("sod", 0.0), ("filter_type", 9), ("n_proj", 0)])
+def test_forward_projector_refuses_geometries_that_have_no_rays(field, value):
+    """A pitch of 0 would step along a ray for ever, a size of 0 read outside the volume: refused before any
+    device call."""
+    g = F.config("c1").to_c()
+    setattr(g, field, value)
+    assert F.lib().fdk_forward_project(C.byref(g), NO_MEMORY, 0, 1, NO_MEMORY, None) == -1
