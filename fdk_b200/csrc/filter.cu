@@ -11,7 +11,7 @@
 // FFT: radix-2 decimation in frequency (natural -> bit-reversed order), multiply by H, radix-2
 // decimation in time back.  W / 16 threads hold the W points of a row pair in registers, 16 each, and
 // run the stages four at a time: the 16 points that differ in four adjacent index bits form a closed
-// group (W = 16 x 16 x W/256, 4096 = 16^3).
+// group (W = 16 x 16 x W/256, 4096 = 16^3).  Calls of few rows take 4 or 8 points a thread instead (launch_filter).
 // The samples go from global memory straight into the first pass's registers and from the last
 // pass's registers out again, the spectrum is multiplied by H between the forward and the inverse
 // half of the innermost pass, and so a row pair crosses shared memory four times in all.  Bound:
@@ -112,17 +112,18 @@ struct Roots {
     }
 };
 
-// Passes of a W-point transform: 16 points over stride W / 16, then (W > 256) 16 over stride W / 256, then
-// RL contiguous ones.
-template <int LOG2W>
+// Passes of a W-point transform by threads of E = 2^LOG2E points: E points over stride W / E, then over W / E^2
+// and so on, then RL contiguous ones.
+template <int LOG2W, int LOG2E>
 struct Fft {
     static constexpr int W = 1 << LOG2W;
-    static constexpr int E = W < 16 ? W : 16;       // points per thread, and of the first pass
-    static constexpr int TPF = W / E;               // threads per transform
-    static constexpr bool MID = W > 256;            // a middle pass
-    static constexpr int RL = MID ? W / 256 : TPF;  // points of the last pass (1: none)
+    static constexpr int E = LOG2W < LOG2E ? W : 1 << LOG2E;                // points per thread
+    static constexpr int TPF = W / E;                                       // threads per transform
+    static constexpr int PASSES = LOG2W > LOG2E ? (LOG2W - 1) / LOG2E : 0;  // strided passes
+    static constexpr int RL = W >> (PASSES * LOG2E);                        // points of the last pass
+    __host__ __device__ static constexpr int stride(int pass) { return W >> ((pass + 1) * LOG2E); }
     // shared-memory slots of one transform: one float2 of padding per 16, so that the contiguous
-    // runs of the last pass (16 points a thread) and the strided ones of the others are all free
+    // runs of the last pass and the strided ones of the others are (16 points a thread) all free
     // of bank conflicts
     static constexpr int PITCH = W + W / 16;
     // CTAs per SM that the register budget is set for: 1024 threads of 64 registers
@@ -133,14 +134,21 @@ struct Fft {
 // multiple of d, it is slot(i) + slot(q): the passes' slots are one address and constants.
 __host__ __device__ constexpr int slot(int p) { return p + (p >> 4); }
 
+enum class Twiddles {
+    Planes,  // the passes' planes, each pass's loaded as it begins
+    Roots,   // gathered from tw, each pass's as it begins
+    // All asked for at the start and kept in registers, as are the response and the pads' samples: from the planes
+    // with 16 points a thread (pairs by 16-byte loads), else gathered from tw.
+    Early
+};
+
 // Row pairs (r, nv-1-r), r = G * blockIdx.x + g, g < G, of view blockIdx.y.
-// FEW: for calls of few CTAs, which are one chain of latencies: all that the passes read from global memory is
-// asked for at the start and kept in registers (121 to 167 of them).  2 views of 33 rows to MIRROR FP16, rows of
-// 200, 1000 and 2048: 8.2, 10.3 and 10.4 us before, 6.3, 8.2 and 10.3 so.
-template <int LOG2W, int G, bool GATHER, bool FEW>
-__global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blocks(G)) filter_kernel(const FilterArgs a) {
-    using F = Fft<LOG2W>;
-    constexpr int W = F::W, E = F::E, TPF = F::TPF, RL = F::RL, THREADS = TPF * G;
+template <int LOG2W, int LOG2E, int G, Twiddles TW>
+__global__ void __launch_bounds__(Fft<LOG2W, LOG2E>::TPF * G, TW == Twiddles::Early ? 1 : Fft<LOG2W, LOG2E>::blocks(G))
+    filter_kernel(const FilterArgs a) {
+    using F = Fft<LOG2W, LOG2E>;
+    constexpr bool EARLY = TW == Twiddles::Early;
+    constexpr int W = F::W, E = F::E, TPF = F::TPF, RL = F::RL, THREADS = TPF * G, PASSES = F::PASSES;
     extern __shared__ __align__(16) float2 fsm[];
     __shared__ float pads[G][4];
     const int g = threadIdx.x / TPF, t = threadIdx.x % TPF;
@@ -161,9 +169,36 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blo
     const float *w1 = a.cos ? a.cos + (long long)r1 * a.cos_pitch : nullptr;
     const float *w2 = a.cos ? a.cos + (long long)r2 * a.cos_pitch : nullptr;
     const int c0 = t - a.off;  // this thread's first column
-    float4 early[2][8], hearly[4];  // FEW: the twiddles of the two loaded passes, the response
-    float ex[4], ew[4];             // and the samples of one pad
-    if constexpr (FEW) {
+
+    // The twiddles of a strided pass: E/2 of its first stage, E/4 of the next and so on, for the thread's place
+    // i < n in a block (n: the pass's stride).  In the planes as float4 pairs, pair-major; in tw entry j of the
+    // stage of half-width h is root (i + j n) E/2h of the pass's, which are every (TPF / n)-th.
+    float2 early[EARLY && PASSES ? PASSES : 1][E], tq[E];
+    auto fetch = [&](float2 (&q)[E], int pass) {
+        const int n = F::stride(pass), i = t % n;
+        if constexpr (TW == Twiddles::Roots || E < 16) {
+#pragma unroll
+            for (int h = E / 2; h; h >>= 1)
+#pragma unroll
+                for (int j = 0; j < h; j++) q[E - 2 * h + j] = __ldg(a.tw + (i + j * n) * (E / 2 / h) * (TPF / n));
+        } else {
+            const float4 *plane = reinterpret_cast<const float4 *>(a.twp + (pass ? W : 0)) + i;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float4 f = load_here(plane + k * n);
+                q[2 * k] = make_float2(f.x, f.y);
+                q[2 * k + 1] = make_float2(f.z, f.w);
+            }
+        }
+    };
+    // Four neighbouring entries of the response: quad q of the thread's E points (FilterTables)
+    auto response = [&](int q) {
+        return __ldg(reinterpret_cast<const float4 *>(a.hb) + (t * E % 16) / 4 * (W / 16) + t * E / 16 + q * (W / 16));
+    };
+    float4 hearly[4];
+    constexpr bool PADS_EARLY = EARLY && TPF >= 4;
+    float ex[4], ew[4];
+    if constexpr (PADS_EARLY) {
         if (t < 4) {
             const float *p = t < 2 ? p1 : p2, *w = t < 2 ? w1 : w2;
 #pragma unroll
@@ -174,13 +209,13 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blo
                     if (w) ew[k] = __ldg(w + c);
                 }
         }
+    }
+    if constexpr (EARLY) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            early[0][k] = load_here(reinterpret_cast<const float4 *>(a.twp) + t + k * TPF);
-            if constexpr (F::MID) early[1][k] = load_here(reinterpret_cast<const float4 *>(a.twp + W) + t % RL + k * RL);
-        }
+        for (int p = 0; p < PASSES; p++) fetch(early[p], p);
+        if constexpr (W >= 16)
 #pragma unroll
-        for (int q = 0; q < 4; q++) hearly[q] = load_here(reinterpret_cast<const float4 *>(a.hb) + t + q * TPF);
+            for (int q = 0; q < E / 4; q++) hearly[q] = response(q);
     }
     float2 v[E];
 #pragma unroll
@@ -194,7 +229,7 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blo
                 v[m] = make_float2(__fmul_rn(v[m].x, __ldg(w1 + c0 + m * TPF)), __fmul_rn(v[m].y, __ldg(w2 + c0 + m * TPF)));
     }
     // the pads: means of the first and last pad_n weighted samples
-    if constexpr (FEW) {
+    if constexpr (PADS_EARLY) {
         if (t < 4) {
             float s = 0.f;
 #pragma unroll
@@ -202,17 +237,18 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blo
                 if (k < a.pad_n) s += w1 ? __fmul_rn(ex[k], ew[k]) : ex[k];
             pads[g][t] = s / (float)a.pad_n;
         }
-    }
-    for (int q = t; !FEW && q < 4; q += TPF) {
-        const float *p = q < 2 ? p1 : p2, *w = q < 2 ? w1 : w2;
-        float s = 0.f;
-        for (int k = 0; k < a.pad_n; k++) {
-            const int c = (q & 1) ? a.nu - 1 - k : k;
-            float x = __ldg(p + c);
-            if (w) x *= __ldg(w + c);
-            s += x;
+    } else {
+        for (int q = t; q < 4; q += TPF) {
+            const float *p = q < 2 ? p1 : p2, *w = q < 2 ? w1 : w2;
+            float s = 0.f;
+            for (int k = 0; k < a.pad_n; k++) {
+                const int c = (q & 1) ? a.nu - 1 - k : k;
+                float x = __ldg(p + c);
+                if (w) x *= __ldg(w + c);
+                s += x;
+            }
+            pads[g][q] = s / (float)a.pad_n;
         }
-        pads[g][q] = s / (float)a.pad_n;
     }
     meet();
 #pragma unroll
@@ -222,66 +258,41 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blo
         else if (c >= a.nu) v[m] = make_float2(pads[g][1], pads[g][3]);
     }
 
-    // The twiddles of a pass: 8 + 4 + 2 + 1 of the first to the last stage of its four, for the thread's place
-    // i < n in a block (n: the pass's stride).  plane: as float4 pairs, pair-major; gathered: entry j of the
-    // stage of half-width h is root (i + j n) 8/h of the pass's, which are every (TPF / n)-th of tw.
-    float2 tq[16];
-    auto load_twiddles = [&](const float2 *plane, int n, int i) {
-        if constexpr (GATHER) {
+    auto load_twiddles = [&](int pass) {
+        if constexpr (EARLY) {
 #pragma unroll
-            for (int h = E / 2; h; h >>= 1)
-#pragma unroll
-                for (int j = 0; j < h; j++) tq[E - 2 * h + j] = __ldg(a.tw + (i + j * n) * (E / 2 / h) * (TPF / n));
-        } else if constexpr (FEW) {
-            const bool mid = n != TPF;
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const float4 f = mid ? early[1][k] : early[0][k];
-                tq[2 * k] = make_float2(f.x, f.y);
-                tq[2 * k + 1] = make_float2(f.z, f.w);
-            }
+            for (int j = 0; j < E - 1; j++) tq[j] = early[pass][j];
         } else {
-            const float4 *q = reinterpret_cast<const float4 *>(plane) + i;
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const float4 f = load_here(q + k * n);
-                tq[2 * k] = make_float2(f.x, f.y);
-                tq[2 * k + 1] = make_float2(f.z, f.w);
-            }
+            fetch(tq, pass);
         }
     };
     auto loaded = [&](auto conj, float2 x, int h, int j) { return cmul<decltype(conj)::value>(x, tq[E - 2 * h + j]); };
-    float2 *outer = buf + slot(t);                               // points t + k TPF
-    float2 *middle = buf + slot((t / RL) * (E * RL)) + t % RL;  // points of the middle pass, RL apart
-    float2 *inner = buf + slot(t * E);                           // the last pass's run of points
+    // the thread's points of the strided passes, slot(k stride) apart, and its run of points of the last pass
+    float2 *at[PASSES + 1], *inner = buf + slot(t * E);
+#pragma unroll
+    for (int p = 0; p < PASSES; p++) at[p] = buf + slot(t / F::stride(p) * (E * F::stride(p))) + slot(t % F::stride(p));
 
-    if constexpr (TPF > 1) {
-        load_twiddles(a.twp, TPF, t);
+#pragma unroll
+    for (int p = 0; p < PASSES; p++) {
+        const int n = F::stride(p);
+        if (p)
+#pragma unroll
+            for (int k = 0; k < E; k++) v[k] = at[p][slot(k * n)];
+        load_twiddles(p);
         dif<E>(v, 0, loaded);
 #pragma unroll
-        for (int k = 0; k < E; k++) outer[slot(k * TPF)] = v[k];
+        for (int k = 0; k < E; k++) at[p][slot(k * n)] = v[k];
         meet();
-        if constexpr (F::MID) {
-#pragma unroll
-            for (int k = 0; k < E; k++) v[k] = middle[slot(k * RL)];
-            load_twiddles(a.twp + W, RL, t % RL);
-            dif<E>(v, 0, loaded);
-#pragma unroll
-            for (int k = 0; k < E; k++) middle[slot(k * RL)] = v[k];
-            meet();
-        }
+    }
+    if constexpr (PASSES > 0)
 #pragma unroll
         for (int k = 0; k < E; k++) v[k] = inner[k];
 #pragma unroll
-        for (int b = 0; b < E; b += RL) dif<RL>(v, b, Roots{});
-    } else {
-        dif<E>(v, 0, Roots{});
-    }
-    if constexpr (E == 16) {  // four planes of float4
-        const float4 *h4 = reinterpret_cast<const float4 *>(a.hb) + t;
+    for (int b = 0; b < E; b += RL) dif<RL>(v, b, Roots{});
+    if constexpr (W >= 16) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float4 h = FEW ? hearly[q] : __ldg(h4 + q * TPF);
+        for (int q = 0; q < E / 4; q++) {
+            const float4 h = EARLY ? hearly[q] : response(q);
             v[4 * q] = make_float2(__fmul_rn(v[4 * q].x, h.x), __fmul_rn(v[4 * q].y, h.x));
             v[4 * q + 1] = make_float2(__fmul_rn(v[4 * q + 1].x, h.y), __fmul_rn(v[4 * q + 1].y, h.y));
             v[4 * q + 2] = make_float2(__fmul_rn(v[4 * q + 2].x, h.z), __fmul_rn(v[4 * q + 2].y, h.z));
@@ -290,31 +301,29 @@ __global__ void __launch_bounds__(Fft<LOG2W>::TPF * G, FEW ? 1 : Fft<LOG2W>::blo
     } else if constexpr (W > 1) {  // (a single sample is passed through)
 #pragma unroll
         for (int k = 0; k < E; k++) {
-            const float h = __ldg(a.hb + k);
+            const float h = __ldg(a.hb + t * E + k);
             v[k] = make_float2(__fmul_rn(v[k].x, h), __fmul_rn(v[k].y, h));
         }
     }
-    if constexpr (TPF > 1) {
 #pragma unroll
-        for (int b = 0; b < E; b += RL) dit<RL>(v, b, Roots{});
+    for (int b = 0; b < E; b += RL) dit<RL>(v, b, Roots{});
+    if constexpr (PASSES > 0) {
 #pragma unroll
         for (int k = 0; k < E; k++) inner[k] = v[k];
         meet();
-        if constexpr (F::MID) {
+    }
 #pragma unroll
-            for (int k = 0; k < E; k++) v[k] = middle[slot(k * RL)];
-            load_twiddles(a.twp + W, RL, t % RL);
-            dit<E>(v, 0, loaded);
+    for (int p = PASSES - 1; p >= 0; p--) {
+        const int n = F::stride(p);
 #pragma unroll
-            for (int k = 0; k < E; k++) middle[slot(k * RL)] = v[k];
+        for (int k = 0; k < E; k++) v[k] = at[p][slot(k * n)];
+        load_twiddles(p);
+        dit<E>(v, 0, loaded);
+        if (p) {
+#pragma unroll
+            for (int k = 0; k < E; k++) at[p][slot(k * n)] = v[k];
             meet();
         }
-#pragma unroll
-        for (int k = 0; k < E; k++) v[k] = outer[slot(k * TPF)];
-        load_twiddles(a.twp, TPF, t);
-        dit<E>(v, 0, loaded);
-    } else {
-        dit<E>(v, 0, Roots{});
     }
 
     bool over = false;
@@ -479,38 +488,59 @@ void FilterTables::release() {
     hb = nullptr;
 }
 
-template <int LOG2W, int G, bool GATHER, bool FEW = false>
+template <int LOG2W, int LOG2E, int G, Twiddles TW>
 static int launch_group(const FilterArgs &a, int n_views, cudaStream_t st) {
-    using F = Fft<LOG2W>;
+    using F = Fft<LOG2W, LOG2E>;
+    const auto kernel = filter_kernel<LOG2W, LOG2E, G, TW>;
     const int smem = (int)sizeof(float2) * std::max(F::TPF > 1 ? F::PITCH * G : 0, a.layout != FDK_LAYOUT_ROWS ? a.nu * G : 0);
     // per device and size, and needed at 48 KB too (the kernel also has static shared memory):
     // cheap, so set on every launch
-    if (smem > 40 * 1024)
-        FDK_CUDA(cudaFuncSetAttribute(filter_kernel<LOG2W, G, GATHER, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    filter_kernel<LOG2W, G, GATHER, FEW><<<dim3((unsigned)ceil_div(a.n_pairs, G), n_views), F::TPF * G, smem, st>>>(a);
+    if (smem > 40 * 1024) FDK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kernel<<<dim3((unsigned)ceil_div(a.n_pairs, G), n_views), F::TPF * G, smem, st>>>(a);
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
 }
 
-// Transforms per CTA.  The column layouts write runs of G elements, so they take the largest CTA that
-// still fills the SM's 1024 resident threads evenly: 1024 threads at W = 4096 (G = 4, 32-byte runs of
-// FP32 pairs: 971 against 1139 us at 512 threads and G = 2, 32 views of 2048^2 to MIRROR FP32; these and the
-// next figures with radix-16 butterflies, 2% to 4% below the present ones), 512
-// below, where G is 4 or more anyway (1500 x 1000 to MIRROR FP16 at 512 / 256 threads: 226 / 236 us).
-// ROWS stores are coalesced at any G, and smaller CTAs overlap each other's loads and transforms
-// better (48 views of 1536 x 1024 at 512 / 256 threads: 285 / 260 us).  A call whose CTAs would
-// not give every SM two takes the smallest group of whole warps, for more CTAs, and FEW from 128 points on
-// (below, a thread holds too few points for its planes).
+// Transforms per CTA and points per thread.
+//
+// Calls that fill the chip hold 16 points a thread.  The column layouts write runs of G elements, so they take the
+// largest CTA that still fills the SM's 1024 resident threads evenly: 1024 threads at W = 4096 (G = 4, 32-byte
+// runs of FP32 pairs: 971 against 1139 us at 512 threads and G = 2, 32 views of 2048^2 to MIRROR FP32; these and
+// the next figures with radix-16 butterflies, 2% to 4% below the present ones), 512 below, where G is 4 or more
+// anyway (1500 x 1000 to MIRROR FP16 at 512 / 256 threads: 226 / 236 us).  ROWS stores are coalesced at any G, and
+// smaller CTAs overlap each other's loads and transforms better (48 views of 1536 x 1024 at 512 / 256 threads:
+// 285 / 260 us).
+//
+// A call of few transforms is one chain of latencies, the longer the more points a thread carries through it: up
+// to 2^17 points (pairs x W) 4 a thread are the fastest, to 2^19 8 a thread, all they read asked for at the
+// start.  Microseconds of a call (B200, back to back) with 4 / 8 / 16 points a thread, ROWS FP32:
+//   rows of 200 (W 256):     33 rows x 2 views 2.4 / 3.4 / 5.1, 1200 rows 3.5 / 4.1 / 5.8, 2400 x 2 7.9 / 6.0 / 6.9
+//   rows of 511 (W 512):     256 rows 2.8 / 3.5 / 6.7, 1200 rows 5.5 / 4.8 / 7.2, 2400 x 2 14.4 / 11.4 / 11.1
+//   rows of 1000 (W 1024):   256 rows 4.0 / 4.2 / 7.4, 616 rows 7.4 / 6.3 / 7.6, 1200 rows 11.3 / 9.8 / 8.3
+//   rows of 2047 (W 2048):   16 rows 6.0 / 5.3 / 7.1, 616 rows 16.1 / 11.8 / 8.8
+//   rows of 2048 (W 4096):   16 rows 11.7 / 8.1 / 7.0, 616 rows 33.2 / 22.2 / 12.1
+// (W 4096: a CTA of 512 threads or more to a pair is slower than the longer chain.)  From there to 2^21 points small
+// CTAs of 16 points a thread fill the SMs more evenly (1200 rows of 1000: 8.3 against 10.1 us), but for the columns of
+// longer rows, whose runs would be short (TRANSPOSED 11.7 against 14.6).
 static int launch_filter(const FilterArgs &a, int log2W, int n_views, cudaStream_t st) {
     return with_length(log2W, [&](auto l) {
-        constexpr int L = decltype(l)::value, TPF = Fft<L>::TPF;
+        constexpr int L = decltype(l)::value, W = 1 << L;
+        constexpr int TPF = Fft<L, 4>::TPF, TPF4 = Fft<L, 2>::TPF, TPF8 = Fft<L, 3>::TPF;
         constexpr int cols = std::min((L == 12 ? 1024 : 512) / TPF, 64), rows = std::min(256 / TPF, 64);
-        constexpr int least = std::max(1, std::min(64 / TPF, 16));
-        const int g = a.layout == FDK_LAYOUT_ROWS ? rows : cols;
-        if (!a.twp) return launch_group<L, least, true>(a, n_views, st);
-        if (ceil_div(a.n_pairs, g) * n_views < 2 * 148) return launch_group<L, least, false, (L >= 7)>(a, n_views, st);
-        if (g == rows) return launch_group<L, rows, false>(a, n_views, st);
-        return launch_group<L, cols, false>(a, n_views, st);
+        constexpr int least = std::max(1, std::min(64 / TPF, 16));  // 64 threads
+        constexpr int few4 = std::max(1, std::min(64 / TPF4, 16)), few8 = std::max(1, std::min(128 / TPF8, 16));
+        const long long points = (long long)a.n_pairs * n_views * W;
+        if constexpr (L <= 10)
+            if (points <= 1 << 17) return launch_group<L, 2, few4, Twiddles::Early>(a, n_views, st);
+        if constexpr (L <= 11)
+            if (points <= (L <= 8 ? 3 << 18 : 1 << 19)) return launch_group<L, 3, few8, Twiddles::Early>(a, n_views, st);
+        if (!a.twp) return launch_group<L, 4, least, Twiddles::Roots>(a, n_views, st);
+        if constexpr (L == 12)
+            if (points <= 1 << 19) return launch_group<L, 4, least, Twiddles::Early>(a, n_views, st);
+        const bool by_rows = a.layout == FDK_LAYOUT_ROWS;
+        if (points <= 1 << 21 && (by_rows || L <= 8)) return launch_group<L, 4, least, Twiddles::Planes>(a, n_views, st);
+        if (by_rows) return launch_group<L, 4, rows, Twiddles::Planes>(a, n_views, st);
+        return launch_group<L, 4, cols, Twiddles::Planes>(a, n_views, st);
     });
 }
 
@@ -519,6 +549,7 @@ int filter_views(const float *src, int src_pitch, long long src_vstride, void *d
                  long long dst_vstride, const float *cos, int cos_pitch, const FilterTables &t, int nu,
                  int nv, int pad_n, int n_views, int layout, int dtype, cudaStream_t st, float out_scale,
                  unsigned int *overflow) {
+    FDK_CHECK_ARG(t.hb && t.tw, "filter tables are missing");
     FDK_CHECK_ARG(((uintptr_t)t.hb & 15) == 0 && ((uintptr_t)t.twp & 15) == 0, "filter tables must start on 16-byte boundaries");
     FilterArgs a;
     a.src = src;
@@ -717,12 +748,14 @@ int fdk_filter_row_real32(const fdk_dataref *src, fdk_dataref *dst, const fdk_da
     FilterTables t;
     t.W = W;
     while ((1 << t.log2W) < W) t.log2W++;
-    // The response first: W floats are whole 16-byte words (W >= 4), which the kernel reads both tables by.
+    // The response first: W floats are whole 16-byte words (W >= 4), which the kernel reads it and the
+    // passes' planes by.
     const size_t planes = (size_t)W + W / 16;
     Scratch tables;
-    FDK_TRY(tables.alloc(sizeof(float) * W + sizeof(float2) * planes, cudaStreamLegacy));
+    FDK_TRY(tables.alloc(sizeof(float) * W + sizeof(float2) * (planes + W / 2), cudaStreamLegacy));
     t.hb = static_cast<float *>(tables.p);
     t.twp = reinterpret_cast<float2 *>(t.hb + W);
+    t.tw = t.twp + planes;
     FDK_TRY(filter_tables_on_device(filter->data, t, cudaStreamLegacy));
     FDK_TRY(filter_views(src->data, src->pitch, (long long)src->pitch * src->height, dst->data, dst->pitch,
                          (long long)dst->pitch * dst->height, nullptr, 0, t, src->width, src->height, 3, src->depth,

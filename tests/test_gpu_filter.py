@@ -161,3 +161,27 @@ def test_row_entry_points_over_every_length(log2w, nv, views):
         ref = [C.byref(DataRef(t.data_ptr(), t.shape[-1], nv, views, t.shape[-1])) for t in (src, again)]
         check(lib().fdk_filter_row_real32_noalloc(*ref, C.byref(DataRef(filt.data_ptr(), W, 1, 1, W))))
         assert max_rel(again.cpu().numpy(), want) <= 3e-6
+
+
+@pytest.mark.parametrize("nu", [24, 100, 200, 511, 1000, 2047, 4000])
+def test_points_per_thread_agree(nu):
+    """Calls of growing size hold 4, 8 and 16 points a thread, in small and large CTAs: at every length and
+    layout the first view comes out alike.  The butterflies are the same; only where a stage's roots are exact
+    (1 and -i) may one variant add 6e-17 of a sample that another one leaves out, so 1e-7 of the largest output
+    is less than two of its last bits."""
+    import torch
+
+    nv = 37
+    rng = np.random.default_rng(nu)
+    cos = rng.uniform(0.9, 1.0, (nv, nu)).astype(np.float32)
+    eng = F.FilterEngine(cos, O.filter_design("hann", nu).astype(np.float32))
+    pairs = (nv + 1) // 2 * eng.W
+    counts = sorted({max(1, n // pairs) for n in (1, 1 << 17, (1 << 17) + pairs, 1 << 19, 3 << 18, (3 << 18) + pairs, 1 << 21, 3 << 20)})
+    src = torch.from_numpy((rng.standard_normal((1, nv, nu)) + 2.0).astype(np.float32)).cuda().repeat(counts[-1], 1, 1)
+    for layout in (F.LAYOUT_ROWS, F.LAYOUT_TRANSPOSED, F.LAYOUT_MIRROR):
+        first = None
+        for n in counts:
+            out = torch.full((n, nv * nu * (2 if layout == F.LAYOUT_MIRROR else 1)), 7.0, device="cuda")
+            eng.run_device(src.data_ptr(), out.data_ptr(), n, layout, F.DTYPE_F32)
+            first = out[:1] if first is None else first
+            assert float((out - first).abs().max()) <= 1e-7 * float(first.abs().max()), (layout, n)
