@@ -46,7 +46,7 @@ EXPORTED = [
     "fdk_recon_push_folder", "fdk_recon_flush", "fdk_recon_filter_kind", "fdk_recon_bp_kernel", "fdk_recon_sync",
     "fdk_recon_get_volume", "fdk_recon_sample", "fdk_recon_stats", "fdk_recon_launch_count", "fdk_recon_reset", "fdk_recon_destroy",
     "fdk_phantom_project", "fdk_forward_project", "fdk_probe_smem", "fdk_probe_fma",
-    "fdk_nn_param_count", "fdk_nn_forward", "fdk_nn_backward", "fdk_adam_step", "fdk_transmission_noise",
+    "fdk_nn_param_count", "fdk_nn_forward", "fdk_nn_backward", "fdk_nn_check", "fdk_adam_step", "fdk_transmission_noise",
     "fdk_voxelize", "fdk_rows_to_mirror", "fdk_volume_mse", "fdk_bp_adjoint",
     "fdk_proj_path", "fdk_load_proj_folder", "fdk_save_proj_folder", "fdk_save_volume", "fdk_load_volume",
     "fdk_save_volume_slices",
@@ -156,6 +156,7 @@ def lib() -> C.CDLL:
         "fdk_forward_project": ([G, vp, i64, i64, vp, vp], C.c_int),
         "fdk_nn_param_count": ([], C.c_int),
         "fdk_nn_forward": ([vp, vp, vp, i64, i32, C.c_float, vp], C.c_int),
+        "fdk_nn_check": ([vp], C.c_int),
         "fdk_nn_backward": ([vp, vp, vp, vp, i64, i32, C.c_float, vp], C.c_int),
         "fdk_adam_step": ([vp, vp, vp, vp, i64, C.c_float, C.c_float, C.c_float, C.c_float, i64, vp], C.c_int),
         "fdk_transmission_noise": ([vp, i64, C.c_double, C.c_double, C.c_uint64, vp], C.c_int),

@@ -727,20 +727,6 @@ inline int tma_prepare(int &ctas, int device) {
     return FDK_OK;
 }
 
-// Limit of the kernel's mbarrier waits: FDK_BP_WAIT_NS nanoseconds, default 10 s.
-inline unsigned long long bp_wait_ns() {
-    const char *e = getenv("FDK_BP_WAIT_NS");
-    const long long v = e ? atoll(e) : 0;
-    return v > 0 ? (unsigned long long)v : kWaitNs;
-}
-// Test switch FDK_BP_TEST_WITHHOLD=1: CTA 0's producer never fills the first pipeline stage,
-// so its consumers' bounded wait runs out and the launch reports FDK_ERR_DEVICE_CHECK (the
-// timeout path, exercised without a GPU fault).  Off unless the environment sets it.
-inline int bp_test_withhold() {
-    const char *e = getenv("FDK_BP_TEST_WITHHOLD");
-    return (e && atoi(e) == 1) ? 1 : 0;
-}
-
 // Square of the source distance of the volume centre in view 0, rounded to a power of four
 // (within a factor of two of it): keeps f^2 * wscale near 1, and its square root is a power of
 // two, so scaling by it is exact (fold_lerp_meta folds wscale^-1/2 into the matrix rows).

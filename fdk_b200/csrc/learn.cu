@@ -433,6 +433,12 @@ __global__ void __launch_bounds__(256, 3) bp_adjoint_kernel(AdjArgs a) {
 
 using namespace fdk;
 
+// The status of the network kernels' error word.
+static int network_status(unsigned word) {
+    if (word) return fail(FDK_ERR_DEVICE_CHECK, "a network kernel's pipeline wait timed out on the device (error word %u)", word);
+    return FDK_OK;
+}
+
 extern "C" {
 
 int fdk_nn_param_count(void) { return kNParam; }
@@ -447,7 +453,8 @@ int fdk_nn_forward(const float *params, const float *x, float *y, int64_t rows, 
     FDK_CUDA(cudaGetDevice(&dev));
     FDK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int blocks = (int)std::min<long long>(ceil_div(rows, nn::rows_per_step(len)), 2 * sms);  // two resident CTAs per SM
-    nn::forward_kernel<<<blocks, nn::THREADS, nn::Fwd::BYTES, (cudaStream_t)stream>>>(params, x, y, len, rows, scale);
+    nn::forward_kernel<<<blocks, nn::THREADS, nn::Fwd::BYTES, (cudaStream_t)stream>>>(params, x, y, len, rows, scale,
+                                                                                   bp_wait_ns(), bp_test_withhold());
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
     FDK_ABI_END
@@ -465,10 +472,23 @@ int fdk_nn_backward(const float *params, const float *x, const float *dy, float 
     FDK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int blocks = (int)std::min<long long>(ceil_div(rows, nn::rows_per_step(len)), sms);
     FDK_CUDA(cudaMemsetAsync(dparams, 0, sizeof(float) * kNParam, (cudaStream_t)stream));
-    nn::backward_kernel<<<blocks, nn::Bwd::THREADS, nn::Bwd::BYTES, (cudaStream_t)stream>>>(params, x, dy, dparams, len, rows,
-                                                                                          scale);
+    nn::backward_kernel<<<blocks, nn::Bwd::THREADS, nn::Bwd::BYTES, (cudaStream_t)stream>>>(
+        params, x, dy, dparams, len, rows, scale, bp_wait_ns(), bp_test_withhold());
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
+    FDK_ABI_END
+}
+
+int fdk_nn_check(void *stream) {
+    FDK_ABI_BEGIN
+    clear_error();
+    unsigned *word = nullptr, got = 0;
+    FDK_CUDA(cudaGetSymbolAddress((void **)&word, nn::g_nn_err));
+    cudaStream_t st = (cudaStream_t)stream;
+    FDK_CUDA(cudaMemcpyAsync(&got, word, sizeof(got), cudaMemcpyDeviceToHost, st));
+    FDK_CUDA(cudaStreamSynchronize(st));
+    if (got) FDK_CUDA(cudaMemsetAsync(word, 0, sizeof(got), st));
+    return network_status(got);
     FDK_ABI_END
 }
 
@@ -554,10 +574,7 @@ int fdk_volume_mse(const float *dev_vol_xyz, const float *dev_truth, float *dev_
     FDK_CUDA(cudaMemcpyAsync(got, d_sse, sizeof(got), cudaMemcpyDeviceToHost, st));
     FDK_CUDA(cudaStreamSynchronize(st));
     *sse_host = got[0];
-    if (got[1] != 0)
-        return fail(FDK_ERR_DEVICE_CHECK, "a network kernel's pipeline wait timed out on the device (error word %u)",
-                    (unsigned)got[1]);
-    return FDK_OK;
+    return network_status((unsigned)got[1]);
     FDK_ABI_END
 }
 

@@ -111,16 +111,19 @@ __device__ __forceinline__ unsigned pack2(float a, float b) {
 }
 
 // A wait of the CTA ran out: records it and waits, bounded, for the operations the CTA still has in flight
-// (fin: a barrier used for nothing else) before the caller gives its TMEM back.
+// (fin: a barrier of 32 arrivals used for nothing else) before the caller gives its TMEM back.  A commit covers its
+// own thread's operations and any lane of warp 0 may have issued, so that all of them commit.
 __device__ __noinline__ void give_up(unsigned fin, unsigned *err) {
-    if (threadIdx.x == 0) {
-        atomicOr(err, kErrTimeout);
+    if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) atomicOr(err, kErrTimeout);
         tc_commit(fin);
         mbar_wait(fin, 0);
     }
 }
+// What a CTA that gave up leaves in the outputs it owes.
+__device__ __forceinline__ float lost() { return __int_as_float(0x7FFFFFFF); }
 
-// Device-side failures of the network kernels (a bounded wait that ran out), read by fdk_volume_mse.
+// Device-side failures of the network kernels (a bounded wait that ran out), read by fdk_nn_check and fdk_volume_mse.
 static __device__ unsigned int g_nn_err;
 
 // The small layers' weights, in the order the position threads read them.
@@ -299,6 +302,14 @@ struct Fwd {
 };
 static_assert(Fwd::XS % 16 == 0 && Fwd::PART % 16 == 0 && Fwd::BARS % 8 == 0, "alignment");
 
+// The CTA gave up at step st: its rows from there on.
+__device__ __noinline__ void lose_rows(float *y, int L, long long rows, long long st) {
+    const int per = rows_per_step(L);
+    const Place me = place(threadIdx.x, L, per);
+    for (; st * per < rows; st += gridDim.x)
+        if (me.in && st * per + me.row < rows) y[(st * per + me.row) * L + me.p] = lost();
+}
+
 // y = x + net(x).  23,040 rows of 256: 545 us; FP32 FMAs, register-blocked, took 2283 (69% of the FP32 rate).
 // The tensor core is busy for about 2100 clocks of a step's 11,000 (two CTAs share an SM); the rest is
 // layers 1 and 3 on the FP32 pipe and the barriers between the phases.  A CTA of 256 threads takes the rows of one step (256 positions) at a time: layer 1 in
@@ -306,7 +317,8 @@ static_assert(Fwd::XS % 16 == 0 && Fwd::PART % 16 == 0 && Fwd::BARS % 8 == 0, "a
 // x 288), layer 3 in FP32 by position, its 9 taps' partial sums exchanged through shared memory.
 // Two CTAs per SM run their phases against each other.
 __global__ void __launch_bounds__(THREADS, 2) forward_kernel(const float *__restrict__ params, const float *__restrict__ x,
-                                                           float *__restrict__ y, int L, long long rows, float s) {
+                                                           float *__restrict__ y, int L, long long rows, float s,
+                                                           unsigned long long wait_ns, int withhold) {
     extern __shared__ __align__(128) unsigned char smem[];
     Small &w = *reinterpret_cast<Small *>(smem + Fwd::SMALL);
     float *xs = reinterpret_cast<float *>(smem + Fwd::XS);      // s x, position p at p + 4
@@ -320,7 +332,7 @@ __global__ void __launch_bounds__(THREADS, 2) forward_kernel(const float *__rest
     for (int i = t; i < kK * PITCH; i += THREADS) part[i] = 0.f;
     if (t == 0) {
         mbar_init(bar, 1);
-        mbar_init(bar + 8, 1);
+        mbar_init(bar + 8, 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (t < 32) tc_alloc(smem_u32(tmem_word), Fwd::COLUMNS);
@@ -331,6 +343,7 @@ __global__ void __launch_bounds__(THREADS, 2) forward_kernel(const float *__rest
     const int per = rows_per_step(L), tiles = per * (L + kHalo) - kHalo > 128 ? 2 : 1;
     const long long steps = (rows + per - 1) / per;
     const Place me = place(t, L, per), l0 = place(t & 127, L, per), l1 = place((t & 127) + 128, L, per);
+    const unsigned stall = withhold && blockIdx.x == 0 ? 1 : 0;
     unsigned phase = 0;
     for (long long st = blockIdx.x; st < steps; st += gridDim.x, phase ^= 1) {
         const long long r0 = st * per;
@@ -347,12 +360,13 @@ __global__ void __launch_bounds__(THREADS, 2) forward_kernel(const float *__rest
             tc_after();
             const unsigned leader = tc_leader();
             issue_layer2(d, base + Fwd::A1, base + Fwd::WF, tiles, 128, leader);
-            if (leader) tc_commit(bar);
+            if (leader > stall) tc_commit(bar);
             __syncwarp();
         }
-        const bool ok = mbar_wait(bar, phase);
+        const bool ok = mbar_wait(bar, phase, wait_ns);
         if (__syncthreads_or(!ok)) {
             give_up(bar + 8, &g_nn_err);
+            lose_rows(y, L, rows, st);
             break;
         }
         tc_after();
@@ -457,7 +471,8 @@ __device__ __forceinline__ void issue_sum(unsigned d, unsigned a, unsigned b, in
 
 __global__ void __launch_bounds__(Bwd::THREADS, 1) backward_kernel(const float *__restrict__ params,
                                                                  const float *__restrict__ x, const float *__restrict__ dy,
-                                                                 float *__restrict__ dparams, int L, long long rows, float s) {
+                                                                 float *__restrict__ dparams, int L, long long rows, float s,
+                                                                 unsigned long long wait_ns, int withhold) {
     extern __shared__ __align__(128) unsigned char smem[];
     Small &w = *reinterpret_cast<Small *>(smem + Bwd::SMALL);
     float *xs = reinterpret_cast<float *>(smem + Bwd::XS);  // s x, position p at p + 4
@@ -474,7 +489,7 @@ __global__ void __launch_bounds__(Bwd::THREADS, 1) backward_kernel(const float *
         mbar_init(bar_l2, 1);
         mbar_init(bar_dz1, 1);
         mbar_init(bar_all, 1);
-        mbar_init(fin, 1);
+        mbar_init(fin, 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (t < 32) tc_alloc(smem_u32(tmem_word), Bwd::COLUMNS);
@@ -527,7 +542,7 @@ __global__ void __launch_bounds__(Bwd::THREADS, 1) backward_kernel(const float *
             tc_after();
             const unsigned leader = tc_leader();
             issue_layer2(d + Bwd::LAYER2, base + Bwd::A1, base + Bwd::WF, tiles, 96, leader);
-            if (leader) tc_commit(bar_l2);
+            if (leader && !(withhold && blockIdx.x == 0)) tc_commit(bar_l2);
             __syncwarp();
         }
         // while layer 2 runs: the column operands (tap 8 - k of d3's window is d3[p - k + 4])
@@ -539,7 +554,7 @@ __global__ void __launch_bounds__(Bwd::THREADS, 1) backward_kernel(const float *
 #pragma unroll
         for (int k = 0; k < kK; k++) win[k] = d3[m + 8 - k];
         if (!h) store_columns(smem + Bwd::T3 + (m + ROW0) * 16, win);
-        ok = mbar_wait(bar_l2, phase);
+        ok = mbar_wait(bar_l2, phase, wait_ns);
         tc_after();
         // a2 and dz2[c][p] = [a2 > 0] sum_k W3[c][k] d3[p - k + 4], 8 channels at a time
         if ((r & 1) < tiles) {
@@ -604,7 +619,7 @@ __global__ void __launch_bounds__(Bwd::THREADS, 1) backward_kernel(const float *
             for (int k = 0; k < kK; k++)
                 issue_sum(d + Bwd::DW2 + 32 * k, base + Bwd::DZ2 + ROW0 * 16, base + Bwd::A1 + (ROW0 - kHalo + k) * 16, ksteps, leader);
         } else {
-            ok = mbar_wait(bar_dz1, phase);
+            ok = mbar_wait(bar_dz1, phase, wait_ns);
             tc_after();
         }
         // dz1[ci][p] = [a1 > 0] of the sums; channel 8 g + i, part j of W2 in column 8 (3 g + j) + i.  The issuing
@@ -643,7 +658,7 @@ __global__ void __launch_bounds__(Bwd::THREADS, 1) backward_kernel(const float *
             if (leader) tc_commit(bar_all);
             __syncwarp();
         }
-        ok = mbar_wait(bar_all, phase);
+        ok = mbar_wait(bar_all, phase, wait_ns);
         tc_after();
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -671,11 +686,16 @@ __global__ void __launch_bounds__(Bwd::THREADS, 1) backward_kernel(const float *
         }
         tc_before();
     }
-    if (__syncthreads_or(!ok)) give_up(fin, &g_nn_err);
+    const bool gave_up = __syncthreads_or(!ok);
+    if (gave_up) give_up(fin, &g_nn_err);
     tc_before();
     __syncthreads();
     tc_after();
     if (t < 32) tc_dealloc(d, Bwd::COLUMNS);
+    if (gave_up) {
+        for (int i = t; i < kNParam; i += Bwd::THREADS) atomicAdd(dparams + i, lost());
+        return;
+    }
 
     // dW2: the three parts' rows through shared memory (one float of padding per row), then one add per
     // parameter

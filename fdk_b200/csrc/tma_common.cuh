@@ -161,4 +161,18 @@ inline EncodeTiledFn tensor_map_encoder() {
     return fn;
 }
 
+// Limit of the kernels' mbarrier waits: FDK_BP_WAIT_NS nanoseconds, default 10 s.
+inline unsigned long long bp_wait_ns() {
+    const char *e = getenv("FDK_BP_WAIT_NS");
+    const long long v = e ? atoll(e) : 0;
+    return v > 0 ? (unsigned long long)v : kWaitNs;
+}
+// Test switch FDK_BP_TEST_WITHHOLD=1: CTA 0's producer never fills the first pipeline stage (the network
+// kernels: never commits its products), so its consumers' bounded wait runs out and the launch reports
+// FDK_ERR_DEVICE_CHECK (the timeout path, exercised without a GPU fault).  Off unless the environment sets it.
+inline int bp_test_withhold() {
+    const char *e = getenv("FDK_BP_TEST_WITHHOLD");
+    return (e && atoi(e) == 1) ? 1 : 0;
+}
+
 }  // namespace fdk

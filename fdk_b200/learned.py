@@ -121,6 +121,8 @@ class Pipeline:
 
     # ------------------------------------------------------------------ forward / loss / backward
     def reconstruct(self, params_d, x_rows) -> None:
+        """Asynchronous.  A network kernel that gives up leaves rows, and so voxels, that are not numbers; mse() and
+        check() raise."""
         p = self.p
         if params_d is None:
             src = x_rows
@@ -161,6 +163,10 @@ class Pipeline:
         check(lib().fdk_volume_mse(vol, self.truth.data_ptr(), self.res.data_ptr() if with_grad else None, p.nx, p.ny,
                                    p.nz, C.byref(sse), None))
         return sse.value / (p.nx * p.ny * p.nz)
+
+    def check(self) -> None:
+        """Waits for the calls so far; raises if a network kernel gave up (fdk_nn_check)."""
+        check(lib().fdk_nn_check(None))
 
     def gradient(self, params_d, x_rows, fov_only: bool = False) -> None:
         """After reconstruct() + mse(with_grad=True): parameter gradient into self.dparams.
@@ -219,6 +225,7 @@ def train(n_train: int = 2000, epochs: int = 20, lr: float = 1e-3, seed0: int = 
             if batch > 1:
                 torch.mul(gsum, 1.0 / batch, out=pl.dparams)
                 gsum.zero_()
+            pl.check()  # before the weights take the gradient
             lr_t = lr if schedule == "constant" else lr * (0.01 + 0.99 * 0.5 * (1 + math.cos(math.pi * step / total)))
             check(lib().fdk_adam_step(w.data_ptr(), pl.dparams.data_ptr(), m.data_ptr(), v.data_ptr(), w.numel(),
                                       lr_t, 0.9, 0.999, 1e-8, step, None))

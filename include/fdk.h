@@ -371,6 +371,10 @@ int fdk_nn_forward(const float *params, const float *x, float *y, int64_t rows, 
 /* Parameter gradient dparams (overwritten) of sum(dy . y) over all rows; recomputes activations. */
 int fdk_nn_backward(const float *params, const float *x, const float *dy, float *dparams, int64_t rows,
                     int32_t len, float scale, void *stream);
+/* Waits for the stream; FDK_ERR_DEVICE_CHECK, once, if a bounded pipeline wait (FDK_BP_WAIT_NS, default 10 s) of
+ * fdk_nn_forward or fdk_nn_backward ran out on the current device since the last report.  The rows of y, or
+ * the gradient, that such a call still owed are not-a-number. */
+int fdk_nn_check(void *stream);
 /* One Adam step (bias-corrected, step t >= 1) on n parameters. */
 int fdk_adam_step(float *params, const float *grads, float *m, float *v, int64_t n, float lr, float beta1,
                   float beta2, float eps, int64_t t, void *stream);
@@ -381,8 +385,7 @@ int fdk_voxelize(const fdk_geometry *g, const double *ell, int32_t n_ell, float 
 /* ROWS views (n x nv x nu) -> MIRROR f32 pairs (n x nu x nv x 2), the staged backprojection's input. */
 int fdk_rows_to_mirror(const float *dev_rows, void *dev_mirror, int64_t n_views, int32_t nu, int32_t nv,
                        void *stream);
-/* (fdk_volume_mse, synchronous, also reports FDK_ERR_DEVICE_CHECK once if a bounded pipeline wait of
- * fdk_nn_forward or fdk_nn_backward ran out on the device since its last call.) */
+/* (fdk_volume_mse, synchronous, also reports what fdk_nn_check does.) */
 /* Sum of squared errors of a backprojection volume ([x][y][z], as fdk_bp_volume_device of a full slab
  * pair) against truth ([z][y][x]) into *sse_host; dev_res (may be NULL) = 2 (vol - truth) / N, [z][y][x]. */
 int fdk_volume_mse(const float *dev_vol_xyz, const float *dev_truth, float *dev_res, int32_t nx, int32_t ny,

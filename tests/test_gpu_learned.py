@@ -346,3 +346,37 @@ def test_voxelizer_vs_fp64(nx, ny, nz, n_ell):
         close |= np.abs(q - 1) < 1e-12
     got = out.cpu().numpy()
     assert (np.abs(got - want) <= 1e-6)[~close].all() and np.isfinite(got).all()
+
+
+@pytest.mark.parametrize("rows", [3, 700])  # one step a CTA, and several for the one that stalls
+def test_network_wait_that_runs_out_is_reported_at_once(rows, monkeypatch):
+    """FDK_BP_TEST_WITHHOLD makes CTA 0 withhold its products' commit; with a 1 ms limit it gives up.  fdk_nn_check
+    reports it once, what the CTA owed is not a number, and the next calls give what they gave before."""
+    import torch
+
+    L = 200
+    rng = np.random.default_rng(rows)
+    dp = torch.from_numpy((rng.standard_normal(N.NPARAM) * 0.1).astype(np.float32)).cuda()
+    x, dy = (torch.from_numpy(rng.standard_normal((rows, L)).astype(np.float32)).cuda() for _ in range(2))
+
+    def run():
+        y, g = torch.full_like(x, 7.0), torch.full_like(dp, 7.0)
+        check(lib().fdk_nn_forward(dp.data_ptr(), x.data_ptr(), y.data_ptr(), rows, L, 0.25, None))
+        rc = [lib().fdk_nn_check(None)]
+        check(lib().fdk_nn_backward(dp.data_ptr(), x.data_ptr(), dy.data_ptr(), g.data_ptr(), rows, L, 0.25, None))
+        return y.cpu().numpy(), g.cpu().numpy(), rc + [lib().fdk_nn_check(None), lib().fdk_nn_check(None)]
+
+    want, grad, rc = run()
+    assert rc == [0, 0, 0] and np.isfinite(want).all() and np.isfinite(grad).all()
+    monkeypatch.setenv("FDK_BP_WAIT_NS", "1000000")
+    monkeypatch.setenv("FDK_BP_TEST_WITHHOLD", "1")
+    y, g, rc = run()
+    assert rc == [-7, -7, 0]  # FDK_ERR_DEVICE_CHECK, once each
+    gone = np.isnan(y).all(1)
+    assert gone[0] and not gone.all() and (rows == 3) == (gone.sum() == 1)
+    assert np.array_equal(y[~gone], want[~gone]) and np.isnan(g).all()
+    monkeypatch.delenv("FDK_BP_WAIT_NS")
+    monkeypatch.delenv("FDK_BP_TEST_WITHHOLD")
+    y, g, rc = run()
+    assert rc == [0, 0, 0] and np.array_equal(y, want)
+    assert np.abs(g - grad).max() <= 1e-5 * np.abs(grad).max()  # the order of the CTAs' FP32 additions
