@@ -268,6 +268,7 @@ struct fdk_bp {
     // [band_z[k], band_z[k+1]) with their mirrors), each recording band_done[k]; a readback
     // copies band k to the host while the later bands of the last batch still run.
     int n_bands = 1;
+    bool whole_batches = false;  // batches that no readback follows run as one launch (plan_bands)
     long long band_z[kMaxBands + 1] = {};
     int band_tz[kMaxBands + 1] = {};          // the same bounds in z tiles of the staged kernel
     cudaEvent_t band_done[kMaxBands] = {};
@@ -611,7 +612,7 @@ void set_bands(fdk_bp *h, int unit) {
 void plan_bands(fdk_bp *h, int unit, long long views, bool quarter) {
     const bool mixed = h->precision == FDK_BP_MIXED;
     const int R = quarter ? (mixed ? SymCfg<HalfLerp>::R : SymCfg<float2>::R) : staged_rows(h);
-    const long long w = (long long)h->top.width, d = (long long)h->top.height;
+    const long long w = (long long)h->top.width, d = (long long)h->top.height, d_z = (long long)h->top.depth;
     const long long cols = quarter ? ceil_div((w + 1) / 2, 16) * ceil_div((d + 1) / 2, 16) : ceil_div(w, 16) * ceil_div(d, 16);
     const int ctas = quarter ? h->sym_ctas : h->plan.tma_ctas;
     const double rate = mixed ? 2.7e12 : 1.75e12;  // voxel updates a second
@@ -629,6 +630,10 @@ void plan_bands(fdk_bp *h, int unit, long long views, bool quarter) {
         }
     }
     cut_bands(h, nb, unit);
+    // Bands of fewer than 8 tiles a CTA cost a batch (set_bands), and only the flush before a readback has
+    // something to gain by them: 200^3 MIXED from 300 views in batches of 32 took 4553 us with every batch in
+    // bands, 3476 with none in bands, 3444 so.
+    h->whole_batches = nb > 1 && cols * (ceil_div(d_z, R) / nb) < 8ll * ctas;
 }
 
 // The fast kernels need circular-orbit matrices: rows 0 and 2 without a z term.
@@ -1318,7 +1323,8 @@ int release_list(fdk_bp *h, int i, cudaStream_t st) {
 // reconstructor (recon.cu): `n_single` views by (slot, view) through the staged kernel and
 // `n_quad` quarter-turn quadruples (4 slots each, members b, b + N/4, b + N/2, b + 3N/4 mod N, and
 // the base view b; one per view of each whole orbit) through the quarter-turn kernel.  d_mats / host_mats: every view's matrix.
-// band: -1 = every z band, else one.  Internal to the library.
+// band: -1 = every z band, -2 = every band where no readback follows (one launch of each kernel where the plan
+// says so), else one.  Internal to the library.
 int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const float *d_mats, const float *host_mats,
                              const int *s_slot, const int *s_view, int n_single, const int *q_slot,
                              const int *q_view, int n_quad, void *stream, int band) {
@@ -1336,7 +1342,9 @@ int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const fl
     cudaStream_t st = (cudaStream_t)stream;
     const bool mixed = h->precision == FDK_BP_MIXED;
     const float *acc_scale = mixed ? h->ext_scale : nullptr;
-    const int kb = band < 0 ? 0 : band, ke = band < 0 ? h->n_bands : band + 1;
+    const int kb = band < 0 ? 0 : band;
+    const int step = band == -2 && h->whole_batches ? h->n_bands : 1;  // bands a launch covers
+    const int ke = band < 0 ? h->n_bands : band + 1;
     std::pair<cudaEvent_t, cudaEvent_t> tm;
     FDK_TRY(take_timer(h, tm));
     FDK_CUDA(cudaEventRecord(tm.first, st));
@@ -1349,7 +1357,7 @@ int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const fl
         FDK_CHECK_ARG(used <= n_slots, "slot outside the views buffer");
         FDK_TRY(lerp_views(h, views, used, band, st, acc_scale, &lv, &lerp_sc));
     }
-    for (int k = kb; k < ke; k++) {
+    for (int k = kb; k < ke; k += step) {
         for (int q0 = 0; q0 < n_quad; q0 += kSymMaxQuads) {
             const int nq = std::min(kSymMaxQuads, n_quad - q0);
             fdk_bp::ListRec *rec = nullptr, *dev = nullptr;
@@ -1364,10 +1372,10 @@ int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const fl
             FDK_CUDA(cudaMemcpyAsync(dev, rec, sizeof(SymQuads), cudaMemcpyHostToDevice, st));
             const int r = mixed ? bp_sym_launch<HalfLerp>(h->plan, h->sym_ctas, h->d_vol, h->d_comp, lv, n_slots,
                                                           d_mats, host_mats, sq, &dev->quads, nq, h->sym_rot, st,
-                                                          lerp_sc, h->band_z[k], h->band_z[k + 1])
+                                                          lerp_sc, h->band_z[k], h->band_z[k + step])
                                 : bp_sym_launch<float2>(h->plan, h->sym_ctas, h->d_vol, h->d_comp, views, n_slots,
                                                         d_mats, host_mats, sq, &dev->quads, nq, h->sym_rot, st,
-                                                        acc_scale, h->band_z[k], h->band_z[k + 1]);
+                                                        acc_scale, h->band_z[k], h->band_z[k + step]);
             FDK_TRY(release_list(h, e, st));
             FDK_TRY(r);
             h->launches++;
@@ -1387,11 +1395,11 @@ int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const fl
                 FDK_TRY(lv && h->lerp_compact
                             ? bp_tma_launch<HalfLerpCompact>(h->plan, h->d_vol, h->d_comp, pv, d_mats + m0,
                                                              host_mats + m0, ns, st, lerp_sc, h->band_tz[k],
-                                                             h->band_tz[k + 1])
+                                                             h->band_tz[k + step])
                         : lv ? bp_tma_launch<HalfLerp>(h->plan, h->d_vol, h->d_comp, pv, d_mats + m0, host_mats + m0,
-                                                     ns, st, lerp_sc, h->band_tz[k], h->band_tz[k + 1])
+                                                     ns, st, lerp_sc, h->band_tz[k], h->band_tz[k + step])
                         : launch_staged_f32(h, pv, d_mats + m0, host_mats + m0, ns, st, acc_scale, h->band_tz[k],
-                                            h->band_tz[k + 1]));
+                                            h->band_tz[k + step]));
                 h->launches++;
                 continue;
             }
@@ -1407,18 +1415,18 @@ int fdk_bp_bp_lists_internal(fdk_bp *h, const void *views, int n_slots, const fl
             FDK_CUDA(cudaMemcpyAsync(dev, rec, sizeof(ViewList), cudaMemcpyHostToDevice, st));
             const int r = lv && h->lerp_compact
                               ? bp_tma_launch<HalfLerpCompact>(h->plan, h->d_vol, h->d_comp, lv, d_mats, host_mats, ns,
-                                                               st, lerp_sc, h->band_tz[k], h->band_tz[k + 1], &vl,
+                                                               st, lerp_sc, h->band_tz[k], h->band_tz[k + step], &vl,
                                                                &dev->views, n_slots)
                           : lv ? bp_tma_launch<HalfLerp>(h->plan, h->d_vol, h->d_comp, lv, d_mats, host_mats, ns, st,
-                                                       lerp_sc, h->band_tz[k], h->band_tz[k + 1], &vl, &dev->views,
+                                                       lerp_sc, h->band_tz[k], h->band_tz[k + step], &vl, &dev->views,
                                                        n_slots)
                           : launch_staged_f32(h, views, d_mats, host_mats, ns, st, acc_scale, h->band_tz[k],
-                                              h->band_tz[k + 1], &vl, &dev->views, n_slots);
+                                              h->band_tz[k + step], &vl, &dev->views, n_slots);
             FDK_TRY(release_list(h, e, st));
             FDK_TRY(r);
             h->launches++;
         }
-        FDK_CUDA(cudaEventRecord(h->band_done[k], st));
+        for (int j = k; j < k + step; j++) FDK_CUDA(cudaEventRecord(h->band_done[j], st));
     }
     FDK_CUDA(cudaEventRecord(tm.second, st));
     h->timers.push_back(tm);

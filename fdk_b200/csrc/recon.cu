@@ -148,8 +148,8 @@ int collect_filter_timers(fdk_recon *h) {
     return FDK_OK;
 }
 
-// Backproject the n filtered views of buffer b: every z band (band -1) or one, on the compute
-// stream.  FP32_EXACT: one consecutive run.  Staged precisions: the views whose quarter-turn
+// Backproject the n filtered views of buffer b on the compute stream: every z band (band -1, or -2 where more
+// views follow), or one.  FP32_EXACT: one consecutive run.  Staged precisions: the views whose quarter-turn
 // partners (v mod N/4 equal, one from each quarter of the scan) are in the same batch go to the
 // quarter-turn kernel -- each such view as the base of one quadruple, its partners as the other
 // three members -- the rest to the staged kernel by (slot, view).
@@ -158,7 +158,7 @@ int launch_batch(fdk_recon *h, int b, int n, int band) {
     if (h->precision == FDK_BP_FP32_EXACT) {
         const long long first = vw[0];
         return fdk_bp_bp_device_mats_internal(h->bp, h->d_filt[b], h->layout, h->d_mats + 12 * first, n,
-                                              h->mats.data() + 12 * first, h->compute, band);
+                                              h->mats.data() + 12 * first, h->compute, std::max(band, -1));
     }
     std::vector<int> s_slot, s_view, q_slot, q_view;
     if (h->sym_rot && n >= h->pair_least) {
@@ -207,7 +207,7 @@ int launch_batch(fdk_recon *h, int b, int n, int band) {
 // queues behind the filters already issued, and the next filters write its buffer after it),
 // hold the full one, fill the other buffer.
 int rotate_full(fdk_recon *h) {
-    if (h->held) FDK_TRY(launch_batch(h, h->cur ^ 1, h->batch, -1));
+    if (h->held) FDK_TRY(launch_batch(h, h->cur ^ 1, h->batch, -2));
     h->held = true;
     h->cur ^= 1;
     h->pending = 0;
@@ -291,7 +291,7 @@ int process_chunk(fdk_recon *h, const float *d_src, const int64_t *ids, int n, c
         if (h->ramp == 1 && h->pending == ramp_n) {
             // the first batch goes now; the next fills the other buffer (its filters queue behind
             // this launch on the compute stream)
-            FDK_TRY(launch_batch(h, h->cur, h->pending, -1));
+            FDK_TRY(launch_batch(h, h->cur, h->pending, -2));
             h->cur ^= 1;
             h->pending = 0;
             h->bviews[h->cur].clear();

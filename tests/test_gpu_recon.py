@@ -385,3 +385,29 @@ def test_host_scan_starts_with_a_quarter_batch():
     h.close()
     d.close()
     assert rel_l2(vh, vd) <= 1e-6
+
+
+@pytest.mark.parametrize("precision", ["fp32", "mixed"])
+def test_batches_that_no_readback_follows_run_whole(precision, monkeypatch):
+    """128^3 is read back in z bands too thin to fill the chip, so only the flush before the readback runs band by
+    band: until then as many launches as with one band (FDK_BP_BANDS=1), and the same bits at the end."""
+    n, views, batch = 128, 64, 16
+    p = small_param(n, 64, 64, views)
+    rng = np.random.default_rng(5)
+    proj = rng.standard_normal((views, 64, 64)).astype(np.float32)
+
+    def run():
+        r = F.Reconstructor(p, precision, batch=batch)
+        for c in range(0, views, batch):
+            r.push(proj[c:c + batch].copy(), c)
+        before = r.launch_count
+        v = r.volume().copy()
+        after = r.launch_count
+        r.close()
+        return v, before, after
+
+    banded, b0, b1 = run()
+    monkeypatch.setenv("FDK_BP_BANDS", "1")
+    whole, w0, w1 = run()
+    assert b0 == w0 and b1 - b0 > w1 - w0
+    assert np.array_equal(banded, whole) and np.abs(whole).max() > 0
