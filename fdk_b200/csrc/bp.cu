@@ -305,7 +305,8 @@ struct fdk_bp {
     // the reconstructor's MIXED launches read through the compact boxes (every tile fits them)
     bool lerp_compact = false;
     bool lerp_compact_ok = false;  // the compact kernel runs at the same grid
-    bool tall_tiles = false;       // FP32: the staged kernel takes its taller tiles (TallFloat2)
+    bool tall_tiles = false;       // FP32: the staged kernel takes its taller tiles (TallFloat2), choose_tiles
+    int tile_ctas[2] = {0, 0};     // FP32: persistent grid sizes of the lower and the taller tiles
     ListRec *h_list = nullptr, *d_list = nullptr;
     cudaEvent_t list_ev[kListRing] = {};
     bool list_used[kListRing] = {};
@@ -340,16 +341,52 @@ int take_timer(fdk_bp *h, std::pair<cudaEvent_t, cudaEvent_t> &t) {
     return FDK_OK;
 }
 
-// FP32: the staged kernel's taller tiles where the slab gives every CTA of its grid at least four of them.
-// Tall / short there: 1522 / 1434 GUPS at 256^3 (7 tiles a CTA), 1889 / 1756 at 512^3; below it the short
-// tiles are up to 1.23x the faster (133 against 150 us, 86 x 51 x 58 slices from 22 views).
-int choose_tiles(fdk_bp *h) {
-    int ctas = 0;
-    FDK_TRY(tma_prepare<TallFloat2>(ctas, h->device));
+// Of a sample of the (tile, view) pairs, those whose footprint fits the staged FP32 kernel's box (tile_box), for
+// tiles of R slices: 4 x 4 tiles, 5 heights and 4 views, spread evenly from the first to the last.
+constexpr int kFitSample = 4 * 4 * 5 * 4;
+int sampled_fits(const BpFastPlan &p, const float *mats, int n, int R) {
+    using C = TmaCfg<float2>;
+    const int tx = (int)ceil_div(p.nxs, 16), ty = (int)ceil_div(p.nys, 16), tz = (int)ceil_div(p.nzz, R);
+    int fits = 0;
+    for (int i = 0; i < kFitSample; i++) {
+        const float *m = mats + 12 * (long long)((i & 3) * (n - 1) / 3);
+        const float xa = (float)(p.x0 + (i >> 2 & 3) * (tx - 1) / 3 * 16), ya = (float)(p.y0 + (i >> 4 & 3) * (ty - 1) / 3 * 16);
+        const float za = (float)(p.z0 + (i >> 6) * (tz - 1) / 4 * R);
+        float u[2] = {3e38f, -3e38f}, v[2] = {3e38f, -3e38f};
+        for (int c = 0; c < 4; c++) {
+            const float x = xa + (c & 1) * 15, y = ya + (c >> 1) * 15;
+            const float rw = 1.f / (m[8] * x + m[9] * y + m[11]), U = (m[0] * x + m[1] * y + m[3]) * rw;
+            const float va = (m[4] * x + m[5] * y + m[6] * za + m[7]) * rw, vb = va + m[6] * (R - 1) * rw;
+            u[0] = std::min(u[0], U);
+            u[1] = std::max(u[1], U);
+            v[0] = std::min(v[0], std::min(va, vb));
+            v[1] = std::max(v[1], std::max(va, vb));
+        }
+        const float ulo = std::max(std::floor(u[0]) - 1, -1.f), uhi = std::min(std::floor(u[1]) + 2, (float)p.nu);
+        const float vlo = std::max(std::floor(v[0]) - 1, -8.f), vhi = std::min(std::floor(v[1]) + 2, p.nv + 4.f);
+        fits += uhi - ulo + 1 <= C::BH && vhi - std::floor(vlo / 4) * 4 + 1 <= C::BW;
+    }
+    return fits;
+}
+
+// FP32: the staged kernel's taller tiles (TallFloat2) where their footprints fit the box as often and their whole
+// waves hold fewer slices, a staged slice of theirs costing 0.95 of a lower tile's (tall / short: 1522 / 1434 GUPS
+// at 256^3, 1889 / 1756 at 512^3; but 150 / 133 us for 86 x 51 x 58 slices from 22 views, one wave of either).  A
+// box that fewer fit costs more than the height gives: 90 views of 512^2 to 256^3, 10% against 52% fitting, 5637
+// / 4715 us, and with 384^2, 97% against 99%, 1403 / 1301.  n views' matrices; before the first launch.
+void choose_tiles(fdk_bp *h, const float *mats, int n) {
     const BpFastPlan &p = h->plan;
-    h->tall_tiles = ceil_div(p.nxs, 16) * ceil_div(p.nys, 16) * ceil_div(p.nzz, TmaCfg<TallFloat2>::R) >= 4ll * ctas;
-    if (h->tall_tiles) h->plan.tma_ctas = ctas;
-    return FDK_OK;
+    constexpr int low = TmaCfg<float2>::R, tall = TmaCfg<TallFloat2>::R;
+    const auto slices = [&](int R) {
+        return R * (double)ceil_div(ceil_div(p.nxs, 16) * ceil_div(p.nys, 16) * ceil_div(p.nzz, R), h->tile_ctas[R == tall]);
+    };
+    h->tall_tiles = false;
+    if (0.95 * slices(tall) < slices(low)) {
+        const int fits = sampled_fits(p, mats, n, low);
+        const double cost = fits > kFitSample / 2 ? 0.95 : 1.0;
+        h->tall_tiles = cost * slices(tall) < slices(low) && sampled_fits(p, mats, n, tall) >= fits;
+    }
+    h->plan.tma_ctas = h->tile_ctas[h->tall_tiles];
 }
 
 // Tile height of the handle's staged kernel.
@@ -415,9 +452,15 @@ int lerp_call_views(fdk_bp *h, const void *dev_proj, int n, cudaStream_t st, con
     return FDK_OK;
 }
 
+void set_bands(fdk_bp *h, int unit);
+
 int launch_bp(fdk_bp *h, const void *dev_proj, int layout, int transpose, const float *d_mats,
               const float *host_mats, int n, int width, int height, cudaStream_t st,
               const float *acc_scale = nullptr, int band = -1) {
+    if (h->precision == FDK_BP_FP32 && h->plan.tma_ok && h->launches == 0) {
+        choose_tiles(h, host_mats, n);
+        if (h->sym) set_bands(h, staged_rows(h));
+    }
     FDK_CHECK_ARG(band < h->n_bands, "band %d outside 0..%d", band, h->n_bands - 1);
     const int kb = band < 0 ? 0 : band, ke = band < 0 ? h->n_bands : band + 1;
     std::pair<cudaEvent_t, cudaEvent_t> tm;
@@ -840,7 +883,10 @@ int fdk_bp_create(fdk_bp **out, int32_t proj_width, int32_t proj_height, int32_t
             if (h->plan.tma_ok) {
                 s = precision == FDK_BP_MIXED ? tma_prepare<HalfLerp>(h->plan.tma_ctas, device)
                                               : tma_prepare<float2>(h->plan.tma_ctas, device);
-                if (s == FDK_OK && precision != FDK_BP_MIXED) s = choose_tiles(h);
+                if (s == FDK_OK && precision != FDK_BP_MIXED) {
+                    h->tile_ctas[0] = h->plan.tma_ctas;
+                    s = tma_prepare<TallFloat2>(h->tile_ctas[1], device);
+                }
                 if (s == FDK_OK && precision == FDK_BP_MIXED) {
                     int c = 0;
                     s = tma_prepare<HalfLerpCompact>(c, device);
@@ -1174,6 +1220,15 @@ int fdk_bp_choose_lerp_box_internal(fdk_bp *h, const float *mats, int n_proj) {
     }
     using C = TmaCfg<HalfLerpCompact>;
     h->lerp_compact = lerp_compact_fits(mats, n_proj, h->plan, C::R, C::BW, C::BH);
+    return FDK_OK;
+}
+
+// The reconstructor's scan: the staged FP32 kernel's tile height (choose_tiles).  Before fdk_bp_plan_bands_internal.
+// Internal to the library (recon.cu).
+int fdk_bp_choose_tiles_internal(fdk_bp *h, const float *mats, int n_proj) {
+    FDK_CHECK_ARG(h && mats && n_proj > 0, "NULL argument or no views");
+    if (h->precision != FDK_BP_FP32 || !h->plan.tma_ok || h->launches > 0) return FDK_OK;
+    choose_tiles(h, mats, n_proj);
     return FDK_OK;
 }
 

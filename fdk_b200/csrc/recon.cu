@@ -92,6 +92,7 @@ long long fdk_bp_launches_internal(const fdk_bp *h);
 int fdk_bp_bp_device_mats_internal(fdk_bp *h, const void *dev_proj, int32_t layout, const float *dev_mats,
                                    int32_t n_proj, const float *host_mats, void *stream, int32_t band);
 int fdk_bp_band_count_internal(const fdk_bp *h);
+int fdk_bp_choose_tiles_internal(fdk_bp *h, const float *mats, int n_proj);
 int fdk_bp_plan_bands_internal(fdk_bp *h, long long views, bool quarter);
 int fdk_bp_check_internal(fdk_bp *h);
 
@@ -473,6 +474,7 @@ int fdk_recon_create_slab(fdk_recon **out, const fdk_geometry *g, int64_t top_z,
         if (s == FDK_OK && precision == FDK_BP_MIXED) s = fdk_bp_reserve_lerp_internal(h->bp, h->batch);
         if (s == FDK_OK && precision == FDK_BP_MIXED)
             s = fdk_bp_choose_lerp_box_internal(h->bp, h->mats.data(), (int)g->n_proj);
+        if (s == FDK_OK) s = fdk_bp_choose_tiles_internal(h->bp, h->mats.data(), (int)g->n_proj);
         // a flush runs the held batch and the filling one
         if (s == FDK_OK)
             s = fdk_bp_plan_bands_internal(h->bp, std::min<long long>(g->n_proj, 2ll * batch),

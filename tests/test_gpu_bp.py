@@ -193,3 +193,29 @@ def test_exact_views_of_4_gb():
 
     got, want = run(big, rows, rows - crop + 130.5), run(small, crop, 130.5)
     assert np.array_equal(got, want) and np.abs(want).max() > 0
+
+
+@pytest.mark.parametrize("nu", [64, 320, 400, 704])
+def test_fp32_footprints_that_miss_the_box(nu):
+    """Detectors of 0.4 to 4.4 rows a slice: all, some and none of the tiles fit the staged kernel's box, in a slab
+    that fills the taller tiles better (10 x 10 columns of tiles, 176 slices).  The second scan of the handle has
+    pixels of twice the size, so that its tiles are chosen anew.  Against FP32_EXACT; tolerance as
+    test_fp32_tile_heights."""
+    n, half, views = 160, 176, 3
+    p = small_param(n, nu, nu, views)
+    p.nz = 2 * half
+    top, bot = [0, 0, 0, n, n, half], [0, 0, half, n, n, half]
+    filt = random_views(views, nu, nu, seed=nu)
+    bps = [F.BackProjectionFDK(nu, nu, 4, n, n, 2 * half, F.BoxT(*top), F.BoxT(*bot), k) for k in ("fp32", "fp32_exact")]
+    for pitch in (384.0 / nu, 768.0 / nu):
+        p.du = p.dv = pitch
+        vols = []
+        for bp in bps:
+            bp.reset()
+            bp.BP(1, filt, nu, nu, p.proj_matrices(), views)
+            vols.append(bp.GetVolumeData().copy())
+        m = knife_edge_mask(p, top, half)
+        assert np.abs(vols[1]).max() > 0 and m.mean() > 0.5
+        assert rel_l2(vols[0][m], vols[1][m]) <= 4 * 2.0 ** -24 * nu * 2.2
+    for bp in bps:
+        bp.close()
