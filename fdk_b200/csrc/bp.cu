@@ -174,8 +174,9 @@ __global__ void to_lerp_kernel(const __half2 *__restrict__ src, HalfLerp *__rest
     const int k = (M > 0.f && M < 65536.f) ? ilogbf(M) + 1 : 0;  // M is an FP16 magnitude: -23 <= k <= 16
     const float se = pow2i(-k), sd = pow2i(14 - k);
     if (blockIdx.x == 0 && threadIdx.x == 0) *out_scale = (acc_scale ? *acc_scale : 1.0f) * pow2i(k);
-    // 4 pairs a thread and step: nv is a multiple of 4 (the 16-byte rule of the TMA rows).  64 views of
-    // 2048^2: 707 us a pair at a time, 658 so.
+    // 4 pairs a thread and step: nv is a multiple of 4 (the 16-byte rule of the TMA rows).  64 views of 2048^2: 694
+    // us a pair at a time, 600 so.  A grid of a fourth of this size, several steps a thread, took 655 us, and 10.8
+    // against 8.9 us for 16 views of 687 x 328, whose backprojection then took 251 us instead of 237.
     const int groups = nv / 4;
     const long long stride = (long long)gridDim.x * blockDim.x, total = rows * groups;
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -423,7 +424,7 @@ int convert_lerp(fdk_bp *h, const void *src, HalfLerp *dst, long long n_views, i
         static_cast<const __half2 *>(src), pairs, lerp_absmax(h, j));
     FDK_CUDA(cudaGetLastError());
     FDK_CHECK_ARG(h->plan.nv % 4 == 0, "rows of %d pairs are not whole 16-byte words", h->plan.nv);
-    to_lerp_kernel<<<(int)std::min<long long>(ceil_div(pairs / 4, 256), 148 * 8), 256, 0, st>>>(
+    to_lerp_kernel<<<(int)std::min<long long>(ceil_div(pairs / 4, 256), 148 * 32), 256, 0, st>>>(
         static_cast<const __half2 *>(src), dst, rows, h->plan.nv, lerp_absmax(h, j), acc_scale, lerp_scale(h, j));
     FDK_CUDA(cudaGetLastError());
     h->launches += 2;
