@@ -733,6 +733,16 @@ int fdk_correct_image_real32(const fdk_dataref *src, const fdk_dataref *table, f
     FDK_ABI_END
 }
 
+int fdk_scratch_trim(void) {
+    FDK_ABI_BEGIN
+    clear_error();
+    cudaMemPool_t pool = nullptr;
+    FDK_TRY(scratch_pool(&pool, false));
+    if (pool) FDK_CUDA(cudaMemPoolTrimTo(pool, 0));
+    return FDK_OK;
+    FDK_ABI_END
+}
+
 int fdk_filter_row_real32(const fdk_dataref *src, fdk_dataref *dst, const fdk_dataref *filter) {
     FDK_ABI_BEGIN
     clear_error();

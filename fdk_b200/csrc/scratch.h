@@ -1,13 +1,18 @@
 // scratch.h -- short-lived device workspaces of the entry points that have no handle to keep them in.
 //
-// Each device has one stream-ordered memory pool of the library.  Memory that a call frees stays in
+// Each context has one stream-ordered memory pool of the library.  Memory that a call frees stays in
 // the pool up to kScratchKeep bytes (the rest goes back to the device when a stream is next waited
-// for), so that a repeated call does not map and unmap it again: cudaMallocAsync from the default
-// pool, which keeps nothing, cost a forward projection 0.4 ms for a few KB and 1.4 ms for 68 MB.
-// The pool orders reuse across streams and takes calls from any thread.
+// for; fdk_scratch_trim gives back all of it), so that a repeated call does not map and unmap it again:
+// cudaMallocAsync from the default pool, which keeps nothing, cost a forward projection 0.4 ms for a few
+// KB and 1.4 ms for 68 MB.  The pool orders reuse across streams and takes calls from any thread.  A pool goes
+// with its context (cudaDeviceReset): it is remembered with the context's id, which no later context has.
 #pragma once
+#include <cuda.h>
+
 #include <algorithm>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "common.h"
 
@@ -15,26 +20,42 @@ namespace fdk {
 
 constexpr unsigned long long kScratchKeep = 256ull << 20;
 
-// The current device's pool, created at its first use.
-inline int scratch_pool(cudaMemPool_t *out) {
+// The id of the calling thread's context (the primary one is created where there is none).  cuCtxGetId
+// through the runtime's driver entry point: no libcuda link.
+inline int context_id(unsigned long long *out) {
+    using Fn = CUresult (*)(CUcontext, unsigned long long *);
+    static const Fn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess;
+        return ok && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(p) : nullptr;
+    }();
+    FDK_CUDA(cudaFree(nullptr));
+    if (!fn || fn(nullptr, out) != CUDA_SUCCESS) return fail(FDK_ERR_CUDA, "cuCtxGetId failed");
+    return FDK_OK;
+}
+
+// The current context's pool, created at its first use; null if it has none and create is false.
+inline int scratch_pool(cudaMemPool_t *out, bool create = true) {
     static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
-    int dev = 0;
-    FDK_CUDA(cudaGetDevice(&dev));
-    FDK_CHECK_ARG(dev < 64, "device %d", dev);
+    static std::vector<std::pair<unsigned long long, cudaMemPool_t>> pools;  // (context id, pool)
+    *out = nullptr;
+    unsigned long long context = 0;
+    FDK_TRY(context_id(&context));
     std::lock_guard<std::mutex> lock(mu);
-    if (!pools[dev]) {
-        cudaMemPoolProps p{};
-        p.allocType = cudaMemAllocationTypePinned;
-        p.location.type = cudaMemLocationTypeDevice;
-        p.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        FDK_CUDA(cudaMemPoolCreate(&pool, &p));
-        unsigned long long keep = kScratchKeep;
-        FDK_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        pools[dev] = pool;
-    }
-    *out = pools[dev];
+    for (const auto &p : pools)
+        if (p.first == context) *out = p.second;
+    if (*out || !create) return FDK_OK;
+    cudaMemPoolProps p{};
+    p.allocType = cudaMemAllocationTypePinned;
+    p.location.type = cudaMemLocationTypeDevice;
+    FDK_CUDA(cudaGetDevice(&p.location.id));
+    cudaMemPool_t pool = nullptr;
+    FDK_CUDA(cudaMemPoolCreate(&pool, &p));
+    unsigned long long keep = kScratchKeep;
+    FDK_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    pools.emplace_back(context, pool);
+    *out = pool;
     return FDK_OK;
 }
 

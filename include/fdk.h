@@ -163,6 +163,10 @@ typedef struct fdk_dataref {
 } fdk_dataref;
 int fdk_correct_image_real32(const fdk_dataref *src, const fdk_dataref *table, fdk_dataref *dst);
 int fdk_filter_row_real32(const fdk_dataref *src, fdk_dataref *dst, const fdk_dataref *filter);
+/* fdk_filter_row_real32 (tables of a few KB) and fdk_forward_project (a second copy of the volume, where
+ * memory for it can be had) work in a memory pool of the library, one per context, which keeps up to 256 MB of
+ * what they return for the next call.  This gives all of that back to the current device. */
+int fdk_scratch_trim(void);
 /* No counterpart in the reference.  fdk_filter_row_real32 without any device allocation, for
  * callers that cannot allocate device memory when they filter (they reserve the device budget up
  * front, or cannot afford cudaMalloc/cudaFree, which may synchronise the device, in their

@@ -185,3 +185,63 @@ def test_points_per_thread_agree(nu):
             eng.run_device(src.data_ptr(), out.data_ptr(), n, layout, F.DTYPE_F32)
             first = out[:1] if first is None else first
             assert float((out - first).abs().max()) <= 1e-7 * float(first.abs().max()), (layout, n)
+
+
+RESET = """
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, %r)
+from fdk_b200._lib import DataRef, lib
+rt = C.CDLL(%r)
+rng = np.random.default_rng(3)
+views, H = rng.standard_normal((3, 20, 48)).astype(np.float32), rng.uniform(0, 1, 64).astype(np.float32)
+def device(a):
+    p = C.c_void_p()
+    assert rt.cudaMalloc(C.byref(p), C.c_size_t(a.nbytes)) == 0
+    assert rt.cudaMemcpy(p, a.ctypes.data_as(C.c_void_p), C.c_size_t(a.nbytes), 1) == 0
+    return p
+def run():
+    out = np.zeros_like(views)
+    s, d, h = device(views), device(out), device(H)
+    ref = lambda p, w, n, m: C.byref(DataRef(p.value, w, n, m, w))
+    rc = lib().fdk_filter_row_real32(ref(s, 48, 20, 3), ref(d, 48, 20, 3), ref(h, 64, 1, 1))
+    assert rc == 0, lib().fdk_last_error()
+    assert rt.cudaMemcpy(out.ctypes.data_as(C.c_void_p), d, C.c_size_t(out.nbytes), 2) == 0
+    return out
+first = run()
+assert np.array_equal(run(), first) and np.abs(first).max() > 0
+assert lib().fdk_scratch_trim() == 0 and np.array_equal(run(), first)
+assert rt.cudaDeviceReset() == 0
+assert np.array_equal(run(), first)
+print("same after a reset")
+"""
+
+
+def test_scratch_pool_goes_with_its_context():
+    """The row filter's workspace pool is given back on request and made anew after cudaDeviceReset (a process of its
+    own: a reset ends every handle of the context)."""
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", RESET % (root, "/usr/local/cuda/lib64/libcudart.so")], capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and "same after a reset" in r.stdout, r.stderr[-2000:]
+
+
+def test_scratch_pool_is_given_back():
+    """A projection's copy of a 134 MB volume stays in the pool until fdk_scratch_trim."""
+    import ctypes as C
+
+    import torch
+
+    from fdk_b200._lib import check, lib
+
+    p = small_param(320, 600, 600, 2)
+    vol, out = torch.zeros((320, 320, 320), device="cuda"), torch.empty((2, 600, 600), device="cuda")
+    check(lib().fdk_scratch_trim())
+    free = torch.cuda.mem_get_info()[0]
+    check(lib().fdk_forward_project(C.byref(p.to_c()), vol.data_ptr(), 0, 2, out.data_ptr(), None))
+    held = free - torch.cuda.mem_get_info()[0]
+    check(lib().fdk_scratch_trim())
+    assert 100 << 20 < held <= 256 << 20 and free - torch.cuda.mem_get_info()[0] < 8 << 20
