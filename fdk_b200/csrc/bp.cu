@@ -308,6 +308,7 @@ struct fdk_bp {
     bool lerp_compact_ok = false;  // the compact kernel runs at the same grid
     bool tall_tiles = false;       // FP32: the staged kernel takes its taller tiles (TallFloat2), choose_tiles
     int tile_ctas[2] = {0, 0};     // FP32: persistent grid sizes of the lower and the taller tiles
+    float tile_mats[4 * 12] = {};  // the matrices that the choice was made for
     ListRec *h_list = nullptr, *d_list = nullptr;
     cudaEvent_t list_ev[kListRing] = {};
     bool list_used[kListRing] = {};
@@ -345,12 +346,12 @@ int take_timer(fdk_bp *h, std::pair<cudaEvent_t, cudaEvent_t> &t) {
 // Of a sample of the (tile, view) pairs, those whose footprint fits the staged FP32 kernel's box (tile_box), for
 // tiles of R slices: 4 x 4 tiles, 5 heights and 4 views, spread evenly from the first to the last.
 constexpr int kFitSample = 4 * 4 * 5 * 4;
-int sampled_fits(const BpFastPlan &p, const float *mats, int n, int R) {
+int sampled_fits(const BpFastPlan &p, const float (&mats)[4 * 12], int R) {
     using C = TmaCfg<float2>;
     const int tx = (int)ceil_div(p.nxs, 16), ty = (int)ceil_div(p.nys, 16), tz = (int)ceil_div(p.nzz, R);
     int fits = 0;
     for (int i = 0; i < kFitSample; i++) {
-        const float *m = mats + 12 * (long long)((i & 3) * (n - 1) / 3);
+        const float *m = mats + 12 * (i & 3);
         const float xa = (float)(p.x0 + (i >> 2 & 3) * (tx - 1) / 3 * 16), ya = (float)(p.y0 + (i >> 4 & 3) * (ty - 1) / 3 * 16);
         const float za = (float)(p.z0 + (i >> 6) * (tz - 1) / 4 * R);
         float u[2] = {3e38f, -3e38f}, v[2] = {3e38f, -3e38f};
@@ -374,18 +375,23 @@ int sampled_fits(const BpFastPlan &p, const float *mats, int n, int R) {
 // waves hold fewer slices, a staged slice of theirs costing 0.95 of a lower tile's (tall / short: 1522 / 1434 GUPS
 // at 256^3, 1889 / 1756 at 512^3; but 150 / 133 us for 86 x 51 x 58 slices from 22 views, one wave of either).  A
 // box that fewer fit costs more than the height gives: 90 views of 512^2 to 256^3, 10% against 52% fitting, 5637
-// / 4715 us, and with 384^2, 97% against 99%, 1403 / 1301.  n views' matrices; before the first launch.
+// / 4715 us, and with 384^2, 97% against 99%, 1403 / 1301.  n views' matrices; before the first launch.  The sample
+// takes 20 us, so that a scan like the last one keeps its choice.
 void choose_tiles(fdk_bp *h, const float *mats, int n) {
     const BpFastPlan &p = h->plan;
+    float m[4 * 12];
+    for (int i = 0; i < 4; i++) std::copy_n(mats + 12 * (long long)(i * (n - 1) / 3), 12, m + 12 * i);
+    if (std::equal(m, m + 4 * 12, h->tile_mats)) return;
+    std::copy_n(m, 4 * 12, h->tile_mats);
     constexpr int low = TmaCfg<float2>::R, tall = TmaCfg<TallFloat2>::R;
     const auto slices = [&](int R) {
         return R * (double)ceil_div(ceil_div(p.nxs, 16) * ceil_div(p.nys, 16) * ceil_div(p.nzz, R), h->tile_ctas[R == tall]);
     };
     h->tall_tiles = false;
     if (0.95 * slices(tall) < slices(low)) {
-        const int fits = sampled_fits(p, mats, n, low);
+        const int fits = sampled_fits(p, m, low);
         const double cost = fits > kFitSample / 2 ? 0.95 : 1.0;
-        h->tall_tiles = cost * slices(tall) < slices(low) && sampled_fits(p, mats, n, tall) >= fits;
+        h->tall_tiles = cost * slices(tall) < slices(low) && sampled_fits(p, m, tall) >= fits;
     }
     h->plan.tma_ctas = h->tile_ctas[h->tall_tiles];
 }
