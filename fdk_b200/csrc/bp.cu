@@ -371,12 +371,14 @@ int sampled_fits(const BpFastPlan &p, const float (&mats)[4 * 12], int R) {
     return fits;
 }
 
-// FP32: the staged kernel's taller tiles (TallFloat2) where their footprints fit the box as often and their whole
-// waves hold fewer slices, a staged slice of theirs costing 0.95 of a lower tile's (tall / short: 1522 / 1434 GUPS
-// at 256^3, 1889 / 1756 at 512^3; but 150 / 133 us for 86 x 51 x 58 slices from 22 views, one wave of either).  A
-// box that fewer fit costs more than the height gives: 90 views of 512^2 to 256^3, 10% against 52% fitting, 5637
-// / 4715 us, and with 384^2, 97% against 99%, 1403 / 1301.  n views' matrices; before the first launch.  The sample
-// takes 20 us, so that a scan like the last one keeps its choice.
+// FP32: the staged kernel's taller tiles (TallFloat2) where the slab gives every CTA of its grid at least four of
+// them, their whole waves hold fewer slices, a staged slice of theirs costing 0.95 of a lower tile's, and their
+// footprints fit the box as often.  Tall / short: 1522 / 1434 GUPS at 256^3 (7 tiles a CTA), 1889 / 1756 at 512^3;
+// 580 x 280 x 20 slices from 47 views 1027 / 804 us (two tiles of 16 slices for 20).  A box that fewer fit costs more
+// than the height gives: 90 views of 512^2 to 256^3, 10% against 52% fitting, 5637 / 4715 us, and with 384^2, 97%
+// against 99%, 1403 / 1301.  (Below four tiles a CTA the two are within a few percent, and a rank's slab rounds
+// as the whole volume does.)  n views' matrices; before the first launch.  The sample takes 20 us, so that a scan
+// like the last one keeps its choice.
 void choose_tiles(fdk_bp *h, const float *mats, int n) {
     const BpFastPlan &p = h->plan;
     float m[4 * 12];
@@ -384,11 +386,10 @@ void choose_tiles(fdk_bp *h, const float *mats, int n) {
     if (std::equal(m, m + 4 * 12, h->tile_mats)) return;
     std::copy_n(m, 4 * 12, h->tile_mats);
     constexpr int low = TmaCfg<float2>::R, tall = TmaCfg<TallFloat2>::R;
-    const auto slices = [&](int R) {
-        return R * (double)ceil_div(ceil_div(p.nxs, 16) * ceil_div(p.nys, 16) * ceil_div(p.nzz, R), h->tile_ctas[R == tall]);
-    };
+    const auto tiles = [&](int R) { return ceil_div(p.nxs, 16) * ceil_div(p.nys, 16) * ceil_div(p.nzz, R); };
+    const auto slices = [&](int R) { return R * (double)ceil_div(tiles(R), h->tile_ctas[R == tall]); };
     h->tall_tiles = false;
-    if (0.95 * slices(tall) < slices(low)) {
+    if (tiles(tall) >= 4ll * h->tile_ctas[1] && 0.95 * slices(tall) < slices(low)) {
         const int fits = sampled_fits(p, m, low);
         const double cost = fits > kFitSample / 2 ? 0.95 : 1.0;
         h->tall_tiles = cost * slices(tall) < slices(low) && sampled_fits(p, m, tall) >= fits;

@@ -198,10 +198,10 @@ def test_exact_views_of_4_gb():
 @pytest.mark.parametrize("nu", [64, 320, 400, 704])
 def test_fp32_footprints_that_miss_the_box(nu):
     """Detectors of 0.4 to 4.4 rows a slice: all, some and none of the tiles fit the staged kernel's box, in a slab
-    that fills the taller tiles better (10 x 10 columns of tiles, 176 slices).  The second scan of the handle has
-    pixels of twice the size, so that its tiles are chosen anew.  Against FP32_EXACT; tolerance as
+    that fills the taller tiles better (10 x 10 columns of tiles, 216 slices: five waves of two CTAs per SM against
+    seven).  The second scan of the handle has pixels of twice the size, so that its tiles are chosen anew.  Against FP32_EXACT; tolerance as
     test_fp32_tile_heights."""
-    n, half, views = 160, 176, 3
+    n, half, views = 160, 216, 3
     p = small_param(n, nu, nu, views)
     p.nz = 2 * half
     top, bot = [0, 0, 0, n, n, half], [0, 0, half, n, n, half]
