@@ -392,7 +392,7 @@ def accuracy_leg(F, param, views, chunks_of, steps: int, slab, local: int, log) 
         for ptr, ids in pushes:
             r.push_device_views(ptr, ids)
         got[prec] = r.sample(vox)
-        kind[prec] = kernel_run(r, param, BATCH)
+        kind[prec] = r.bp_kernel
         r.close()
     S = O.SampledFDK(param, vox)
     frame = param.nu * param.nv
@@ -472,7 +472,7 @@ def reference_gpu_leg(F, param, views, chunks_of, local: int, log) -> dict | Non
             r.push_device_views(ptr, ids)
         r.sync()
         st = r.stats()
-        ran = kernel_run(r, param, 128, sym)
+        ran = r.bp_kernel
         key = prec if sym is None else f"{prec}_{ran}"
         ours[key] = {"gups": param.nx * param.ny * 2 * dc * 128 / (st["bp_ms"] * 1e-3) / 1e9, "kernel": ran}
         r.close()
@@ -584,7 +584,7 @@ def run_ours(args, param, rank: int, world: int, local: int) -> None:
     clocks.start()
     r, ms, bp_ms, flt_ms, n_launches = timed_device_run(args.precision, args.steps, args.warmup)
     filter_kind = r.filter_kind
-    bp_kind = kernel_run(r, param, BATCH)
+    bp_kind = r.bp_kernel
     clk = clocks.stop()
     r.close()
     del r
@@ -601,7 +601,7 @@ def run_ours(args, param, rank: int, world: int, local: int) -> None:
     fp32 = None
     if not args.no_compare and args.precision == "mixed":
         r2, ms2, bp2, _, _ = timed_device_run("fp32", args.steps, args.warmup, order_of("fp32"))
-        fp32_kind = kernel_run(r2, param, BATCH)
+        fp32_kind = r2.bp_kernel
         r2.close()
         del r2
         torch.cuda.empty_cache()
@@ -944,20 +944,12 @@ def kernel_learned(args) -> None:
 
 
 def pairs_views(param, precision: str) -> bool:
-    """Whether the reconstructor pairs views into quarter-turn quadruples for this precision by
+    """Whether the reconstructor may pair views into quarter-turn quadruples for this precision by
     default (fdk_recon_bp_kernel): FP32 (MIXED with FDK_BP_SYM=1) on a square grid from a scan of
     N % 4 == 0 views; the library's own checks decide in the end."""
     sym = os.environ.get("FDK_BP_SYM", "")
     on = (precision == "fp32" and sym != "0") or (precision == "mixed" and sym == "1")
     return on and param.nx == param.ny and param.nProj % 4 == 0
-
-
-def kernel_run(r, param, batch: int, sym: str | None = None) -> str:
-    """The backprojection kernel that whole batches take: Reconstructor.bp_kernel, but 'staged' where the
-    quarter-turn kernel is set up and not chosen (FDK_BP_SYM=1, or 256 views and more on grids of up to 256)."""
-    sym = os.environ.get("FDK_BP_SYM", "") if sym is None else sym
-    paired = r.bp_kernel == "quarter-turn" and (sym == "1" or (param.nx <= 256 and batch >= 256))
-    return r.bp_kernel if paired or r.bp_kernel != "quarter-turn" else "staged"
 
 
 def main():

@@ -69,6 +69,7 @@ struct fdk_recon {
     std::vector<int> bviews[2];
     int sym_rot = 0;  // quarter-turn kernel's column map (0: not available for this scan)
     int pair_least = 0;  // views of a batch that have to pair for it to take that kernel (fdk_recon_create)
+    bool launched = false, paired = false;  // a batch ran, and one took that kernel, since creation or reset
     double filter_ms = 0;
     long long views = 0;
     long long filter_launches = 0;   // kernel launches of the filter since creation or reset
@@ -199,6 +200,8 @@ int launch_batch(fdk_recon *h, int b, int n, int band) {
             s_view.push_back(vw[i]);
         }
     }
+    h->launched = true;
+    if (!q_view.empty()) h->paired = true;
     return fdk_bp_bp_lists_internal(h->bp, h->d_filt[b], h->batch, h->d_mats, h->mats.data(), s_slot.data(),
                                     s_view.data(), (int)s_slot.size(), q_slot.data(), q_view.data(),
                                     (int)q_view.size(), h->compute, band);
@@ -612,7 +615,8 @@ int fdk_recon_filter_kind(fdk_recon *h, int32_t *kind) {
 
 int fdk_recon_bp_kernel(fdk_recon *h, int32_t *kind) {
     FDK_CHECK_ARG(h && kind, "NULL argument");
-    *kind = h->precision == FDK_BP_FP32_EXACT ? 0 : (h->sym_rot ? 2 : 1);
+    const bool quarter = h->sym_rot && (h->paired || !h->launched);
+    *kind = h->precision == FDK_BP_FP32_EXACT ? 0 : quarter ? 2 : 1;
     return FDK_OK;
 }
 
@@ -714,6 +718,7 @@ int fdk_recon_reset(fdk_recon *h) {
     h->pending = 0;  // filtered views not yet backprojected are dropped with the volume
     h->held = false;
     h->ramp = 0;
+    h->launched = h->paired = false;
     h->bviews[0].clear();
     h->bviews[1].clear();
     h->cur = 0;

@@ -68,8 +68,9 @@ class Reconstructor:
 
     @property
     def bp_kernel(self) -> str:
-        """'exact', 'staged' or 'quarter-turn' (the staged kernel plus the quarter-turn kernel for
-        views whose three quarter-turn partners share their batch, where that is the faster one)."""
+        """What the batches since creation or the last reset ran: 'exact', 'staged' or 'quarter-turn' (the staged
+        kernel plus the quarter-turn kernel for views whose three quarter-turn partners share their batch, where that
+        is the faster one); before the first batch, what is set up."""
         k = C.c_int32()
         check(lib().fdk_recon_bp_kernel(self._h, C.byref(k)))
         return ("exact", "staged", "quarter-turn")[k.value]

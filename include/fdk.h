@@ -301,13 +301,14 @@ int fdk_recon_flush(fdk_recon *h);
  * tensor-core GEMM (fdk_toeplitz_*, MIXED precision when nu % 256 == 0 and nv % 128 == 0 on an
  * sm_100 GPU, unless the environment sets FDK_FILTER=fft). */
 int fdk_recon_filter_kind(fdk_recon *h, int32_t *kind);
-/* The backprojection this reconstructor runs: 0 the reference arithmetic (FP32_EXACT), 1 the
- * staged kernel, 2 the staged kernel plus the quarter-turn kernel: views whose partners
- * v + N/4, v + N/2, v + 3N/4 (mod N) are in the same batch may be backprojected four at a time
+/* The backprojection of the batches since creation or the last reset: 0 the reference arithmetic (FP32_EXACT), 1
+ * the staged kernel, 2 the staged kernel and the quarter-turn kernel: views whose partners
+ * v + N/4, v + N/2, v + 3N/4 (mod N) are in the same batch are backprojected four at a time
  * with one address computation (a circular scan of N % 4 == 0 views about a square, centred
- * grid).  FP32 sets it up by default and uses it for the batches where it measured faster (256 paired
- * views or more, on grids of up to 256 x 256 columns); FDK_BP_SYM=1 uses it for every batch that
- * pairs, in FP32 and MIXED, FDK_BP_SYM=0 never.  No counterpart in the reference. */
+ * grid).  Before the first batch has run: 2 where that kernel is set up.  FP32 sets it up by default and uses it
+ * for the batches where it measured faster (256 paired views or more, on grids of up to 256 x 256 columns);
+ * FDK_BP_SYM=1 uses it for every batch that pairs, in FP32 and MIXED, FDK_BP_SYM=0 never.  No counterpart in
+ * the reference. */
 int fdk_recon_bp_kernel(fdk_recon *h, int32_t *kind);
 /* Wait (bounded by timeout_ms; <= 0 means 10 minutes) until every pushed view is backprojected. */
 int fdk_recon_sync(fdk_recon *h, int64_t timeout_ms);

@@ -122,3 +122,30 @@ def test_full_size_c2_paired_matches_unpaired():
     e = rel_l2(vols[True][0], vols[False][0])
     print("c2 mixed paired vs unpaired", e)
     assert e <= 3e-4
+
+
+@pytest.mark.parametrize("n,views,batch,ran", [
+    (128, 256, 256, "quarter-turn"),  # 256 paired views
+    (128, 256, 252, "staged"),        # 248 of 252 pair
+    (128, 252, 252, "staged"),        # 252 pair
+    (256, 256, 256, "quarter-turn"),
+    (258, 256, 256, "staged"),        # the grid is too large
+    (128, 320, 256, "quarter-turn"),  # a last batch of 64
+])
+def test_default_kernel_on_both_sides_of_its_limits(n, views, batch, ran, monkeypatch):
+    """Without FDK_BP_SYM, FP32: the kernel that ran is the one reported; before anything has run, the one set up."""
+    import torch
+
+    p = small_param(n, 64, 64, views)
+    dev = torch.from_numpy(np.random.default_rng(n + batch).standard_normal((views, 64, 64)).astype(np.float32)).cuda()
+    for sym in ("", "0"):
+        monkeypatch.setenv("FDK_BP_SYM", sym)
+        r = F.Reconstructor(p, "fp32", batch=batch)
+        assert r.bp_kernel == ("staged" if sym else "quarter-turn")
+        for first, k in [(0, views)] if views <= batch else quarter_order(views, 16):
+            r.push_device(dev[first:].data_ptr(), first, k)
+        r.sync()
+        assert r.bp_kernel == ("staged" if sym else ran)
+        r.reset()
+        assert r.bp_kernel == ("staged" if sym else "quarter-turn")
+        r.close()
