@@ -464,12 +464,13 @@ int fdk_recon_create_slab(fdk_recon **out, const fdk_geometry *g, int64_t top_z,
         if (s == FDK_OK && h->d_scale) s = fdk_bp_set_acc_scale_internal(h->bp, h->d_scale);
         // the quarter-turn kernel where the scan and the grid have the symmetry
         if (s == FDK_OK) s = fdk_bp_sym_setup_internal(h->bp, h->mats.data(), (int)g->n_proj, &h->sym_rot);
-        // The quarter-turn kernel on request (FDK_BP_SYM=1), else where it is the faster one: a batch of 256
-        // paired views or more on a grid of up to 256 (1662 against 1522 GUPS at 256^3).  The staged kernel
-        // is ahead below that (256^3 from 128 and 32 views: 1343 and 1092 against 1224 and 671).  On larger
-        // grids it is near or ahead (2048^3 1830 against 1779 GUPS, 512^3 1889 against 1937 from 512 views
-        // and 1719 against 1551 from 128) and needs no order of views: a 512^3 scan from host memory takes
-        // 41.7 ms with it and 46.7 paired.
+        // The quarter-turn kernel on request (FDK_BP_SYM=1), else for batches of 256 paired views or more on grids
+        // of up to 256: 1663 against 1425 GUPS at 256^3, 919 against 845 at 128^3.  (The line is coarse: on grids
+        // whose quadrant leaves its waves half empty the staged kernel is ahead there too, 1390 against 1022 at
+        // 160^3, 837 against 572 at 96^3.)  The staged kernel is ahead with fewer views (256^3 from 128 and 32:
+        // 1346 and 1069 against 1228 and 674).  On larger grids it is near or ahead (2048^3 1830 against 1779 GUPS,
+        // 512^3 1889 against 1937 from 512 views and 1719 against 1551 from 128) and needs no order of
+        // views: a 512^3 scan from host memory takes 41.7 ms with it and 46.7 paired.
         const char *sym_env = std::getenv("FDK_BP_SYM");
         if (sym_env && std::string(sym_env) == "1") h->pair_least = 0;
         else h->pair_least = g->nx <= 256 ? 256 : batch + 1;
