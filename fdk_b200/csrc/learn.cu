@@ -534,8 +534,10 @@ int fdk_voxelize(const fdk_geometry *g, const double *ell, int32_t n_ell, float 
             f.b[r] = (float)b;
             if (!(m <= most)) most = m;
         }
-        const float off = (float)(100.0 / 16777216.0 * (1.0 + most));
-        f.in = 1.f - off;  // not a number (an axis of 0): neither limit holds, FP64 decides
+        // The limits hold to first order: up to M 2^-24 = 1/16.  Beyond (an axis of a millionth of the volume, or of
+        // 0: not a number) no q is outside them, and FP64 decides.
+        const float off = most < (1 << 20) ? (float)(100.0 / 16777216.0 * (1.0 + most)) : INFINITY;
+        f.in = 1.f - off;
         f.out = 1.f + off;
     }
     const dim3 grid((unsigned)ceil_div(g->nx, 32), (unsigned)ceil_div(g->ny, 8 * kVoxRows),

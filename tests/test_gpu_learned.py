@@ -380,3 +380,25 @@ def test_network_wait_that_runs_out_is_reported_at_once(rows, monkeypatch):
     y, g, rc = run()
     assert rc == [0, 0, 0] and np.array_equal(y, want)
     assert np.abs(g - grad).max() <= 1e-5 * np.abs(grad).max()  # the order of the CTAs' FP32 additions
+
+
+def test_voxelizer_keeps_points():
+    """Ellipsoids far smaller than a voxel, each centred on one, turned at random: that voxel is inside (q = 0 in FP64),
+    however large FP32's error of l / a is."""
+    import torch
+
+    p = small_param(64, 64, 64, 4)
+    p.dx = p.dy = p.dz = 1.0
+    rng = np.random.default_rng(4)
+    e = np.zeros((64, 16))
+    at = rng.permutation(64 ** 3)[:64]
+    z, y, x = np.unravel_index(at, (64, 64, 64))
+    e[:, :3] = np.stack([x - 31.5, 31.5 - y, 31.5 - z], -1)
+    e[:, 3:6] = 10.0 ** rng.uniform(-9, -4, (64, 3))
+    e[:, 6:15] = [np.linalg.qr(rng.standard_normal((3, 3)))[0].ravel() for _ in range(64)]
+    e[:, 15] = 1.0
+    out = torch.full((64, 64, 64), 9.0, device="cuda")
+    check(lib().fdk_voxelize(C.byref(p.to_c()), e.ctypes.data, 64, out.data_ptr(), None))
+    want = np.zeros(64 ** 3, np.float32)
+    want[at] = 1.0
+    assert np.array_equal(out.cpu().numpy().ravel(), want)
