@@ -117,8 +117,9 @@ __device__ __forceinline__ bool in_ellipsoid(const double *e, double px, double 
 }
 
 constexpr int kVoxRows = 4;
+// Grid: x and y tiles of 32 x 32 voxels (first_ty: of blockIdx.y = 0), slices.
 __global__ void __launch_bounds__(256) voxelize_kernel(const __grid_constant__ EllipsoidSet ell, int n_ell, int nx, int ny, int nz,
-                                                     double dx, double dy, double dz, float *out) {
+                                                     double dx, double dy, double dz, int first_ty, float *out) {
     __shared__ double se[64 * 16];
     __shared__ EllipsoidForm form[64];
     const int t = threadIdx.y * 32 + threadIdx.x;
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(256) voxelize_kernel(const __grid_constant__ E
         reinterpret_cast<float *>(form)[i] = reinterpret_cast<const float *>(ell.f)[i];
     }
     __syncthreads();
-    const int x = blockIdx.x * 32 + threadIdx.x, y0 = (blockIdx.y * 8 + threadIdx.y) * kVoxRows;
+    const int x = blockIdx.x * 32 + threadIdx.x, y0 = ((first_ty + blockIdx.y) * 8 + threadIdx.y) * kVoxRows;
     if (x >= nx) return;
     const double px = (x - (nx - 1) / 2.0) * dx;
     const float fx = (float)px;
@@ -516,6 +517,7 @@ int fdk_transmission_noise(float *dev_views, int64_t n, double i0, double mu, ui
 int fdk_voxelize(const fdk_geometry *g, const double *ell, int32_t n_ell, float *dev_vol, void *stream) {
     FDK_ABI_BEGIN
     FDK_CHECK_ARG(g && ell && dev_vol && n_ell >= 0 && n_ell <= 64, "bad arguments");
+    if (g->nx <= 0 || g->ny <= 0 || g->nz <= 0) return FDK_OK;  // no voxels
     EllipsoidSet set;
     for (int i = 0; i < 16 * n_ell; i++) set.e[i] = ell[i];
     const double half[3] = {0.5 * (g->nx - 1) * g->dx, 0.5 * (g->ny - 1) * g->dy, 0.5 * (g->nz - 1) * g->dz};
@@ -540,10 +542,12 @@ int fdk_voxelize(const fdk_geometry *g, const double *ell, int32_t n_ell, float 
         f.in = 1.f - off;
         f.out = 1.f + off;
     }
-    const dim3 grid((unsigned)ceil_div(g->nx, 32), (unsigned)ceil_div(g->ny, 8 * kVoxRows),
-                    (unsigned)std::min<int64_t>(g->nz, std::max<int64_t>(1, 148 * 8 / (ceil_div(g->nx, 32) * ceil_div(g->ny, 8 * kVoxRows)))));
-    voxelize_kernel<<<grid, dim3(32, 8), 0, (cudaStream_t)stream>>>(set, n_ell, (int)g->nx, (int)g->ny, (int)g->nz, g->dx,
-                                                                  g->dy, g->dz, dev_vol);
+    const int64_t tiles_x = ceil_div(g->nx, 32), tiles_y = ceil_div(g->ny, 8 * kVoxRows);
+    const unsigned slices = (unsigned)std::min<int64_t>(g->nz, std::max<int64_t>(1, 148 * 8 / (tiles_x * tiles_y)));
+    for (int64_t ty = 0; ty < tiles_y; ty += 65535)  // (the grid's limit)
+        voxelize_kernel<<<dim3((unsigned)tiles_x, (unsigned)std::min<int64_t>(tiles_y - ty, 65535), slices), dim3(32, 8), 0,
+                          (cudaStream_t)stream>>>(set, n_ell, (int)g->nx, (int)g->ny, (int)g->nz, g->dx, g->dy, g->dz,
+                                                  (int)ty, dev_vol);
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
     FDK_ABI_END

@@ -76,3 +76,12 @@ def test_forward_projector_refuses_geometries_that_have_no_rays(field, value):
     g = F.config("c1").to_c()
     setattr(g, field, value)
     assert F.lib().fdk_forward_project(C.byref(g), NO_MEMORY, 0, 1, NO_MEMORY, None) == -1
+
+
+@pytest.mark.skipif(F.device_count() > 0, reason="must not reach a GPU")
+@pytest.mark.parametrize("field", ["nx", "ny", "nz"])
+def test_voxelizer_of_no_voxels_does_nothing(field):
+    g = F.config("c1").to_c()
+    setattr(g, field, 0)
+    e = np.ones((1, 16))
+    assert F.lib().fdk_voxelize(C.byref(g), e.ctypes.data, 1, NO_MEMORY, None) == 0

@@ -402,3 +402,18 @@ def test_voxelizer_keeps_points():
     want = np.zeros(64 ** 3, np.float32)
     want[at] = 1.0
     assert np.array_equal(out.cpu().numpy().ravel(), want)
+
+
+def test_voxelizer_of_a_long_line():
+    """2,200,000 rows of one voxel: more 32-row tiles than a grid's second and third dimensions take."""
+    import torch
+
+    p = small_param(64, 64, 64, 4)
+    p.nx, p.ny, p.nz = 1, 2200000, 1
+    p.dx = p.dy = p.dz = 1.0
+    e = np.zeros((1, 16))
+    e[0, 1], e[0, 3:6], e[0, 6:15], e[0, 15] = -1e6, 100.25, np.eye(3).ravel(), 1.0
+    out = torch.full((p.ny,), 9.0, device="cuda")
+    check(lib().fdk_voxelize(C.byref(p.to_c()), e.ctypes.data, 1, out.data_ptr(), None))
+    y = -(torch.arange(p.ny, device="cuda", dtype=torch.float64) - (p.ny - 1) / 2)
+    assert torch.equal(out, ((y + 1e6).abs() <= 100.25).float())
