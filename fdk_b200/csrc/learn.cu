@@ -18,6 +18,7 @@
 // and its gradient, Adam, Poisson transmission noise, an ellipsoid voxelizer, and the
 // ROWS -> MIRROR layout change that feeds the backprojection.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -223,7 +224,8 @@ __global__ void mse_kernel(const float *__restrict__ vol, const float *__restric
 //
 // The sums are issue-bound (81% of the slots).  256^3 from 90 views of 256^2: 3.04 ms with four atomics a
 // voxel and view and every warp working out each view's footprint; 2.64 with two (a column's row sums
-// stay in registers), 2.39 with the footprints of 8 views shared out among the warps.  Four CTAs per SM (64
+// stay in registers), 2.36 with the footprints of 8 views shared out among the warps, 2.29 with the residuals
+// taken as they are (what is not finite goes past the boxes).  Four CTAs per SM (64
 // registers) instead of three are slower (2.07 against 1.99 ms on another residual).
 //
 // Shared-memory float atomics run as load + compare-and-swap loops, so the boxes hold 32-bit
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(256, 3) bp_adjoint_kernel(AdjArgs a) {
     const int zt = blockIdx.z * kAdjR, nzz = a.nz / 2;
     // residuals of column (x0 + lx, y0 + ly) [mapping 0] and (x0 + ly, y0 + lx) [mapping 1]
     float rm[2][kAdjR], rr[2][kAdjR];
-    bool col_ok[2];
+    bool col_ok[2], lost = false;
 #pragma unroll
     for (int mp = 0; mp < 2; mp++) {
         const int xi = blockIdx.x * 16 + (mp ? ly : lx), yi = blockIdx.y * 16 + (mp ? lx : ly);
@@ -271,8 +273,9 @@ __global__ void __launch_bounds__(256, 3) bp_adjoint_kernel(AdjArgs a) {
             const bool ok = col_ok[mp] && z < nzz;
             const float g = ok ? a.res[((long long)z * a.ny + yi) * a.nx + xi] : 0.f;
             const float gr = ok ? a.res[((long long)(a.nz - 1 - z) * a.ny + yi) * a.nx + xi] : 0.f;
-            rm[mp][k] = g == g ? g : 0.f;  // what is not a number has no fixed-point value and adds nothing
-            rr[mp][k] = gr == gr ? gr : 0.f;
+            rm[mp][k] = g;
+            rr[mp][k] = gr;
+            lost |= !(g == g) || !(gr == gr);
         }
     }
     // largest |residual| of the tile: the fixed-point range
@@ -283,11 +286,13 @@ __global__ void __launch_bounds__(256, 3) bp_adjoint_kernel(AdjArgs a) {
     for (int o = 16; o; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xFFFFFFFFu, gmax, o));
     if ((tid & 31) == 0) warp_max[tid >> 5] = gmax;
     for (int i = tid; i < 2 * 2 * kAdjBV * kAdjBU; i += 256) (&box[0][0][0])[i] = 0;
-    __syncthreads();
+    lost = __syncthreads_or(lost);
     gmax = warp_max[0];
 #pragma unroll
     for (int i = 1; i < 8; i++) gmax = fmaxf(gmax, warp_max[i]);
-    if (!(gmax > 0.f)) return;  // the tile adds nothing (the whole CTA leaves together)
+    if (!(gmax > 0.f || lost)) return;  // the tile adds nothing (the whole CTA leaves together)
+    // what is not finite has no fixed point: the tile's sums go to the pixels as they are
+    const bool fixed_point = gmax <= FLT_MAX && !lost;
     const float zf0 = (float)zt;
     const int warp = tid >> 5;
     for (int s = 0; s < a.n; s++) {
@@ -325,7 +330,7 @@ __global__ void __launch_bounds__(256, 3) bp_adjoint_kernel(AdjArgs a) {
             v.v_lo = (int)floorf(vmin) - 1;
             v.rows = (int)floorf(umax) + 3 - v.u_lo;  // u, v extents
             v.cols = (int)floorf(vmax) + 3 - v.v_lo;
-            v.boxed = v.rows <= kAdjBU && v.cols <= kAdjBV;
+            v.boxed = v.rows <= kAdjBU && v.cols <= kAdjBV && fixed_point;
             v.swap = fabsf(du_y) > fabsf(du_x) ? 1 : 0;  // 16 lanes along the axis with the larger |dU|
             v.scale = ldexpf(1.f, e);
             v.inv_scale = ldexpf(1.f, -e);

@@ -417,3 +417,34 @@ def test_voxelizer_of_a_long_line():
     check(lib().fdk_voxelize(C.byref(p.to_c()), e.ctypes.data, 1, out.data_ptr(), None))
     y = -(torch.arange(p.ny, device="cuda", dtype=torch.float64) - (p.ny - 1) / 2)
     assert torch.equal(out, ((y + 1e6).abs() <= 100.25).float())
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("nu", [24, 128])  # footprints that fit a tile's box, and eight times finer pixels, whose do not
+def test_adjoint_of_residuals_that_are_not_finite(bad, nu):
+    """The pixels of a residual that is not finite are not finite either, all others keep their values."""
+    import torch
+
+    n = 16
+    p = small_param(n, nu, nu, 3)
+    rng = np.random.default_rng(2)
+    res = torch.from_numpy(rng.standard_normal((n, n, n)).astype(np.float32)).cuda()
+    mats = p.proj_matrices().reshape(-1, 12)
+    d_mats = torch.from_numpy(mats.reshape(-1)).cuda()
+    z, y, x = 3, 5, 9
+
+    def adjoint(r):
+        g = torch.zeros((3, nu, nu), device="cuda")
+        check(lib().fdk_bp_adjoint(C.byref(p.to_c()), r.data_ptr(), d_mats.data_ptr(), 3, g.data_ptr(), None))
+        return g.cpu().numpy()
+
+    one = torch.zeros_like(res)
+    one[z, y, x] = 1.0
+    touched = adjoint(one) != 0
+    assert touched.sum() == 12
+    want = adjoint(res)
+    res[z, y, x] = bad
+    got = adjoint(res)
+    assert not np.isfinite(got[touched]).any()
+    # a tile adds in fixed point (2^-19 of its largest term) where its residuals are finite, in FP32 where not
+    assert np.abs(got - want)[~touched].max() <= 2.0 ** -16 * np.abs(want).max()
