@@ -493,7 +493,7 @@ int launch_bp(fdk_bp *h, const void *dev_proj, int layout, int transpose, const 
         a.D = h->D;
         const dim3 grid((unsigned)ceil_div(a.nzz, 32), (unsigned)ceil_div(a.nys, 8), a.nxs);
         if (kb == 0) {
-            const bool wide = (size_t)width * height >= (1ull << 30) - width;
+            const bool wide = (size_t)width * height >= (1ull << 30) - width || std::max(width, height) > 1 << 22;
             auto go = [&](auto sym, auto tr) {
                 constexpr bool S = decltype(sym)::value, T = decltype(tr)::value;
                 if (wide) bp_exact_kernel<S, T, unsigned long long><<<grid, dim3(32, 8), 0, st>>>(a);
@@ -887,7 +887,9 @@ int fdk_bp_create(fdk_bp **out, int32_t proj_width, int32_t proj_height, int32_t
             // The TMA kernel needs 16-byte row strides; FDK_BP_KERNEL=staged selects the
             // synchronous-staging kernel instead (kept for comparison and as the fallback).
             const char *sel = getenv("FDK_BP_KERNEL");
-            h->plan.tma_ok = ((size_t)proj_width * esz) % 16 == 0 && !(sel && std::string(sel) == "staged");
+            // (The FP32 kernel's detector rows end at 2^23: column_view_f32.)
+            h->plan.tma_ok = ((size_t)proj_width * esz) % 16 == 0 && !(sel && std::string(sel) == "staged") &&
+                             (precision == FDK_BP_MIXED || proj_width <= 1 << 22);
             if (h->plan.tma_ok) {
                 s = precision == FDK_BP_MIXED ? tma_prepare<HalfLerp>(h->plan.tma_ctas, device)
                                               : tma_prepare<float2>(h->plan.tma_ctas, device);

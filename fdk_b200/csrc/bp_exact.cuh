@@ -48,15 +48,24 @@ struct __align__(16) BpExactView {
 };
 __device__ __forceinline__ float low2f(f32x2 a) { return __uint_as_float((unsigned)a); }
 
+// Cell and fraction of a coordinate: 64-bit offsets come with detectors of any length, whole_part ends at 2^23.
+template <typename Off>
+__device__ __forceinline__ unsigned cell(float x, float &fraction) {
+    if constexpr (sizeof(Off) == 4) return whole_part(x, fraction);
+    const float i = floorf(x);
+    fraction = x - i;
+    return (unsigned)i;
+}
+
 // SUBPIXEL at detector row v of a view (zero outside [0, last)): frame rows are detector columns
 // (TRANSPOSE: v runs along the row) or detector rows.  `stride`: bytes of a frame row.
 template <bool TRANSPOSE, typename Off>
 __device__ __forceinline__ float subpixel_exact(const char *view, const BpExactView<Off> &m, Off stride, float v, float last) {
     if (!(v >= 0.f && v < last)) return 0.f;
     float e;
-    const unsigned i = whole_part(v, e);
+    const unsigned i = cell<Off>(v, e);
     const float e1 = 1.0f - e;
-    const Off o = m.off + (TRANSPOSE ? i * 4u : i * stride);
+    const Off o = m.off + (TRANSPOSE ? i * (Off)4 : i * stride);
     const float *p0 = reinterpret_cast<const float *>(view + o), *p1 = reinterpret_cast<const float *>(view + (o + stride));
     float x0 = __ldg(p0), x1 = __ldg(p0 + 1), x2 = __ldg(p1), x3 = __ldg(p1 + 1);
     const float d = low2f(m.d), d1 = low2f(m.d1);
@@ -96,7 +105,7 @@ __device__ __forceinline__ f32x2 subpixel_pair(const char *view, const BpExactVi
 // one, with scalar arithmetic, had 72, filled as many slots and 81% of the L1 wavefronts, and took 14.55
 // ms; with voxel and mirror in packed registers where both rows are inside (all but the detector's edge)
 // 13.72.  Two z runs a thread on one record took 15.3 ms, the view loop unrolled twice 16.0 (both scalar).
-// Off: unsigned, or 64 bits for views of 4 GB and more.
+// Off: unsigned, or 64 bits for views of 4 GB and more and for more than 2^22 rows or columns (cell).
 template <bool SYM, bool TRANSPOSE, typename Off>
 __global__ void __launch_bounds__(256, 6) bp_exact_kernel(BpExactArgs a) {
     __shared__ BpExactView<Off> views[8][32];
@@ -125,8 +134,8 @@ __global__ void __launch_bounds__(256, 6) bp_exact_kernel(BpExactArgs a) {
             r.f2 = pack2f(Z * Z, Z * Z);
             if (u >= 0 && u < nu - 1) {
                 float d;
-                const unsigned i = whole_part(u, d);
-                r.off = TRANSPOSE ? i * stride : i * 4u;
+                const unsigned i = cell<Off>(u, d);
+                r.off = TRANSPOSE ? i * stride : i * (Off)4;
                 r.d = pack2f(d, d);
                 r.d1 = pack2f(1.0f - d, 1.0f - d);
                 r.f = Z;
@@ -147,7 +156,7 @@ __global__ void __launch_bounds__(256, 6) bp_exact_kernel(BpExactArgs a) {
             const BpExactView<Off> r = mine[s];
             const float v = fma_rz(r.vz, ijkw.z, r.v0) * r.f;
             const float mirror = last - v, f2 = low2f(r.f2);
-            if (SYM && v >= 0.f && v < last && mirror >= 0.f && mirror < last) {
+            if (SYM && sizeof(Off) == 4 && v >= 0.f && v < last && mirror >= 0.f && mirror < last) {
                 sums = fma2f_rz_ftz(subpixel_pair<TRANSPOSE>(view, r, stride, pack2f(v, mirror)), r.f2, sums);
             } else {
                 float sum, _sum;

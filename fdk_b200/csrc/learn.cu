@@ -254,6 +254,8 @@ struct AdjView {  // a view's footprint of the tile
     float scale, inv_scale;
 };
 
+// LONG: more than 2^22 detector rows.
+template <bool LONG>
 __global__ void __launch_bounds__(256, 3) bp_adjoint_kernel(AdjArgs a) {
     __shared__ int box[2][2][kAdjBV * kAdjBU];  // [buffer][main, mirror], fixed point
     __shared__ float warp_max[8];
@@ -389,8 +391,8 @@ __global__ void __launch_bounds__(256, 3) bp_adjoint_kernel(AdjArgs a) {
                     const bool rv = vr >= 0.f && vr < (float)(a.nv - 1);
                     if (!(mv || rv)) continue;
                     // 0 <= v <= nv - 1 here: its whole part by an addition rounded toward zero
-                    const float vf = fminf(__fadd_rz(v, 8388608.f) - 8388608.f, (float)(a.nv - 2));
-                    const int vi = __float_as_int(vf + 8388608.f) - 0x4B000000;
+                    const float vf = fminf(LONG ? floorf(v) : __fadd_rz(v, 8388608.f) - 8388608.f, (float)(a.nv - 2));
+                    const int vi = LONG ? (int)vf : __float_as_int(vf + 8388608.f) - 0x4B000000;
                     const float fv = v - vf;
                     if (vi != cur) {
                         const bool next = vi == cur + 1;
@@ -605,7 +607,8 @@ int fdk_bp_adjoint(const fdk_geometry *g, const float *dev_res, const float *dev
     a.nu = (int)g->nu;
     a.nv = (int)g->nv;
     const dim3 grid((unsigned)ceil_div(a.nx, 16), (unsigned)ceil_div(a.ny, 16), (unsigned)ceil_div(a.nz / 2, kAdjR));
-    bp_adjoint_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+    if (a.nv > 1 << 22) bp_adjoint_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+    else bp_adjoint_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(a);
     FDK_CUDA(cudaGetLastError());
     return FDK_OK;
     FDK_ABI_END

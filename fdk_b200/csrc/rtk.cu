@@ -16,6 +16,7 @@
 //  * rtk_bp_kernel: the same gathers through L1 (__ldg).  Used where TMA cannot address the
 //    views (width not a multiple of 4 floats, base not 16-byte aligned) or when the environment
 //    sets FDK_RTK_KERNEL=l1.
+#include <algorithm>
 #include <string>
 #include <type_traits>
 
@@ -395,7 +396,8 @@ using namespace fdk;
 namespace fdk {
 
 // Staged kernel where TMA can address the views (rows a multiple of 16 bytes, 16-byte aligned
-// base, a detector at least one box wide and high); the L1 kernel otherwise.
+// base, a detector at least one box wide and high, and no coordinate near the 2^23 at which the packed whole
+// parts end); the L1 kernel otherwise.
 int rtk_launch(const int32_t proj_size[3], const int32_t vol_size[3], const float *host_mats, const float *dev_vol_in,
                float *dev_vol_out, const float *dev_proj, cudaStream_t st) {
     const int W = proj_size[0], H = proj_size[1], n = proj_size[2];
@@ -405,7 +407,7 @@ int rtk_launch(const int32_t proj_size[3], const int32_t vol_size[3], const floa
     const char *sel = getenv("FDK_RTK_KERNEL");
     const bool l1 = sel && std::string(sel) == "l1";
     const bool tma_ok = !l1 && W % 4 == 0 && ((uintptr_t)dev_proj & 15) == 0 && W >= rtkt::BW && H >= rtkt::BH &&
-                        tensor_map_encoder() != nullptr;
+                        std::max(W, H) <= 1 << 22 && tensor_map_encoder() != nullptr;
     if (!tma_ok) {
         const dim3 grid((unsigned)ceil_div(nx, 32), (unsigned)ceil_div(ny, 8), (unsigned)ceil_div(nz, kRtkR));
         rtk_bp_kernel<<<grid, dim3(32, 8), 0, st>>>(dev_vol_in, dev_vol_out, dev_proj, m, W, H, n, nx, ny, nz);

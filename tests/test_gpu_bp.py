@@ -219,3 +219,62 @@ def test_fp32_footprints_that_miss_the_box(nu):
         assert rel_l2(vols[0][m], vols[1][m]) <= 4 * 2.0 ** -24 * nu * 2.2
     for bp in bps:
         bp.close()
+
+
+@pytest.mark.parametrize("precision,layout", [("fp32_exact", "transposed"), ("fp32_exact", "rows"), ("fp32", "mirror")])
+def test_detectors_of_more_than_2_23_rows(precision, layout):
+    """Detector rows beyond 2^23, where adding 2^23 no longer leaves a coordinate's whole part in the low bits, against
+    a crop of the detector.  w = 1, u dyadic and v whole, so that moving the origin changes no rounding: FP32_EXACT gives
+    the same bits, FP32, which takes another kernel, three roundings of a sample.  (Top slices only: the mirror
+    ones fall outside the crop.)"""
+    import torch
+
+    n, nu, rows, crop = 16, 8, (1 << 23) + 512, 512
+    tail = torch.from_numpy(random_views(1, nu, crop, seed=8)).cuda()
+
+    def run(nv, v0):
+        x = torch.zeros((1, nu, nv), device="cuda")  # (views, u, v)
+        x[:, :, nv - crop:] = tail
+        if layout == "rows":
+            x = x.transpose(1, 2).contiguous()
+        if layout == "mirror":
+            x = torch.stack([x, x.flip(2)], -1).contiguous()
+        m = np.array([[0.25, 0, 0, 1.5, 2.0, 1.0, 8.0, v0, 0, 0, 0, 1.0]], np.float32)
+        half = n // 2
+        top, bot = F.BoxT(0, 0, 0, n, n, half), F.BoxT(0, 0, half, n, n, half)
+        w, h = (nu, nv) if layout == "rows" else (nv, nu)
+        bp = F.BackProjectionFDK(w, h, 1, n, n, n, top, bot, precision)
+        if layout == "rows":
+            bp.BP(0, x.cpu().numpy(), w, h, m, 1)
+        else:
+            bp.BP_device(x.data_ptr(), F.LAYOUT_MIRROR if layout == "mirror" else F.LAYOUT_TRANSPOSED, m, 1)
+        vol = np.asarray(bp.GetVolumeData()).reshape(n, n, n)[:half].copy()
+        bp.close()
+        return vol
+
+    got, want = run(rows, rows - 300.0), run(crop, crop - 300.0)
+    assert np.abs(want).max() > 0
+    assert np.array_equal(got, want) if precision == "fp32_exact" else max_rel(got, want) <= 2.0 ** -22
+
+
+def test_adjoint_of_more_than_2_23_rows():
+    """As above, the adjoint: gradient rows of the big detector and of its crop."""
+    import ctypes as C
+
+    import torch
+
+    from fdk_b200._lib import check, lib
+
+    n, nu, rows, crop = 16, 8, (1 << 23) + 512, 512
+    res = torch.randn((n, n, n), device="cuda")
+    res[n // 2:] = 0  # no mirror slices
+
+    def run(nv):
+        p = small_param(n, nu, nv, 1)
+        m = torch.tensor([0.25, 0, 0, 1.5, 2.0, 1.0, 8.0, nv - 300.0, 0, 0, 0, 1.0], device="cuda")
+        g = torch.zeros((1, nv, nu), device="cuda")
+        check(lib().fdk_bp_adjoint(C.byref(p.to_c()), res.data_ptr(), m.data_ptr(), 1, g.data_ptr(), None))
+        return g[0, nv - crop:].cpu().numpy()
+
+    got, want = run(rows), run(crop)
+    assert np.abs(got - want).max() <= 2.0 ** -16 * np.abs(want).max() and np.abs(want).max() > 0
