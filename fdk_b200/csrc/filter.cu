@@ -375,32 +375,33 @@ __global__ void __launch_bounds__(Fft<LOG2W, LOG2E>::TPF * G, TW == Twiddles::Ea
                     d[ra] = y.x;
                     if (rb != ra) d[rb] = y.y;
                 }
-            } else {  // mirror pairs: element (u, v) = (row v, row nv-1-v)
+            } else {  // mirror pairs: element (u, v) = (row v, row nv-1-v); ra last, so that the middle row of an
+                      // odd nv has its real part first
                 const long long o = view * (a.dst_vstride / 2) + (long long)u * a.dst_pitch;
                 if (a.half) {
                     __half2 *d = static_cast<__half2 *>(a.dst) + o;
                     const __half x = __float2half_rn(y.x), z = __float2half_rn(y.y);
                     if (a.pair_stores) {
-                        d[ra] = __halves2half2(x, z);
                         d[rb] = __halves2half2(z, x);
+                        d[ra] = __halves2half2(x, z);
                     } else {
                         __half *e = reinterpret_cast<__half *>(d);
-                        e[2 * ra] = x;
-                        e[2 * ra + 1] = z;
                         e[2 * rb] = z;
                         e[2 * rb + 1] = x;
+                        e[2 * ra] = x;
+                        e[2 * ra + 1] = z;
                     }
                 } else {
                     float2 *d = static_cast<float2 *>(a.dst) + o;
                     if (a.pair_stores) {
-                        d[ra] = y;
                         d[rb] = make_float2(y.y, y.x);
+                        d[ra] = y;
                     } else {
                         float *e = reinterpret_cast<float *>(d);
-                        e[2 * ra] = y.x;
-                        e[2 * ra + 1] = y.y;
                         e[2 * rb] = y.y;
                         e[2 * rb + 1] = y.x;
+                        e[2 * ra] = y.x;
+                        e[2 * ra + 1] = y.y;
                     }
                 }
             }
@@ -551,6 +552,7 @@ int filter_views(const float *src, int src_pitch, long long src_vstride, void *d
                  unsigned int *overflow) {
     FDK_CHECK_ARG(t.hb && t.tw, "filter tables are missing");
     FDK_CHECK_ARG(((uintptr_t)t.hb & 15) == 0 && ((uintptr_t)t.twp & 15) == 0, "filter tables must start on 16-byte boundaries");
+    FDK_CHECK_ARG(layout != FDK_LAYOUT_MIRROR || dst_vstride % 2 == 0, "mirror views are whole pairs apart");
     FilterArgs a;
     a.src = src;
     a.dst = dst;
@@ -570,7 +572,7 @@ int filter_views(const float *src, int src_pitch, long long src_vstride, void *d
     a.dst_vstride = dst_vstride;
     a.layout = layout;
     a.half = dtype == FDK_DTYPE_F16;
-    a.pair_stores = ((uintptr_t)dst & (a.half ? 3 : 7)) == 0 && dst_vstride % 2 == 0;
+    a.pair_stores = ((uintptr_t)dst & (a.half ? 3 : 7)) == 0;
     a.out_scale = out_scale;
     a.overflow = overflow;
     return launch_filter(a, t.log2W, n_views, st);

@@ -187,6 +187,24 @@ def test_points_per_thread_agree(nu):
             assert float((out - first).abs().max()) <= 1e-7 * float(first.abs().max()), (layout, n)
 
 
+@pytest.mark.parametrize("nu,nv,views", [(300, 37, 1), (300, 37, 40), (2000, 5, 3), (2000, 101, 16)])
+@pytest.mark.parametrize("shift", [0, 1])  # dst on a pair's boundary or on a float's
+def test_middle_row_of_an_odd_detector(nu, nv, views, shift):
+    """The MIRROR pair of the middle row is that row twice, as the real and as the imaginary part of its transform: the
+    first is what TRANSPOSED holds, bit for bit."""
+    import torch
+
+    rng = np.random.default_rng(nu + nv)
+    cos = rng.uniform(0.9, 1.0, (nv, nu)).astype(np.float32)
+    eng = F.FilterEngine(cos, O.filter_design("hann", nu).astype(np.float32))
+    src = torch.from_numpy((rng.standard_normal((views, nv, nu)) + 2.0).astype(np.float32)).cuda()
+    t = torch.empty((views, nu, nv), device="cuda")
+    m = torch.empty(views * nu * nv * 2 + shift, device="cuda")[shift:]
+    eng.run_device(src.data_ptr(), t.data_ptr(), views, F.LAYOUT_TRANSPOSED, F.DTYPE_F32)
+    eng.run_device(src.data_ptr(), m.data_ptr(), views, F.LAYOUT_MIRROR, F.DTYPE_F32)
+    assert torch.equal(m.view(views, nu, nv, 2)[..., 0], t)
+
+
 RESET = """
 import ctypes as C, sys
 import numpy as np
