@@ -18,7 +18,8 @@
 // shared-memory wavefronts and FP32 issue about equally (per 512 points and warp some 460
 // wavefronts and 1200 FP32 instructions at W = 4096).  Plain butterflies cost an eighth more
 // arithmetic than radix-16 ones with their constants folded (32 views of 2048^2 to MIRROR FP32:
-// 997 against 973 us) and keep the outputs, bit for bit, those of a stage-by-stage transform.
+// 997 against 973 us) and keep the roundings of a stage-by-stage transform (but for the roots 1 and -i, whose
+// rounded tables may add 6e-17 of the other component).
 #include <cuda_fp16.h>
 
 #include <algorithm>

@@ -1,8 +1,8 @@
 // filter_noalloc.cu -- fdk_filter_row_real32_noalloc: the row filter of fdk_filter_row_real32
 // without any device allocation.
 //
-// fdk_filter_row_real32 allocates two small device tables per call (the FFT twiddles and the
-// reordered, 1/W-scaled response) and frees them again.  Some callers cannot allocate device
+// fdk_filter_row_real32 takes its device tables (the FFT twiddles and the reordered, 1/W-scaled
+// response) from the library's memory pool, which allocates.  Some callers cannot allocate device
 // memory at that point: applications that reserve the whole device budget up front and hand
 // out memory themselves, and processing loops that must not call cudaMalloc/cudaFree because
 // those calls can synchronise the device and stall every other stream.  For them this entry

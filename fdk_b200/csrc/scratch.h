@@ -30,7 +30,8 @@ inline int context_id(unsigned long long *out) {
         const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess;
         return ok && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(p) : nullptr;
     }();
-    FDK_CUDA(cudaFree(nullptr));
+    if (fn && fn(nullptr, out) == CUDA_SUCCESS) return FDK_OK;
+    FDK_CUDA(cudaFree(nullptr));  // makes one (not called where there is one: it would break a capture of another thread)
     if (!fn || fn(nullptr, out) != CUDA_SUCCESS) return fail(FDK_ERR_CUDA, "cuCtxGetId failed");
     return FDK_OK;
 }

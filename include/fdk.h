@@ -360,7 +360,7 @@ int fdk_phantom_project(const fdk_geometry *g, const double *ell, int32_t n_ell,
  *      (genProj/cudaForwardProjection.cu:174-254, Text3DLinear genProj/cudaIterType.cuh:232-276) */
 /* dev_vol: device volume [z][y][x] (x fastest) of g's size.  Writes views first..first+n-1, nv x nu
  * each, to dev_out: per detector pixel, trilinear samples every min(dx, dy, dz) mm along the ray
- * inside the voxel-centre box, times the step.  Asynchronous on stream (returns after queueing). */
+ * inside the voxel-centre box, times the step.  Runs on stream and waits for it. */
 int fdk_forward_project(const fdk_geometry *g, const float *dev_vol, int64_t first, int64_t n, float *dev_out,
                         void *stream);
 
