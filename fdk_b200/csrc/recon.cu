@@ -438,10 +438,11 @@ int fdk_recon_create_slab(fdk_recon **out, const fdk_geometry *g, int64_t top_z,
         if (s == FDK_OK) ck(cudaMalloc(&h->d_scale, sizeof(float)), "scale");
         if (s == FDK_OK)
             ck(cudaMemcpyAsync(h->d_scale, &k, sizeof(float), cudaMemcpyHostToDevice, h->compute), "scale");
-        // the filter, chosen by measurement: on the C3/C4 workloads the split-FP16 tensor-core
-        // GEMM (fdk_toeplitz_*) matches the FFT filter's accuracy (rel-L2 2e-4, the FP16 output
-        // rounding) in 0.61x (C3) / 0.67x (C4) of its time.  The FFT filter remains where the GEMM
-        // cannot run (nu not a multiple of 256, nv of 128) or when FDK_FILTER=fft.
+        // the filter: the split-FP16 tensor-core GEMM (fdk_toeplitz_*) has the FFT filter's accuracy (rel-L2 2e-4,
+        // the FP16 output rounding).  It was chosen when it was the faster: 5.2 against 8.6 ms for 128 views of
+        // 2048^2, 1.58 against 2.37 for 1536 x 1024.  The FFT filter takes 3.9 and 0.97 ms now (FDK_FILTER=fft); the
+        // choice has not been made anew.  The FFT filter also runs where the GEMM cannot (nu not a multiple of
+        // 256, nv of 128).
         const char *want = std::getenv("FDK_FILTER");
         const bool fft_only = want && std::string(want) == "fft";
         if (s == FDK_OK && !fft_only && g->nu % 256 == 0 && g->nv % 128 == 0) {
